@@ -92,7 +92,7 @@ __device__ __forceinline__ double group_sum(double x) {
 // and besides it no spoiler or gradient (they would act on M0 or on the evolved state) and no readout
 // after it that resets the state before the row ends. row_ev[o] = that event, or -1; *all_ok is cleared
 // when a row is not such a row.
-__global__ void adjoint_rows_kernel(const EvRec<double>* __restrict__ rec, int n_off, int n_ev, int reset_after_adc,
+static __global__ void adjoint_rows_kernel(const EvRec<double>* __restrict__ rec, int n_off, int n_ev, int reset_after_adc,
                                     int* __restrict__ row_ev, int* __restrict__ all_ok) {
     const int o = blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= n_off) return;

@@ -63,7 +63,7 @@ constexpr int kAdjBlkWarps = 4;
 // most kAdjL events taken once; the block's events are RF blocks or delays; no spoiler or gradient
 // anywhere; no readout that resets the state before the row ends. out[row] = (first, L, r, 1) or zero;
 // *all_ok is cleared when a row does not qualify.
-__global__ void adjoint_block_rows_kernel(const EvRec<double>* __restrict__ rec, int n_rows, int n_ev, int stride,
+static __global__ void adjoint_block_rows_kernel(const EvRec<double>* __restrict__ rec, int n_rows, int n_ev, int stride,
                                           const int4* __restrict__ seg, int reset_after_adc,
                                           int4* __restrict__ out, int* __restrict__ all_ok) {
     const int o = blockIdx.x * blockDim.x + threadIdx.x;

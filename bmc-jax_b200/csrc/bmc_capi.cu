@@ -1,9 +1,9 @@
 // bmc_capi.cu -- the C ABI declared in include/bmc_b200.h.
 //
-// Host side of the library: argument checks, a per-device workspace cache, the truncated-Taylor
-// tables, event preprocessing, the dispatch over pool count / precision / tangents per launch,
-// and the device-side Levenberg-Marquardt loop (every launch asynchronous on the caller's stream,
-// no host synchronisation inside a call).
+// Host side of the library: argument checks, a per-device workspace cache, the truncated-Taylor tables, the
+// dispatch over pool count, uneven plans and the joint step. What is compiled per pool count (the launches of
+// a call, the Levenberg-Marquardt loop) is in bmc_impl.cu. Every launch is asynchronous on the caller's stream,
+// with no host synchronisation inside a call.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -17,20 +17,21 @@
 #include <string>
 #include <vector>
 
-#include "../../include/bmc_b200.h"
 #include <cub/device/device_radix_sort.cuh>
 
+#include "bmc_host.h"
 #include "bmc_lm.cuh"
 #include "bmc_joint.cuh"
 #include "bmc_adjoint.cuh"
 #include "bmc_adjoint_block.cuh"
-#include "bmc_design.cuh"
 
 using namespace bmc;
 
 namespace {
-
 thread_local std::string g_err;
+}
+
+namespace bmc {
 
 bmc_status fail(bmc_status s, const char* fmt, ...) {
     char buf[512];
@@ -42,23 +43,13 @@ bmc_status fail(bmc_status s, const char* fmt, ...) {
     return s;
 }
 
-#define CUDA_TRY(expr)                                                                          \
-    do {                                                                                        \
-        cudaError_t e_ = (expr);                                                                \
-        if (e_ != cudaSuccess) return fail(BMC_ERR_CUDA, "%s: %s", #expr, cudaGetErrorString(e_)); \
-    } while (0)
-
-}  // namespace
-
-namespace bmc {
 // the same thread-local message for the library's other translation units (bmc_mlp.cu)
 bmc_status record_error(bmc_status s, const char* msg) {
     g_err = msg;
     return s;
 }
-}  // namespace bmc
 
-namespace {
+std::atomic<int> g_tangent_mode{BMC_TANGENTS_AUTO};
 
 // ------------------------------------------------------------------------------------------------
 // truncated-Taylor tables: theta[m] = max t with t^(m+1)/(m+1)! / (1 - t/(m+2)) <= tol, a bound of the
@@ -216,20 +207,6 @@ bmc_status workspace(size_t bytes, cudaStream_t st, void** out) {
     return BMC_OK;
 }
 
-struct Carve {
-    char* p;
-    size_t used = 0;
-    explicit Carve(void* base) : p((char*)base) {}
-    template <typename T>
-    T* take(size_t n) {
-        used = (used + 255) & ~size_t(255);
-        T* r = (T*)(p + used);
-        used += n * sizeof(T);
-        return r;
-    }
-};
-size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
-
 bmc_status check_problem(const bmc_problem* pr, const double* params, const bmc_events* ev, const double* m0) {
     if (!pr || !params || !ev || !m0) return fail(BMC_ERR_INVALID, "null problem, params, events or m0");
     if (pr->n_voxels < 1 || pr->n_offsets < 1 || pr->n_events < 0)
@@ -272,18 +249,6 @@ bmc_status scan_blocks(const EvRec<double>* rec, int n_rows, int n_ev, int strid
     return BMC_OK;
 }
 
-template <typename R>
-bmc_status prep_events(const bmc_problem* pr, const bmc_events* ev, EvRec<R>* out, cudaStream_t st) {
-    const size_t n = (size_t)pr->n_offsets * pr->n_events;
-    if (n == 0) return BMC_OK;
-    const int blocks = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
-    prep_events_kernel<R><<<blocks, 256, 0, st>>>(pr->n_offsets, pr->n_events, ev->d_type, ev->d_dt, ev->d_rf_amp,
-                                                  ev->d_rf_phase, ev->d_rf_freq, out);
-    CUDA_TRY(cudaGetLastError());
-    return BMC_OK;
-}
-
-
 // ------------------------------------------------------------------------------------------------
 // FMA throughput probe: kChains independent fused multiply-add chains per thread, in registers
 // ------------------------------------------------------------------------------------------------
@@ -307,89 +272,6 @@ __global__ void __launch_bounds__(256) fma_probe_kernel(int iters, R seed, R* si
 // ------------------------------------------------------------------------------------------------
 // launches
 // ------------------------------------------------------------------------------------------------
-template <int NC, typename R, int NT, bool U, bool COUNT>
-bmc_status launch_chain_impl(const ChainArgs& a, const TaylorTable* tt, cudaStream_t st) {
-    constexpr int kWarps = ChainLaunch<NC, NT>::kWarps;
-    const size_t smem = kWarps * sizeof(DenseSmem<NC, typename DenseReal<R>::type, NT>) +
-                        32 * kWarps * sizeof(ChainConst<NC, Dn<R, NT>>);
-    // the attribute once per device and instantiation: later calls then only enqueue work (which keeps
-    // them capturable in a CUDA graph). Atomic: calls on several devices may come from several threads.
-    static std::atomic<unsigned long long> configured{0};
-    int dev = 0;
-    CUDA_TRY(cudaGetDevice(&dev));
-    if (dev >= 64 || !((configured.load(std::memory_order_acquire) >> dev) & 1ull)) {
-        CUDA_TRY(cudaFuncSetAttribute(chain_kernel<NC, R, NT, U, COUNT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
-        if (dev < 64) configured.fetch_or(1ull << dev, std::memory_order_acq_rel);
-    }
-    const long long nch = U ? a.n_chains : (long long)a.n_vox * a.n_off;
-    const long long blocks = (nch + kWarps * 32 - 1) / (kWarps * 32);
-    if (blocks > 0x7fffffffLL) return fail(BMC_ERR_INVALID, "%lld chains exceed one launch", nch);
-    if (blocks == 0) return BMC_OK;
-    TaylorTable th;
-    if (bmc_status s = host_table_of(tt, &th); s != BMC_OK) return s;
-    chain_kernel<NC, R, NT, U, COUNT><<<(unsigned)blocks, kWarps * 32, smem, st>>>(a, th);
-    CUDA_TRY(cudaGetLastError());
-    return BMC_OK;
-}
-
-// the counting instantiation only where a.work asks for counts (the uneven plans never do)
-template <int NC, typename R, int NT, bool U = false>
-bmc_status launch_chain(const ChainArgs& a, const TaylorTable* tt, cudaStream_t st) {
-    if constexpr (!U) {
-        if (a.work) return launch_chain_impl<NC, R, NT, U, true>(a, tt, st);
-    } else {
-        if (a.work) return fail(BMC_ERR_UNSUPPORTED, "work counts of an uneven plan");
-    }
-    return launch_chain_impl<NC, R, NT, U, false>(a, tt, st);
-}
-
-// Tangent mode (bmc_set_tangent_mode): BMC_TANGENTS_AUTO takes the adjoint kernel where it applies.
-std::atomic<int> g_tangent_mode{BMC_TANGENTS_AUTO};
-
-template <int NC, bool kTan = true>
-bmc_status launch_adjoint(const ChainArgs& a, const int* row_ev, int n_tan, const TaylorTable* tt, cudaStream_t st) {
-    const size_t smem = kAdjWarps * AdjGroup<NC>::G * sizeof(AdjSlot<NC>);
-    static std::atomic<unsigned long long> configured{0};
-    int dev = 0;
-    CUDA_TRY(cudaGetDevice(&dev));
-    if (dev >= 64 || !((configured.load(std::memory_order_acquire) >> dev) & 1ull)) {
-        CUDA_TRY(cudaFuncSetAttribute(adjoint_kernel<NC, kTan>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
-        if (dev < 64) configured.fetch_or(1ull << dev, std::memory_order_acq_rel);
-    }
-    const long long nch = (long long)a.n_vox * a.n_off;
-    const long long blocks = (nch + kAdjWarps * 32 - 1) / (kAdjWarps * 32);
-    if (blocks > 0x7fffffffLL) return fail(BMC_ERR_INVALID, "%lld chains exceed one launch", nch);
-    if (blocks == 0) return BMC_OK;
-    TaylorTable th;
-    if (bmc_status s = host_table_of(tt, &th); s != BMC_OK) return s;
-    adjoint_kernel<NC, kTan><<<(unsigned)blocks, kAdjWarps * 32, smem, st>>>(a, row_ev, n_tan, th);
-    CUDA_TRY(cudaGetLastError());
-    return BMC_OK;
-}
-
-template <int NC, bool kTan = true>
-bmc_status launch_adjoint_block(const ChainArgs& a, const int4* blk, int n_tan, const TaylorTable* tt, cudaStream_t st) {
-    const size_t smem = kAdjBlkWarps * DenseGroup<NC>::G * sizeof(AdjBlkSlot<NC, kTan>);
-    static std::atomic<unsigned long long> configured{0};
-    int dev = 0;
-    CUDA_TRY(cudaGetDevice(&dev));
-    if (dev >= 64 || !((configured.load(std::memory_order_acquire) >> dev) & 1ull)) {
-        CUDA_TRY(cudaFuncSetAttribute(adjoint_block_kernel<NC, kTan>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
-        if (dev < 64) configured.fetch_or(1ull << dev, std::memory_order_acq_rel);
-    }
-    const long long blocks = (a.n_chains + kAdjBlkWarps * 32 - 1) / (kAdjBlkWarps * 32);
-    if (blocks > 0x7fffffffLL) return fail(BMC_ERR_INVALID, "%lld chains exceed one launch", a.n_chains);
-    if (blocks == 0) return BMC_OK;
-    TaylorTable th;
-    if (bmc_status s = host_table_of(tt, &th); s != BMC_OK) return s;
-    adjoint_block_kernel<NC, kTan><<<(unsigned)blocks, kAdjBlkWarps * 32, smem, st>>>(a, blk, n_tan, th);
-    CUDA_TRY(cudaGetLastError());
-    return BMC_OK;
-}
-
 // Whether the tangents of a uniform table go through the adjoint kernel: two or more tangents, the
 // automatic mode, and every row a single-event row (adjoint_rows_kernel, which also fills row_ev). The
 // check reads one flag back, so a stream being captured keeps forward mode.
@@ -413,25 +295,6 @@ bmc_status use_adjoint(const EvRec<double>* rec, const bmc_problem* pr, int n_ta
     return BMC_OK;
 }
 
-// Order the chains by estimated cost: `order` and the sort's scratch are carved from `cv`.
-template <int NC, typename R>
-bmc_status order_chains(ChainArgs& a, Carve& cv, cudaStream_t st) {
-    const long long nch = (long long)a.n_vox * a.n_off;
-    if (nch < 2 * 128 || a.n_ev == 0) return BMC_OK;
-    float* k_in = cv.take<float>(nch);
-    float* k_out = cv.take<float>(nch);
-    int* i_in = cv.take<int>(nch);
-    int* i_out = cv.take<int>(nch);
-    size_t tmp = 0;
-    CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp, k_in, k_out, i_in, i_out, (int)nch, 0, 32, st));
-    void* t = cv.take<char>(tmp);
-    cost_kernel<NC, R><<<(unsigned)((nch + 127) / 128), 128, 0, st>>>(a, k_in, i_in);
-    CUDA_TRY(cudaGetLastError());
-    CUDA_TRY(cub::DeviceRadixSort::SortPairs(t, tmp, k_in, k_out, i_in, i_out, (int)nch, 0, 32, st));
-    a.order = i_out;
-    return BMC_OK;
-}
-
 // scratch bytes order_chains carves for n chains
 size_t order_bytes(long long nch) {
     size_t tmp = 0;
@@ -441,340 +304,7 @@ size_t order_bytes(long long nch) {
     return 4 * align256(sizeof(float) * nch) + align256(tmp) + 1024;
 }
 
-// tangents per launch, by pool count (register budget of the dual-number state)
-template <int NC>
-constexpr int tangents_per_pass() { return NC <= 1 ? 2 : 1; }
-
-template <int NC, bool U = false>
-bmc_status run_tangents(ChainArgs a, int P, const TaylorTable* tt, cudaStream_t st) {
-    constexpr int TP = tangents_per_pass<NC>();
-    for (int t0 = 0; t0 < P; t0 += TP) {
-        a.t0 = t0;
-        bmc_status s = (P - t0 >= 2 && TP >= 2) ? launch_chain<NC, double, (TP >= 2 ? 2 : 1), U>(a, tt, st)
-                                                : launch_chain<NC, double, 1, U>(a, tt, st);
-        if (s != BMC_OK) return s;
-    }
-    return BMC_OK;
-}
-
-// An uneven batch: voxels with their own event tables, one pool count. Owns its device buffers
-// (preprocessed records of every table, the chain map, the sort scratch); built by bmc_uneven_create.
-struct UnevenPlan {
-    int dev = 0, n_cest = 0, n_vox = 0, mz = 0, reset = 1, n_tables = 0;
-    long long n_chains = 0, n_rec = 0;
-    EvRec<double>* rec = nullptr;
-    int2* chain_map = nullptr;
-    int* vox_table = nullptr;
-    long long* tab_base = nullptr;
-    int* tab_noff = nullptr;
-    int* tab_nev = nullptr;
-    int4* seg = nullptr;       // the repeated block of every row of every table
-    int* tab_row0 = nullptr;   // first row of each table in seg
-    double dense_switch = 0.0; // > 0: the dense path's norm threshold for this plan (bmc_uneven_set_dense_switch)
-    int4* adj_blk = nullptr;   // per row: the block the adjoint block kernel takes (adjoint_block_rows_kernel)
-    int adj_ok = 0;            // every row of every table qualifies: tangents go through that kernel
-    void* scratch = nullptr;   // sort keys and indices, cub scratch, status word
-    size_t scratch_bytes = 0;
-};
-
-template <int NC>
-struct Impl {
-    static constexpr int N = Layout<NC>::N;
-
-    // one simulation (or tangent set) of an uneven batch: chains sorted by estimated cost, outputs
-    // in canonical chain order (voxel-major, then table row)
-    static bmc_status uneven(const UnevenPlan& pl, const double* params, const double* m0, const bmc_spread* sp,
-                             const bmc_tangents* tg, const int32_t* active, double* z, double* jz, cudaStream_t st) {
-        const TaylorTable* tt = nullptr;
-        bmc_status s = tables(BMC_F64, &tt);
-        if (s != BMC_OK) return s;
-        ChainArgs a{};
-        a.n_vox = pl.n_vox; a.n_off = 1; a.n_ev = 0; a.n_fields = Layout<NC>::NF;
-        a.mz = pl.mz; a.reset_after_adc = pl.reset;
-        if ((s = fill_spread(a, sp)) != BMC_OK) return s;
-        a.params = params; a.m0 = m0; a.out = z; a.jout = jz;
-        a.ev = pl.rec;
-        a.n_chains = pl.n_chains; a.chain_map = pl.chain_map; a.vox_table = pl.vox_table;
-        a.tab_base = pl.tab_base; a.tab_noff = pl.tab_noff; a.tab_nev = pl.tab_nev;
-        a.seg = pl.seg; a.tab_row0 = pl.tab_row0; a.active = active; a.dense_switch = pl.dense_switch;
-        Carve cv(pl.scratch);
-        a.status = cv.take<int>(1);
-        CUDA_TRY(cudaMemsetAsync(a.status, 0, sizeof(int), st));
-        const long long nch = pl.n_chains;
-        if (nch >= 2 * 128) {
-            float* k_in = cv.take<float>(nch);
-            float* k_out = cv.take<float>(nch);
-            int* i_in = cv.take<int>(nch);
-            int* i_out = cv.take<int>(nch);
-            size_t tmp = 0;
-            CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp, k_in, k_out, i_in, i_out, (int)nch, 0, 32, st));
-            void* t = cv.take<char>(tmp);
-            if (cv.used > pl.scratch_bytes) return fail(BMC_ERR_INVALID, "uneven plan: scratch too small");
-            cost_kernel<NC, double, true><<<(unsigned)((nch + 127) / 128), 128, 0, st>>>(a, k_in, i_in);
-            CUDA_TRY(cudaGetLastError());
-            CUDA_TRY(cub::DeviceRadixSort::SortPairs(t, tmp, k_in, k_out, i_in, i_out, (int)nch, 0, 32, st));
-            a.order = i_out;
-        }
-        // the plan's primal passes: the block kernel's layout without tangents where its rows qualify
-        // (forward mode keeps the chain kernel for them too)
-        const bool adj = pl.adj_ok && g_tangent_mode.load(std::memory_order_relaxed) == BMC_TANGENTS_AUTO;
-        if (!tg) return adj ? launch_adjoint_block<NC, false>(a, pl.adj_blk, 0, tt, st)
-                            : launch_chain<NC, double, 0, true>(a, tt, st);
-        for (int t = 0; t < tg->n_tangents; ++t) a.field_row[t] = tg->field_row[t];
-        a.seed = tg->d_seed;
-        a.dm0 = tg->d_dm0;
-        if (adj && tg->n_tangents >= 2) return launch_adjoint_block<NC, true>(a, pl.adj_blk, tg->n_tangents, tt, st);
-        return run_tangents<NC, true>(a, tg->n_tangents, tt, st);
-    }
-
-    static bmc_status simulate(const bmc_problem* pr, const double* params, const bmc_events* ev, const double* m0,
-                               const bmc_spread* sp, double* out, cudaStream_t st, unsigned long long* work = nullptr) {
-        const TaylorTable* tt = nullptr;
-        bmc_status s = tables(pr->precision, &tt);
-        if (s != BMC_OK) return s;
-        const size_t nrec = (size_t)pr->n_offsets * pr->n_events;
-        void* ws = nullptr;
-        const size_t recb = pr->precision == BMC_F32 ? sizeof(EvRec<float>) : sizeof(EvRec<double>);
-        const long long nch = (long long)pr->n_voxels * pr->n_offsets;
-        if ((s = workspace(align256(nrec * recb) + 256 + align256(sizeof(int4) * pr->n_offsets) + order_bytes(nch), st,
-                           &ws)) != BMC_OK)
-            return s;
-        Carve cv(ws);
-        ChainArgs a{};
-        a.n_vox = pr->n_voxels; a.n_off = pr->n_offsets; a.n_ev = pr->n_events; a.n_fields = Layout<NC>::NF;
-        a.mz = pr->mz_loc; a.reset_after_adc = pr->reset_after_adc;
-        if ((s = fill_spread(a, sp)) != BMC_OK) return s;
-        a.params = params; a.m0 = m0; a.out = out; a.work = work;
-        a.status = cv.take<int>(1);
-        CUDA_TRY(cudaMemsetAsync(a.status, 0, sizeof(int), st));
-        if (pr->precision == BMC_F32) {
-            EvRec<float>* rec = cv.take<EvRec<float>>(nrec);
-            if ((s = prep_events<float>(pr, ev, rec, st)) != BMC_OK) return s;
-            a.ev = rec;
-            if ((s = order_chains<NC, float>(a, cv, st)) != BMC_OK) return s;
-            return launch_chain<NC, float, 0>(a, tt, st);
-        }
-        EvRec<double>* rec = cv.take<EvRec<double>>(nrec);
-        if ((s = prep_events<double>(pr, ev, rec, st)) != BMC_OK) return s;
-        a.ev = rec;
-        a.seg = cv.take<int4>(pr->n_offsets);
-        if ((s = scan_blocks(rec, pr->n_offsets, pr->n_events, pr->n_offsets, const_cast<int4*>(a.seg), st)) != BMC_OK)
-            return s;
-        if ((s = order_chains<NC, double>(a, cv, st)) != BMC_OK) return s;
-        return launch_chain<NC, double, 0>(a, tt, st);
-    }
-
-    static bmc_status trajectory(const bmc_problem* pr, const double* params, const bmc_events* ev,
-                                 const double* m0, double* traj, cudaStream_t st) {
-        const TaylorTable* tt = nullptr;
-        bmc_status s = tables(BMC_F64, &tt);
-        if (s != BMC_OK) return s;
-        const size_t nrec = (size_t)pr->n_offsets * pr->n_events;
-        void* ws = nullptr;
-        if ((s = workspace(align256(nrec * sizeof(EvRec<double>)) + 256 + align256(sizeof(double) * pr->n_voxels * pr->n_offsets), st, &ws)) != BMC_OK) return s;
-        Carve cv(ws);
-        ChainArgs a{};
-        a.n_vox = pr->n_voxels; a.n_off = pr->n_offsets; a.n_ev = pr->n_events; a.n_fields = Layout<NC>::NF;
-        a.mz = Layout<NC>::izw; a.reset_after_adc = pr->reset_after_adc;
-        fill_spread(a, nullptr);
-        a.params = params; a.m0 = m0; a.traj = traj;
-        a.status = cv.take<int>(1);
-        a.out = cv.take<double>((size_t)pr->n_voxels * pr->n_offsets);
-        CUDA_TRY(cudaMemsetAsync(a.status, 0, sizeof(int), st));
-        EvRec<double>* rec = cv.take<EvRec<double>>(nrec);
-        if ((s = prep_events<double>(pr, ev, rec, st)) != BMC_OK) return s;
-        a.ev = rec;
-        return launch_chain<NC, double, 0>(a, tt, st);
-    }
-
-    static bmc_status jvp(const bmc_problem* pr, const double* params, const bmc_events* ev, const double* m0,
-                          const bmc_spread* sp, const bmc_tangents* tg, double* z, double* jz, cudaStream_t st,
-                          unsigned long long* work = nullptr) {
-        const TaylorTable* tt = nullptr;
-        bmc_status s = tables(BMC_F64, &tt);
-        if (s != BMC_OK) return s;
-        const size_t nrec = (size_t)pr->n_offsets * pr->n_events;
-        void* ws = nullptr;
-        const long long nch = (long long)pr->n_voxels * pr->n_offsets;
-        if ((s = workspace(align256(nrec * sizeof(EvRec<double>)) + 256 + align256(sizeof(int4) * pr->n_offsets) +
-                               align256(sizeof(int) * pr->n_offsets) + 256 + order_bytes(nch), st, &ws)) != BMC_OK)
-            return s;
-        Carve cv(ws);
-        ChainArgs a{};
-        a.n_vox = pr->n_voxels; a.n_off = pr->n_offsets; a.n_ev = pr->n_events; a.n_fields = Layout<NC>::NF;
-        a.mz = pr->mz_loc; a.reset_after_adc = pr->reset_after_adc;
-        if ((s = fill_spread(a, sp)) != BMC_OK) return s;
-        a.params = params; a.m0 = m0; a.out = z; a.jout = jz; a.work = work;
-        for (int t = 0; t < tg->n_tangents; ++t) a.field_row[t] = tg->field_row[t];
-        a.seed = tg->d_seed; a.dm0 = tg->d_dm0;
-        a.status = cv.take<int>(1);
-        CUDA_TRY(cudaMemsetAsync(a.status, 0, sizeof(int), st));
-        EvRec<double>* rec = cv.take<EvRec<double>>(nrec);
-        if ((s = prep_events<double>(pr, ev, rec, st)) != BMC_OK) return s;
-        a.ev = rec;
-        a.seg = cv.take<int4>(pr->n_offsets);
-        if ((s = scan_blocks(rec, pr->n_offsets, pr->n_events, pr->n_offsets, const_cast<int4*>(a.seg), st)) != BMC_OK)
-            return s;
-        int* row_ev = cv.take<int>(pr->n_offsets);
-        int* flag = cv.take<int>(1);
-        bool adj = false;
-        if ((s = use_adjoint(rec, pr, tg->n_tangents, row_ev, flag, st, &adj)) != BMC_OK) return s;
-        if ((s = order_chains<NC, double>(a, cv, st)) != BMC_OK) return s;
-        if (adj) return launch_adjoint<NC>(a, row_ev, tg->n_tangents, tt, st);
-        return run_tangents<NC>(a, tg->n_tangents, tt, st);
-    }
-
-    // Z, its tangents and the derivatives of both along one design direction (design_kernel): one launch
-    // per tangent, the direction's records prepared beside the table's
-    static bmc_status design(const bmc_problem* pr, const double* params, const bmc_events* ev, const double* m0,
-                             const double* params_dir, const bmc_events* ev_dir, const double* m0_dir,
-                             const bmc_tangents* tg, double* z, double* jz, double* dz, double* djz, cudaStream_t st) {
-        const TaylorTable* tt = nullptr;
-        bmc_status s = tables(BMC_F64, &tt);
-        if (s != BMC_OK) return s;
-        const size_t nrec = (size_t)pr->n_offsets * pr->n_events;
-        const long long nch = (long long)pr->n_voxels * pr->n_offsets;
-        const size_t mats = (size_t)nch * (2 * N * N + N);           // Phi, its square, psi per chain
-        void* ws = nullptr;
-        if ((s = workspace(2 * align256(nrec * sizeof(EvRec<double>)) + 256 + align256(mats * sizeof(Dn<HD, 1>)),
-                           st, &ws)) != BMC_OK)
-            return s;
-        Carve cv(ws);
-        ChainArgs a{};
-        a.n_vox = pr->n_voxels; a.n_off = pr->n_offsets; a.n_ev = pr->n_events; a.n_fields = Layout<NC>::NF;
-        a.mz = pr->mz_loc; a.reset_after_adc = pr->reset_after_adc;
-        if ((s = fill_spread(a, nullptr)) != BMC_OK) return s;
-        a.params = params; a.params_dir = params_dir; a.m0 = m0; a.out = z; a.jout = jz;
-        for (int t = 0; t < tg->n_tangents; ++t) a.field_row[t] = tg->field_row[t];
-        a.seed = tg->d_seed;
-        a.status = cv.take<int>(1);
-        CUDA_TRY(cudaMemsetAsync(a.status, 0, sizeof(int), st));
-        EvRec<double>* rec = cv.take<EvRec<double>>(nrec);
-        if ((s = prep_events<double>(pr, ev, rec, st)) != BMC_OK) return s;
-        a.ev = rec;
-        DesignArgs d{};
-        if (ev_dir && nrec > 0) {
-            EvRec<double>* dr = cv.take<EvRec<double>>(nrec);
-            const int blocks = (int)std::min<size_t>((nrec + 255) / 256, 148 * 16);
-            prep_dir_kernel<<<blocks, 256, 0, st>>>(pr->n_offsets, pr->n_events, ev->d_rf_phase, ev_dir->d_dt,
-                                                   ev_dir->d_rf_amp, ev_dir->d_rf_phase, ev_dir->d_rf_freq, dr);
-            CUDA_TRY(cudaGetLastError());
-            d.ev_dir = dr;
-        }
-        d.m0_dir = m0_dir; d.dz = dz; d.djz = djz;
-        d.scratch = reinterpret_cast<double*>(cv.take<Dn<HD, 1>>(mats));
-        const long long blocks = (nch + 127) / 128;
-        if (blocks > 0x7fffffffLL) return fail(BMC_ERR_INVALID, "%lld chains exceed one launch", nch);
-        for (int t = 0; t < tg->n_tangents; ++t) {
-            a.t0 = t;
-            design_kernel<NC, 1><<<(unsigned)blocks, 128, 0, st>>>(a, d, tt);
-            CUDA_TRY(cudaGetLastError());
-        }
-        return BMC_OK;
-    }
-
-    static bmc_status lm(const bmc_problem* pr, const double* params, const bmc_events* ev, const double* m0,
-                         const bmc_spread* sp, const bmc_fit_spec* fs, const double* zm, const double* x0,
-                         double* x_out, double* cost_traj, double* x_traj, cudaStream_t st) {
-        const TaylorTable* tt = nullptr;
-        bmc_status s = tables(BMC_F64, &tt);
-        if (s != BMC_OK) return s;
-        const int nv = pr->n_voxels, no = pr->n_offsets, P = fs->n_params;
-        constexpr int NF = Layout<NC>::NF;
-        const size_t nrec = (size_t)no * pr->n_events;
-        const size_t bytes = align256(nrec * sizeof(EvRec<double>)) + 2 * align256(sizeof(double) * NF * nv) +
-                             2 * align256(sizeof(double) * N * nv) + 2 * align256(sizeof(double) * nv) +
-                             align256(sizeof(double) * P * nv) + align256(sizeof(double) * P * nv * N) +
-                             2 * align256(sizeof(double) * nv * no) + align256(sizeof(double) * P * nv * no) +
-                             2 * align256(sizeof(double) * nv * P) + 2 * align256(sizeof(double) * nv) +
-                             align256(sizeof(int) * nv) + align256(sizeof(int4) * no) + 4096 +
-                             align256(sizeof(int) * no) + 256 + order_bytes((long long)nv * no);
-        void* ws = nullptr;
-        if ((s = workspace(bytes, st, &ws)) != BMC_OK) return s;
-        Carve cv(ws);
-        EvRec<double>* rec = cv.take<EvRec<double>>(nrec);
-        double* px = cv.take<double>((size_t)NF * nv);
-        double* pt = cv.take<double>((size_t)NF * nv);
-        double* m0x = cv.take<double>((size_t)N * nv);
-        double* m0t = cv.take<double>((size_t)N * nv);
-        double* sgx = cv.take<double>(nv);
-        double* sgt = cv.take<double>(nv);
-        double* seed = cv.take<double>((size_t)P * nv);
-        double* dm0 = cv.take<double>((size_t)P * nv * N);
-        double* z = cv.take<double>((size_t)nv * no);
-        double* zt = cv.take<double>((size_t)nv * no);
-        double* J = cv.take<double>((size_t)P * nv * no);
-        double* x = cv.take<double>((size_t)nv * P);
-        double* xt = cv.take<double>((size_t)nv * P);
-        double* lam = cv.take<double>(nv);
-        double* cost = cv.take<double>(nv);
-        int* need = cv.take<int>(nv);
-        int4* seg = cv.take<int4>(no);
-        int* status = cv.take<int>(1);
-        int* row_ev = cv.take<int>(no);
-        int* flag = cv.take<int>(1);
-        if ((s = prep_events<double>(pr, ev, rec, st)) != BMC_OK) return s;
-        CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), st));
-        CUDA_TRY(cudaMemcpyAsync(x, x0, sizeof(double) * nv * P, cudaMemcpyDeviceToDevice, st));
-        std::vector<double> hl(nv, fs->lam0);
-        std::vector<int> hn(nv, 1);
-        CUDA_TRY(cudaMemcpyAsync(lam, hl.data(), sizeof(double) * nv, cudaMemcpyHostToDevice, st));
-        CUDA_TRY(cudaMemcpyAsync(need, hn.data(), sizeof(int) * nv, cudaMemcpyHostToDevice, st));
-
-        SlotSpec ss{};
-        ss.P = P;
-        bool has_m = false;
-        for (int p = 0; p < P; ++p) {
-            ss.field_row[p] = fs->field_row[p]; ss.mode[p] = fs->mode[p]; ss.scale[p] = fs->scale[p];
-            ss.lo[p] = fs->lo[p]; ss.hi[p] = fs->hi[p];
-            has_m = has_m || fs->field_row[p] == BMC_SLOT_M_START;
-        }
-        ChainArgs a{};
-        a.n_vox = nv; a.n_off = no; a.n_ev = pr->n_events; a.n_fields = NF;
-        a.mz = pr->mz_loc; a.reset_after_adc = pr->reset_after_adc;
-        if ((s = fill_spread(a, sp)) != BMC_OK) return s;
-        const double* sig0 = sp ? sp->d_sigma_hz : nullptr;
-        a.ev = rec; a.status = status; a.seg = seg;
-        if ((s = scan_blocks(rec, no, pr->n_events, no, seg, st)) != BMC_OK) return s;
-        bool adj = false;
-        if ((s = use_adjoint(rec, pr, P, row_ev, flag, st, &adj)) != BMC_OK) return s;
-        a.params = params; a.m0 = m0;
-        if ((s = order_chains<NC, double>(a, cv, st)) != BMC_OK) return s;
-        for (int p = 0; p < P; ++p) a.field_row[p] = fs->field_row[p] == BMC_SLOT_M_START ? BMC_SEED_NONE : fs->field_row[p];
-        const int vb = (nv + 127) / 128, wb = (nv + 3) / 4;
-        for (int it = 0; it < fs->n_iter; ++it) {
-            // residual and Jacobian at x, for the voxels whose x moved
-            lm_params_kernel<NC><<<vb, 128, 0, st>>>(nv, ss, params, m0, sig0, x, fs->d_free, px, m0x,
-                                                      sp ? sgx : nullptr, seed, has_m ? dm0 : nullptr);
-            CUDA_TRY(cudaGetLastError());
-            ChainArgs aj = a;
-            aj.params = px; aj.m0 = m0x; aj.sigma = sp ? sgx : nullptr; aj.seed = seed; aj.dm0 = has_m ? dm0 : nullptr;
-            aj.active = need; aj.out = z; aj.jout = J;
-            if ((s = adj ? launch_adjoint<NC>(aj, row_ev, P, tt, st) : run_tangents<NC>(aj, P, tt, st)) != BMC_OK)
-                return s;
-            lm_solve_kernel<<<wb, 128, 0, st>>>(nv, no, fs->n_points_skip, ss, z, zm, J, fs->d_free, x, lam, cost, xt);
-            CUDA_TRY(cudaGetLastError());
-            // the trial point
-            lm_params_kernel<NC><<<vb, 128, 0, st>>>(nv, ss, params, m0, sig0, xt, fs->d_free, pt, m0t,
-                                                      sp ? sgt : nullptr, nullptr, nullptr);
-            CUDA_TRY(cudaGetLastError());
-            ChainArgs at = a;
-            at.params = pt; at.m0 = m0t; at.sigma = sp ? sgt : nullptr; at.out = zt;
-            // the trial point's Z: with the adjoint tangents, the same dense layout without H
-            if ((s = adj ? launch_adjoint<NC, false>(at, row_ev, 0, tt, st) : launch_chain<NC, double, 0>(at, tt, st)) !=
-                BMC_OK)
-                return s;
-            lm_accept_kernel<<<wb, 128, 0, st>>>(nv, no, fs->n_points_skip, P, it, fs->n_iter, zt, zm, cost, xt, x,
-                                                 lam, need, cost_traj, x_traj);
-            CUDA_TRY(cudaGetLastError());
-        }
-        CUDA_TRY(cudaMemcpyAsync(x_out, x, sizeof(double) * nv * P, cudaMemcpyDeviceToDevice, st));
-        return BMC_OK;
-    }
-};
-
-
-}  // namespace
+}  // namespace bmc
 
 // ------------------------------------------------------------------------------------------------
 // exported entry points
@@ -1254,40 +784,6 @@ bmc_status noalloc_setup(int precision, void** scratch, const TaylorTable** tt) 
     return BMC_OK;
 }
 
-template <int NC>
-struct NoAlloc {
-    template <typename R>
-    static bmc_status run(const bmc_problem* pr, const double* params, const bmc_events* ev, const double* m0,
-                          const bmc_spread* sp, double* out, void* scratch, const TaylorTable* tt, cudaStream_t st) {
-        ChainArgs a{};
-        a.n_vox = pr->n_voxels; a.n_off = pr->n_offsets; a.n_ev = pr->n_events; a.n_fields = Layout<NC>::NF;
-        a.mz = pr->mz_loc; a.reset_after_adc = pr->reset_after_adc;
-        bmc_status s = fill_spread(a, sp);
-        if (s != BMC_OK) return s;
-        a.params = params; a.m0 = m0; a.out = out;
-        a.status = static_cast<int*>(scratch);
-        CUDA_TRY(cudaMemsetAsync(a.status, 0, sizeof(int), st));          // must start at zero each call
-        // the scratch: the status word, every row's repeated block, the event records
-        int4* seg = reinterpret_cast<int4*>(static_cast<char*>(scratch) + kNoAllocStatusBytes);
-        EvRec<R>* rec = reinterpret_cast<EvRec<R>*>(static_cast<char*>(scratch) + kNoAllocStatusBytes +
-                                                    noalloc_seg_bytes(pr->n_offsets));
-        if ((s = prep_events<R>(pr, ev, rec, st)) != BMC_OK) return s;   // overwrites the previous call's
-        a.ev = rec;
-        if constexpr (std::is_same<R, double>::value) {
-            if ((s = scan_blocks(rec, pr->n_offsets, pr->n_events, pr->n_offsets, seg, st)) != BMC_OK) return s;
-            a.seg = seg;
-        }
-        return launch_chain<NC, R, 0>(a, tt, st);
-    }
-
-    static bmc_status simulate(const bmc_problem* pr, const double* params, const bmc_events* ev, const double* m0,
-                               const bmc_spread* sp, double* out, void* scratch, const TaylorTable* tt,
-                               cudaStream_t st) {
-        return pr->precision == BMC_F32 ? run<float>(pr, params, ev, m0, sp, out, scratch, tt, st)
-                                        : run<double>(pr, params, ev, m0, sp, out, scratch, tt, st);
-    }
-};
-
 }  // namespace
 
 extern "C" bmc_status bmc_simulate_noalloc(const bmc_problem* prob, const double* d_params, const bmc_events* ev,
@@ -1309,13 +805,8 @@ extern "C" bmc_status bmc_simulate_noalloc(const bmc_problem* prob, const double
     const TaylorTable* tt = nullptr;
     if ((s = noalloc_setup(prob->precision, &scratch, &tt)) != BMC_OK) return s;
     const cudaStream_t st = (cudaStream_t)stream;
-    switch (prob->n_cest) {
-        case 0: return NoAlloc<0>::simulate(prob, d_params, ev, d_m0, spread, d_out, scratch, tt, st);
-        case 1: return NoAlloc<1>::simulate(prob, d_params, ev, d_m0, spread, d_out, scratch, tt, st);
-        case 2: return NoAlloc<2>::simulate(prob, d_params, ev, d_m0, spread, d_out, scratch, tt, st);
-        case 3: return NoAlloc<3>::simulate(prob, d_params, ev, d_m0, spread, d_out, scratch, tt, st);
-        case 4: return NoAlloc<4>::simulate(prob, d_params, ev, d_m0, spread, d_out, scratch, tt, st);
-        case 5: return NoAlloc<5>::simulate(prob, d_params, ev, d_m0, spread, d_out, scratch, tt, st);
-        default: return fail(BMC_ERR_UNSUPPORTED, "n_cest %d", prob->n_cest);
-    }
+    char* base = static_cast<char*>(scratch);
+    const NoAllocScratch ws{reinterpret_cast<int*>(base), reinterpret_cast<int4*>(base + kNoAllocStatusBytes),
+                            base + fixed};
+    BMC_DISPATCH(prob->n_cest, noalloc(prob, d_params, ev, d_m0, spread, d_out, ws, tt, st));
 }

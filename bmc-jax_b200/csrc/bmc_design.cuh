@@ -29,7 +29,7 @@ struct DesignArgs {
 
 // the design direction of an event table as records: [n_ev][n_off] from the reference layout [n_off][n_ev]
 // (d(dt), 2 pi d(rf_amp), -sin(phase) d(phase), cos(phase) d(phase), 2 pi d(rf_freq)); null arrays are 0
-__global__ void prep_dir_kernel(int n_off, int n_ev, const double* __restrict__ phase, const double* __restrict__ ddt,
+static __global__ void prep_dir_kernel(int n_off, int n_ev, const double* __restrict__ phase, const double* __restrict__ ddt,
                                 const double* __restrict__ damp, const double* __restrict__ dphase,
                                 const double* __restrict__ dfreq, EvRec<double>* __restrict__ out) {
     const size_t n = (size_t)n_off * n_ev;

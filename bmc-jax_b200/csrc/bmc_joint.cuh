@@ -16,7 +16,7 @@ constexpr int kMaxJointP = 9;  // local values + the shared one
 
 // per sample v: H[v] = sum over its chains c of J[:, c] J[:, c]^T, g[v] = J r, cost[v] = r^T r;
 // chains of sample v are seg[v] .. seg[v+1]-1 of the canonical order; J is [P][n_chains]
-__global__ void normal_segments_kernel(int n_vox, int P, long long n_chains, const long long* __restrict__ seg,
+static __global__ void normal_segments_kernel(int n_vox, int P, long long n_chains, const long long* __restrict__ seg,
                                        const double* __restrict__ J, const double* __restrict__ r,
                                        double* __restrict__ H, double* __restrict__ g, double* __restrict__ cost) {
     const int warp = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
@@ -172,7 +172,7 @@ __host__ __device__ inline void schur_eliminate_one(int v, int n_vox, int PL, in
     red[3 * (size_t)n_vox + v] = S ? gv[PL] : 0.0;
 }
 
-__global__ void schur_eliminate_kernel(int n_vox, int PL, int S, const double* __restrict__ H,
+static __global__ void schur_eliminate_kernel(int n_vox, int PL, int S, const double* __restrict__ H,
                                        const double* __restrict__ g, const double* __restrict__ free, double lam,
                                        const double* __restrict__ d_lam,
                                        double* __restrict__ Y, double* __restrict__ w, double* __restrict__ red) {
@@ -182,7 +182,7 @@ __global__ void schur_eliminate_kernel(int n_vox, int PL, int S, const double* _
 
 // one block: the four Schur sums of a batch -- sum h_ss, sum h_ps^T Y, sum h_ps^T w, sum g_s -- in a
 // fixed order (deterministic); a sharded fit adds the batches' sums across ranks before the shared step
-__global__ void schur_sum_kernel(int n_vox, const double* __restrict__ red, double* __restrict__ sums) {
+static __global__ void schur_sum_kernel(int n_vox, const double* __restrict__ red, double* __restrict__ sums) {
     __shared__ double sm[4][1024];
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
     for (int v = threadIdx.x; v < n_vox; v += blockDim.x)
@@ -201,7 +201,7 @@ __global__ void schur_sum_kernel(int n_vox, const double* __restrict__ red, doub
 }
 
 // the shared step ds = -(sum g_s - sum h_ps^T w) / (H_ss + lam (H_ss + 1e-9) - sum h_ps^T Y), H_ss = sum h_ss
-__global__ void schur_shared_kernel(int S, const double* __restrict__ sums, double lam_in,
+static __global__ void schur_shared_kernel(int S, const double* __restrict__ sums, double lam_in,
                                     const double* __restrict__ d_lam, double* __restrict__ ds) {
     const double lam = d_lam ? *d_lam : lam_in;
     if (threadIdx.x == 0) {
@@ -211,7 +211,7 @@ __global__ void schur_shared_kernel(int S, const double* __restrict__ sums, doub
 }
 
 // d_p = -(w + Y ds) per sample
-__global__ void schur_back_kernel(int n_vox, int PL, const double* __restrict__ Y, const double* __restrict__ w,
+static __global__ void schur_back_kernel(int n_vox, int PL, const double* __restrict__ Y, const double* __restrict__ w,
                                   const double* __restrict__ ds, double* __restrict__ d) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= (long long)n_vox * PL) return;

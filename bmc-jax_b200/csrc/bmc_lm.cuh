@@ -155,7 +155,7 @@ __device__ __forceinline__ void gauss_solve(int P, double* A, double* b) {
 }
 
 // normal equations, the damped solve and the clipped trial point
-__global__ void lm_solve_kernel(int n_vox, int n_off, int skip, const SlotSpec sp, const double* __restrict__ z,
+static __global__ void lm_solve_kernel(int n_vox, int n_off, int skip, const SlotSpec sp, const double* __restrict__ z,
                                 const double* __restrict__ zm, const double* __restrict__ J,
                                 const double* __restrict__ freem, const double* __restrict__ x,
                                 const double* __restrict__ lam, double* __restrict__ cost, double* __restrict__ xt) {
@@ -185,7 +185,7 @@ __global__ void lm_solve_kernel(int n_vox, int n_off, int skip, const SlotSpec s
 }
 
 // accept or reject every voxel's trial point
-__global__ void lm_accept_kernel(int n_vox, int n_off, int skip, int P, int it, int n_iter,
+static __global__ void lm_accept_kernel(int n_vox, int n_off, int skip, int P, int it, int n_iter,
                                  const double* __restrict__ zt, const double* __restrict__ zm,
                                  const double* __restrict__ cost, const double* __restrict__ xt,
                                  double* __restrict__ x, double* __restrict__ lam, int* __restrict__ need,
@@ -215,7 +215,7 @@ __global__ void lm_accept_kernel(int n_vox, int n_off, int skip, int P, int it, 
 }
 
 // per-sample H, g, c for a coupled joint fit
-__global__ void normal_blocks_kernel(int n_vox, int n_pts, int P, const double* __restrict__ r,
+static __global__ void normal_blocks_kernel(int n_vox, int n_pts, int P, const double* __restrict__ r,
                                      const double* __restrict__ J, double* __restrict__ Hout,
                                      double* __restrict__ gout, double* __restrict__ cout) {
     const int lane = threadIdx.x & 31;
