@@ -186,7 +186,7 @@ struct GemmArgs {
     int ldo;
     float* out2;        // OUT: caller's y [m_valid2][n_valid2]
     int ld2, m_valid2, n_valid2;
-    float* dbias;       // DHIDDEN: column sums of dz (atomics) [N]
+    float* dbias;       // DW: row sums of A, the bias gradient (atomics) [m_valid]; may be null
     int* status;
 };
 
@@ -259,10 +259,7 @@ __device__ __forceinline__ void epilogue(const GemmArgs& g, int row, int n, floa
             for (int i = 0; i < 16; ++i) dz[i] = 0.0f;
         }
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            db[i] = __float2bfloat16_rn(dz[i]);
-            dz[i] = __bfloat162float(db[i]);  // the bias gradient sums what the weight gradient sees
-        }
+        for (int i = 0; i < 16; ++i) db[i] = __float2bfloat16_rn(dz[i]);
         if (live) {
             uint4* h4 = reinterpret_cast<uint4*>(g.h + size_t(row) * g.ldh + n);
             h4[0] = reinterpret_cast<const uint4*>(db)[0];
@@ -271,14 +268,6 @@ __device__ __forceinline__ void epilogue(const GemmArgs& g, int row, int n, floa
 #pragma unroll
                 for (int i = 0; i < 16; ++i) g.ht[size_t(n + i) * g.ldht + row] = db[i];
             }
-        }
-        // column sums over the warp's 32 rows, one atomic per column
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            float s = dz[i];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if ((threadIdx.x & 31) == 0 && g.dbias) atomicAdd(g.dbias + n + i, s);
         }
     } else {  // EPI_DW
         if (live) {
@@ -328,12 +317,15 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_kernel(GemmArgs g) {
 
     auto load = [&](int stage, int k0) {
         const uint32_t a = s0 + stage * S::STAGE, b = a + S::A_BYTES;
+        // eight neighbouring threads take the eight rows of one core matrix, 128 contiguous bytes of shared memory (a
+        // row's chunks lie 128 bytes apart there, so threads along a row would all write the same banks); a warp
+        // reads 64 bytes of each of its rows
         for (int i = tid; i < 128 * 8; i += kGemmThreads) {
-            const int r = i >> 3, c = i & 7;
+            const int r = (i >> 6) * 8 + (i & 7), c = (i >> 3) & 7;
             cp_async16(a + (r >> 3) * 1024 + c * 128 + (r & 7) * 16, g.A + size_t(m0 + r) * g.lda + k0 + c * 8);
         }
         for (int i = tid; i < BN * 8; i += kGemmThreads) {
-            const int r = i >> 3, c = i & 7;
+            const int r = (i >> 6) * 8 + (i & 7), c = (i >> 3) & 7;
             cp_async16(b + (r >> 3) * 1024 + c * 128 + (r & 7) * 16, g.B + size_t(n0 + r) * g.ldb + k0 + c * 8);
         }
         cp_async_commit();
@@ -345,6 +337,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_kernel(GemmArgs g) {
     int issued = 0;   // chunks whose loads were issued
     for (; issued < min(nk, kGemmStages); ++issued) load(issued, kb + issued * 64);
     int committed = -1;
+    [[maybe_unused]] float bias_sum = 0.0f;
     for (int c = 0; ok && c < nk; ++c) {
         const int st = c % kGemmStages;
         const int pending = issued - (c + 1);   // later chunks' load groups that may still be in flight
@@ -362,6 +355,25 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_kernel(GemmArgs g) {
             umma_commit(smem_addr(&bars[st]));
         }
         committed = c;
+        if constexpr (EPI == EPI_DW) {
+            // the bias gradient: the sums of A's rows (the rounded dz that the product sees), two threads a row, while
+            // the tensor core works on the chunk (column sums by shuffles in the epilogue that formed dz took 10 us
+            // of its 21 at 4,096 x 256)
+            if (g.dbias && blockIdx.y == 0) {
+                const int r = tid & 127;
+                const uint8_t* p = smem + st * S::STAGE + (r >> 3) * 1024 + (tid >> 7) * 512 + (r & 7) * 16;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const uint4 x = *reinterpret_cast<const uint4*>(p + q * 128);
+                    const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        bias_sum += __uint_as_float(w[i] << 16);
+                        bias_sum += __uint_as_float(w[i] & 0xffff0000u);
+                    }
+                }
+            }
+        }
         if (issued < nk) {
             // the stage is free once chunk c's MMAs are done
             const bool w = mbar_wait(smem_addr(&bars[st]), (c / kGemmStages) & 1);
@@ -382,6 +394,9 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_kernel(GemmArgs g) {
     cp_async_wait<0>();
     tc_fence_after();
 
+    if constexpr (EPI == EPI_DW) {
+        if (ok && g.dbias && blockIdx.y == 0 && m0 + (tid & 127) < g.m_valid) atomicAdd(g.dbias + m0 + (tid & 127), bias_sum);
+    }
     if (ok && nk > 0) {
         const int quarter = warp & 3, half = warp >> 2;
         const int row = m0 + quarter * 32 + lane;
@@ -425,29 +440,56 @@ __global__ void prep_input_kernel(const float* __restrict__ x, const float* __re
     }
 }
 
-// gradient of the mean squared error at the output: d = 2 (y - t) / (batch n_out), in bf16 (row and
-// transposed copies), its column sums into the output-bias gradient, and the loss into *loss
-__global__ void loss_kernel(const float* __restrict__ y, int ldy, const float* __restrict__ t, int batch, int n_out,
-                            int rows, int out_pad, bf16* __restrict__ d, bf16* __restrict__ dt,
-                            float* __restrict__ dbias, float* __restrict__ loss) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+// The same without the transposed copy, which only the backward pass reads: a thread per pair of columns, kPrepRows
+// rows of them, its shift and scale in registers (65,536 x 244: 51 us with the copy through shared memory).
+constexpr int kPrepRows = 8;
+__global__ void __launch_bounds__(128) prep_rows_kernel(const float* __restrict__ x, const float* __restrict__ shift,
+                                                        const float* __restrict__ scale, int batch, int n_in, int in_pad,
+                                                        bf16* __restrict__ X) {
+    const int i = 2 * (blockIdx.x * 128 + threadIdx.x), m0 = blockIdx.y * kPrepRows;
+    if (i >= in_pad) return;
+    const bool a = i < n_in, b = i + 1 < n_in;
+    const float s0 = a && shift ? shift[i] : 0.0f, s1 = b && shift ? shift[i + 1] : 0.0f;
+    const float c0 = a && scale ? scale[i] : 1.0f, c1 = b && scale ? scale[i + 1] : 1.0f;
+    float u[kPrepRows], v[kPrepRows];
+#pragma unroll
+    for (int r = 0; r < kPrepRows; ++r) {
+        const float* p = x + size_t(m0 + r) * n_in + i;
+        u[r] = a && m0 + r < batch ? (p[0] - s0) * c0 : 0.0f;
+        v[r] = b && m0 + r < batch ? (p[1] - s1) * c1 : 0.0f;
+    }
+#pragma unroll
+    for (int r = 0; r < kPrepRows; ++r)
+        *reinterpret_cast<__nv_bfloat162*>(X + size_t(m0 + r) * in_pad + i) =
+            __halves2bfloat162(__float2bfloat16_rn(u[r]), __float2bfloat16_rn(v[r]));
+}
+
+// gradient of the mean squared error at the output: d = 2 (y - t) / (batch n_out), in bf16 (row and transposed
+// copies; dt's padding rows are zero already), and the loss into *loss. A thread per row: the n_out real columns of
+// a row are few, the rest of the row is 16-byte stores of zeros.
+__global__ void __launch_bounds__(64) loss_kernel(const float* __restrict__ y, int ldy, const float* __restrict__ t,
+                                                  int batch, int n_out, int rows, int out_pad, bf16* __restrict__ d,
+                                                  bf16* __restrict__ dt, float* __restrict__ loss) {
+    const int m = blockIdx.x * 64 + threadIdx.x;
     const float inv = 1.0f / (float(batch) * float(n_out));
     float lsum = 0.0f;
-    for (int j = 0; j < out_pad; ++j) {
-        float g = 0.0f;
-        if (m < batch && j < n_out) {
-            const float e = y[size_t(m) * ldy + j] - t[size_t(m) * n_out + j];
-            lsum += e * e * inv;
-            g = 2.0f * e * inv;
+    if (m < rows) {
+        for (int j0 = 0; j0 < out_pad; j0 += 8) {
+            __align__(16) bf16 gb[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                float g = 0.0f;
+                const int j = j0 + i;
+                if (m < batch && j < n_out) {
+                    const float e = y[size_t(m) * ldy + j] - t[size_t(m) * n_out + j];
+                    lsum += e * e * inv;
+                    g = 2.0f * e * inv;
+                }
+                gb[i] = __float2bfloat16_rn(g);
+                if (j < n_out) dt[size_t(j) * rows + m] = gb[i];
+            }
+            *reinterpret_cast<uint4*>(d + size_t(m) * out_pad + j0) = *reinterpret_cast<const uint4*>(gb);
         }
-        const bf16 gb = __float2bfloat16_rn(g);
-        if (m < rows) {
-            d[size_t(m) * out_pad + j] = gb;
-            dt[size_t(j) * rows + m] = gb;
-        }
-        float s = __bfloat162float(gb);
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if ((threadIdx.x & 31) == 0 && j < n_out && s != 0.0f) atomicAdd(dbias + j, s);
     }
     for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
     if ((threadIdx.x & 31) == 0 && loss) atomicAdd(loss, lsum);
@@ -670,7 +712,17 @@ bmc_status forward_impl(const Shape& s, const float* params, const bf16* shadow,
                         const float* scale, long long batch, float* y, const Work& w, bool keep,
                         cudaStream_t st) {
     const LayerMap M = layer_map(s);
-    {
+    if (!keep) {
+        // (w.rows is a multiple of 128)
+        for (long long r0 = 0; r0 < w.rows; r0 += 65535ll * kPrepRows) {
+            const long long n = std::min<long long>(w.rows - r0, 65535ll * kPrepRows);
+            dim3 grid(unsigned((s.in_pad + 255) / 256), unsigned(n / kPrepRows));
+            prep_rows_kernel<<<grid, 128, 0, st>>>(x + r0 * s.n_in, shift, scale,
+                                                   int(std::max<long long>(0, std::min<long long>(batch - r0, n))), s.n_in,
+                                                   s.in_pad, w.X + r0 * s.in_pad);
+            MLP_CUDA_TRY(cudaGetLastError());
+        }
+    } else {
         dim3 grid(unsigned(rup(s.in_pad, 32) / 32), unsigned(w.rows / 32));
         prep_input_kernel<<<grid, dim3(32, 8), 0, st>>>(x, shift, scale, int(batch), s.n_in, w.rows, s.in_pad,
                                                          w.X, w.XT);
@@ -727,8 +779,8 @@ bmc_status backward_impl(const Shape& s, const bf16* shadow, const float* target
     MLP_CUDA_TRY(cudaMemsetAsync(grad, 0, size_t(n_params(s)) * sizeof(float), st));
     MLP_CUDA_TRY(cudaMemsetAsync(w.dOT, 0, size_t(w.dot_rows) * w.rows * 2, st));
     const int lo = s.L;  // output layer index
-    loss_kernel<<<unsigned(w.rows / 128), 128, 0, st>>>(w.Y, s.out_pad, target, int(batch), s.n_out, w.rows,
-                                                         s.out_pad, w.dO, w.dOT, grad + M.off_b[lo], loss);
+    loss_kernel<<<unsigned(w.rows / 64), 64, 0, st>>>(w.Y, s.out_pad, target, int(batch), s.n_out, w.rows, s.out_pad,
+                                                      w.dO, w.dOT, loss);
     MLP_CUDA_TRY(cudaGetLastError());
     // output layer weight gradient: dW_o = dO^T H_L   (rows of dO^T padded to 128; rows >= out_pad not stored)
     {
@@ -743,6 +795,7 @@ bmc_status backward_impl(const Shape& s, const bf16* shadow, const float* target
         g.m_valid = s.out_pad;
         g.out = grad + M.off_w[lo];
         g.ldo = s.H;
+        g.dbias = grad + M.off_b[lo];
         g.status = w.status;
         if (bmc_status e = gemm<EPI_DW>(g, dw_splits(g.M, g.N, g.K), st)) return e;
     }
@@ -767,7 +820,6 @@ bmc_status backward_impl(const Shape& s, const bf16* shadow, const float* target
         g.ldh = s.H;
         g.ht = nxtT;
         g.ldht = w.rows;
-        g.dbias = grad + M.off_b[l - 1];
         g.status = w.status;
         if (bmc_status e = gemm<EPI_DHIDDEN>(g, 1, st)) return e;
         // weight gradient of layer l-1: dW = dZ^T (input of layer l-1)
@@ -782,6 +834,7 @@ bmc_status backward_impl(const Shape& s, const bf16* shadow, const float* target
         d.m_valid = s.H;
         d.out = grad + M.off_w[l - 1];
         d.ldo = M.cols[l - 1];
+        d.dbias = grad + M.off_b[l - 1];
         d.status = w.status;
         if (bmc_status e = gemm<EPI_DW>(d, dw_splits(d.M, d.N, d.K), st)) return e;
         dcur = nxt;
