@@ -94,24 +94,31 @@ __device__ __forceinline__ double group_sum(double x) {
 // when a row is not such a row.
 static __global__ void adjoint_rows_kernel(const EvRec<double>* __restrict__ rec, int n_off, int n_ev, int reset_after_adc,
                                     int* __restrict__ row_ev, int* __restrict__ all_ok) {
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
+    const int o = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;   // a warp per row
     if (o >= n_off) return;
-    int e_star = -1, moving = 0;
+    unsigned moving = 0, last = 0, first = 0x7fffffffu, adc = 0;   // last, adc: index + 1, 0 = none
     bool ok = true;
-    for (int e = 0; e < n_ev; ++e) {
+    for (int e = lane; e < n_ev; e += 32) {
         const EvRec<double> r = rec[(size_t)e * n_off + o];
         const int type = (int)r.type;
         if (r.dt > 1e-9) {
             ++moving;
-            e_star = e;
+            last = e + 1;
+            first = min(first, (unsigned)e);
             ok = ok && (type == EV_RF || type == EV_DELAY);
         } else {
             ok = ok && type != EV_GRADIENT && type != EV_SPOILER;
-            if (type == EV_ADC && moving > 0 && reset_after_adc && e + 1 < n_ev) ok = false;
+            if (type == EV_ADC && reset_after_adc && e + 1 < n_ev) adc = e + 1;
         }
     }
-    ok = ok && moving == 1;
-    row_ev[o] = ok ? e_star : -1;
+    moving = __reduce_add_sync(kFull, moving);
+    last = __reduce_max_sync(kFull, last);
+    first = __reduce_min_sync(kFull, first);
+    adc = __reduce_max_sync(kFull, adc);
+    // a readout that resets the state counts once the state has evolved
+    ok = __all_sync(kFull, ok) && moving == 1 && !(adc > 0 && first < adc - 1);
+    if (lane != 0) return;
+    row_ev[o] = ok ? (int)last - 1 : -1;
     if (!ok) atomicAnd(all_ok, 0);
 }
 
@@ -310,9 +317,10 @@ adjoint_kernel(const ChainArgs a, const int* __restrict__ row_ev, int n_tan, con
     const int lane = threadIdx.x & 31, grp = lane / GS, gl = lane % GS;
 
     const long long nch = (long long)a.n_vox * a.n_off;
-    long long ci = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = ci < nch;
-    if (!valid) ci = nch - 1;
+    const long long first = ((long long)blockIdx.x * kAdjWarps + (threadIdx.x >> 5)) * a.cpw;
+    long long ci = first + lane;
+    const bool valid = lane < a.cpw && ci < nch;
+    if (!valid) ci = first < nch ? first : nch - 1;
     if (a.order) ci = a.order[ci];
     const int v = (int)(ci / a.n_off), o = (int)(ci % a.n_off);
     const bool act = valid && (a.active == nullptr || a.active[v] != 0);

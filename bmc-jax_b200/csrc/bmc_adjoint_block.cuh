@@ -58,7 +58,7 @@ struct AdjBlkSlot : AdjBlkSlotBody<NC, kTan> {
 
 constexpr int kAdjBlkWarps = 4;
 
-// Rows the block kernel can take, one thread per row of one table: the evolving events (dt > 1e-9) are
+// Rows the block kernel can take, one warp per row of one table: the evolving events (dt > 1e-9) are
 // exactly the repeated block found by block_scan_kernel (seg), or, with no block, lie in one window of at
 // most kAdjL events taken once; the block's events are RF blocks or delays; no spoiler or gradient
 // anywhere; no readout that resets the state before the row ends. out[row] = (first, L, r, 1) or zero;
@@ -66,24 +66,31 @@ constexpr int kAdjBlkWarps = 4;
 static __global__ void adjoint_block_rows_kernel(const EvRec<double>* __restrict__ rec, int n_rows, int n_ev, int stride,
                                           const int4* __restrict__ seg, int reset_after_adc,
                                           int4* __restrict__ out, int* __restrict__ all_ok) {
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
+    const int o = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;   // a warp per row
     if (o >= n_rows) return;
     const int4 b = seg ? seg[o] : make_int4(0, 0, 0, 0);
-    int first = -1, last = -1, moving = 0;
+    unsigned moved = 0, end = 0, begin = 0x7fffffffu, adc = 0;   // end, adc: index + 1, 0 = none
     bool ok = true;
-    for (int e = 0; e < n_ev; ++e) {
+    for (int e = lane; e < n_ev; e += 32) {
         const EvRec<double> x = rec[(size_t)e * stride + o];
         const int type = (int)x.type;
         ok = ok && type != EV_GRADIENT && type != EV_SPOILER;
         if (x.dt > 1e-9) {
             ok = ok && (type == EV_RF || type == EV_DELAY);
-            if (first < 0) first = e;
-            last = e;
-            ++moving;
-        } else if (type == EV_ADC && moving > 0 && reset_after_adc && e + 1 < n_ev) {
-            ok = false;
+            begin = min(begin, (unsigned)e);
+            end = e + 1;
+            ++moved;
+        } else if (type == EV_ADC && reset_after_adc && e + 1 < n_ev) {
+            adc = e + 1;
         }
     }
+    const int moving = (int)__reduce_add_sync(kFull, moved);
+    const int last = (int)__reduce_max_sync(kFull, end) - 1;
+    const int first = (int)__reduce_min_sync(kFull, begin);
+    adc = __reduce_max_sync(kFull, adc);
+    // a readout that resets the state counts once the state has evolved
+    ok = __all_sync(kFull, ok) && !(moving > 0 && adc > 0 && first < (int)adc - 1);
+    if (lane != 0) return;
     int4 res = make_int4(0, 0, 0, 0);
     if (ok && moving > 0) {
         if (b.z >= 2) {
@@ -362,9 +369,10 @@ adjoint_block_kernel(const ChainArgs a, const int4* __restrict__ blk, int n_tan,
     const int lane = threadIdx.x & 31, grp = lane / GS, gl = lane % GS;
 
     const long long nch = a.n_chains;
-    long long ci = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = ci < nch;
-    if (!valid) ci = nch - 1;
+    const long long first = ((long long)blockIdx.x * kAdjBlkWarps + (threadIdx.x >> 5)) * a.cpw;
+    long long ci = first + lane;
+    const bool valid = lane < a.cpw && ci < nch;
+    if (!valid) ci = first < nch ? first : nch - 1;
     if (a.order) ci = a.order[ci];
     const int2 vm = a.chain_map[ci];
     const int v = vm.x, o = vm.y;

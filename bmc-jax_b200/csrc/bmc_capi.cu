@@ -103,20 +103,21 @@ TaylorTable make_table(double tol, int m_max, double dense_theta, double dense_s
 #define BMC_MIXED_F32 3.0
 #endif
 
-__device__ TaylorTable g_tables[3];   // [BMC_F64, BMC_F32, BMC_MIXED], per device
+__device__ TaylorTable g_tables[kTables];   // [BMC_F64, BMC_F32, BMC_MIXED, kTableFit], per device
 
-// the three tables, in precision order
+// the tables, in precision order; the last is BMC_F64's without the float32 tail
 void host_tables(TaylorTable* h) {
     h[BMC_F64] = make_table(1e-13, 30, 0.5, 100.0, 1e-6);
     h[BMC_F32] = make_table(std::ldexp(1.0, -24), 16, 0.5, 100.0, 0.0);
     h[BMC_MIXED] = make_table(BMC_MIXED_TOL, 30, 0.5, 100.0, BMC_MIXED_F32);
+    h[kTableFit] = make_table(1e-13, 30, 0.5, 100.0, 0.0);
 }
 
 // The host copy of one of the library's device tables: the chain and adjoint kernels take their table by
 // value, as a kernel parameter, so that the loads of the Taylor loops with warp-uniform indices come from the
 // constant bank. `tt` must point into g_tables (as tables() and noalloc_setup() return).
 bmc_status host_table_of(const TaylorTable* tt, TaylorTable* out) {
-    static TaylorTable h[3];
+    static TaylorTable h[kTables];
     static std::once_flag once;
     std::call_once(once, [] { host_tables(h); });
     // the device address of g_tables, looked up once per device (a call under stream capture then
@@ -137,7 +138,7 @@ bmc_status host_table_of(const TaylorTable* tt, TaylorTable* out) {
         base = it->second;
     }
     const long long i = tt - base;
-    if (i < 0 || i > 2) return fail(BMC_ERR_INVALID, "Taylor table %p is not one of the library's", (const void*)tt);
+    if (i < 0 || i >= kTables) return fail(BMC_ERR_INVALID, "Taylor table %p is not one of the library's", (const void*)tt);
     *out = h[i];
     return BMC_OK;
 }
@@ -168,7 +169,7 @@ bmc_status tables(int precision, const TaylorTable** out) {
     std::lock_guard<std::mutex> lk(g_mu);
     DeviceState& ds = dev_state(dev);
     if (!ds.tables_ready) {
-        TaylorTable h[3];
+        TaylorTable h[kTables];
         host_tables(h);
         CUDA_TRY(cudaMemcpyToSymbol(g_tables, h, sizeof(h)));
         CUDA_TRY(cudaGetSymbolAddress((void**)&ds.tables, g_tables));
@@ -224,14 +225,14 @@ bmc_status check_problem(const bmc_problem* pr, const double* params, const bmc_
 }
 
 bmc_status fill_spread(ChainArgs& a, const bmc_spread* sp) {
-    a.n_nodes = 1;
+    a.n_nodes = a.node_hi = 1;
     a.sigma = nullptr;
     a.u[0] = 0.0;
     a.w[0] = 1.0;
     if (!sp) return BMC_OK;
     if (sp->n_nodes < 1 || sp->n_nodes > kMaxNodes || !sp->h_u || !sp->h_w || !sp->d_sigma_hz)
         return fail(BMC_ERR_INVALID, "spread: 1..%d nodes with u, w and sigma required", kMaxNodes);
-    a.n_nodes = sp->n_nodes;
+    a.n_nodes = a.node_hi = sp->n_nodes;
     for (int j = 0; j < sp->n_nodes; ++j) {
         a.u[j] = sp->h_u[j];
         a.w[j] = sp->h_w[j];
@@ -243,8 +244,7 @@ bmc_status fill_spread(ChainArgs& a, const bmc_spread* sp) {
 // the repeated block of every row of a table of records (block_scan_kernel), into seg[n_rows]
 bmc_status scan_blocks(const EvRec<double>* rec, int n_rows, int n_ev, int stride, int4* seg, cudaStream_t st) {
     if (n_rows <= 0) return BMC_OK;
-    block_scan_kernel<double><<<(n_rows + kBlockScanRows - 1) / kBlockScanRows, kBlockScanThreads, 0, st>>>(
-        rec, n_rows, n_ev, stride, seg);
+    block_scan_kernel<double><<<n_rows, kBlockScanThreads, 0, st>>>(rec, n_ev, stride, seg);
     CUDA_TRY(cudaGetLastError());
     return BMC_OK;
 }
@@ -285,7 +285,7 @@ bmc_status use_adjoint(const EvRec<double>* rec, const bmc_problem* pr, int n_ta
     CUDA_TRY(cudaStreamIsCapturing(st, &cs));
     if (cs != cudaStreamCaptureStatusNone) return BMC_OK;
     CUDA_TRY(cudaMemsetAsync(flag, 1, sizeof(int), st));    // nonzero: every row so far qualifies
-    adjoint_rows_kernel<<<(pr->n_offsets + 127) / 128, 128, 0, st>>>(rec, pr->n_offsets, pr->n_events,
+    adjoint_rows_kernel<<<(pr->n_offsets + 3) / 4, 128, 0, st>>>(rec, pr->n_offsets, pr->n_events,
                                                                       pr->reset_after_adc, row_ev, flag);
     CUDA_TRY(cudaGetLastError());
     int h = 0;
@@ -566,8 +566,8 @@ bmc_status bmc_uneven_create(int32_t n_cest, int32_t n_voxels, const int32_t* h_
     }
     for (int t = 0; t < nt; ++t) {
         if (e == cudaSuccess && nev[t] > 0)
-            block_scan_kernel<double><<<(noff[t] + kBlockScanRows - 1) / kBlockScanRows, kBlockScanThreads>>>(
-                pl->rec + base[t], noff[t], nev[t], noff[t], pl->seg + row0[t]);
+            block_scan_kernel<double><<<noff[t], kBlockScanThreads>>>(pl->rec + base[t], nev[t], noff[t],
+                                                                       pl->seg + row0[t]);
         else if (e == cudaSuccess)
             e = cudaMemset(pl->seg + row0[t], 0, sizeof(int4) * noff[t]);
     }
@@ -576,7 +576,7 @@ bmc_status bmc_uneven_create(int32_t n_cest, int32_t n_voxels, const int32_t* h_
     if (e == cudaSuccess) e = cudaMemset(adj_flag, 1, sizeof(int));
     for (int t = 0; t < nt && e == cudaSuccess; ++t) {
         if (nev[t] > 0 && noff[t] > 0)
-            adjoint_block_rows_kernel<<<(noff[t] + 127) / 128, 128>>>(pl->rec + base[t], noff[t], nev[t], noff[t],
+            adjoint_block_rows_kernel<<<(noff[t] + 3) / 4, 128>>>(pl->rec + base[t], noff[t], nev[t], noff[t],
                                                                      pl->seg + row0[t], reset_after_adc,
                                                                      pl->adj_blk + row0[t], adj_flag);
         else
@@ -750,21 +750,28 @@ constexpr int kNoAllocMaxDevices = 64;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
+// ... and a second one for the shaped pulses' amplitudes and propagators: 8 bytes for every record that the first
+// one holds, 40 per row, and at least 24 MB of propagators (8,000 chains at a time with five pools).
+constexpr size_t kNoAllocTrainBytes = size_t(32) << 20;
+static __device__ __align__(256) unsigned char g_noalloc_train[kNoAllocTrainBytes];
+
 std::mutex g_noalloc_mu;
-void* g_noalloc_ptr[kNoAllocMaxDevices] = {};               // device address of the array, per device
+void* g_noalloc_ptr[kNoAllocMaxDevices] = {};               // device addresses of the arrays, per device
+void* g_noalloc_train_ptr[kNoAllocMaxDevices] = {};
 bool g_noalloc_tables[kNoAllocMaxDevices] = {};
 
 // Once per device, with that device current: the device address of the static array (in host code
 // its name is only a host-side stand-in) and the Taylor tables. Runs inside the first call on a
 // device, which should therefore come before any stream capture.
-bmc_status noalloc_setup(int precision, void** scratch, const TaylorTable** tt) {
+bmc_status noalloc_setup(int precision, void** scratch, void** train, const TaylorTable** tt,
+                         const TaylorTable** tt64) {
     int dev = 0;
     CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= kNoAllocMaxDevices)
         return fail(BMC_ERR_UNSUPPORTED, "bmc_simulate_noalloc: device %d above %d", dev, kNoAllocMaxDevices - 1);
     std::lock_guard<std::mutex> lk(g_noalloc_mu);
     if (!g_noalloc_tables[dev]) {
-        TaylorTable h[3];
+        TaylorTable h[kTables];
         host_tables(h);
         CUDA_TRY(cudaMemcpyToSymbol(g_tables, h, sizeof(h)));
         g_noalloc_tables[dev] = true;
@@ -775,11 +782,14 @@ bmc_status noalloc_setup(int precision, void** scratch, const TaylorTable** tt) 
         if (e != cudaSuccess || !p)
             return fail(BMC_ERR_CUDA, "bmc_simulate_noalloc: cudaGetSymbolAddress of the static scratch: %s",
                         cudaGetErrorString(e));
+        CUDA_TRY(cudaGetSymbolAddress(&g_noalloc_train_ptr[dev], g_noalloc_train));
         g_noalloc_ptr[dev] = p;
     }
     TaylorTable* t = nullptr;
     CUDA_TRY(cudaGetSymbolAddress((void**)&t, g_tables));
     *tt = t + precision;
+    *tt64 = t + BMC_F64;
+    *train = g_noalloc_train_ptr[dev];
     *scratch = g_noalloc_ptr[dev];
     return BMC_OK;
 }
@@ -801,12 +811,12 @@ extern "C" bmc_status bmc_simulate_noalloc(const bmc_problem* prob, const double
                     "bmc_simulate_noalloc: the event table (%d offsets x %d events = %zu records of %zu bytes) "
                     "exceeds its static scratch of %zu bytes (at most %zu records); use bmc_simulate",
                     prob->n_offsets, prob->n_events, nrec, rec_bytes, kNoAllocScratchBytes, cap);
-    void* scratch = nullptr;
-    const TaylorTable* tt = nullptr;
-    if ((s = noalloc_setup(prob->precision, &scratch, &tt)) != BMC_OK) return s;
+    void *scratch = nullptr, *train = nullptr;
+    const TaylorTable *tt = nullptr, *tt64 = nullptr;
+    if ((s = noalloc_setup(prob->precision, &scratch, &train, &tt, &tt64)) != BMC_OK) return s;
     const cudaStream_t st = (cudaStream_t)stream;
     char* base = static_cast<char*>(scratch);
     const NoAllocScratch ws{reinterpret_cast<int*>(base), reinterpret_cast<int4*>(base + kNoAllocStatusBytes),
-                            base + fixed};
+                            base + fixed, train, kNoAllocTrainBytes, tt64};
     BMC_DISPATCH(prob->n_cest, noalloc(prob, d_params, ev, d_m0, spread, d_out, ws, tt, st));
 }

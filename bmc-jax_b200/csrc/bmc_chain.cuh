@@ -35,6 +35,16 @@ struct TaylorTable {
     float inv_fact_f[kTaylorMMax + 1];  // 1 / k! in float32
 };
 
+// A row's unit of a shaped-pulse train (bmc_train.cuh): the reference pulse (first event, samples), the gap events
+// it takes in, how many equal units are applied at each mark (run) and the events those cover (span). n = 0: the
+// row has no train.
+struct TrainRow {
+    int first, n, gap, run;
+    int span, uses;
+    double w_max;
+};
+constexpr int kTrainMark = 8;  // added to the type of a record where a unit begins
+
 struct ChainArgs {
     int n_vox, n_off, n_ev, n_fields;
     int mz;                    // state index written; < 0: whole state
@@ -48,6 +58,7 @@ struct ChainArgs {
     const double* sigma;       // [n_vox] spread width [Hz] or null
     // tangents handled by this launch: global tangent indices t0 .. t0 + NT - 1
     int t0;
+    int n_tan;                 // tangents of the whole set (node_jout's layout)
     int field_row[kMaxT];
     const double* seed;        // [P][n_vox]
     const double* dm0;         // [P][n_vox][N] or null
@@ -72,7 +83,35 @@ struct ChainArgs {
     const int4* seg;           // null: no reuse
     const int* tab_row0;       // [n_tables]: first row of each table in `seg` (uneven batches)
     double dense_switch;       // > 0: the norm above which an event takes the dense path (else the table's)
+    int cpw;                   // chains per warp: lanes from cpw on have none (chains_per_warp below)
+    // Isochromats as chains of their own (chain kernel): node j of chain c is chain j * chains + c of the launch,
+    // and its weighted results go to node_out [node][chains (x N)] and node_jout [node][P][chains]; node_sum_kernel
+    // adds them in node order. Null node_out: every chain loops over its nodes.
+    double* node_out;
+    double* node_jout;
+    int node_lo, node_hi;      // with a null node_out: the nodes of this launch (from 1 on added to the output)
+    // Part of the launch order (uniform tables; chain_count 0: all): chains first_chain .. first_chain + chain_count
+    long long first_chain, chain_count;
+    // Propagators of those chains' shaped pulses (null: none), applied at the marked records
+    const TrainRow* train;     // [n_off]
+    const double* prop;
+    const int* prop_ok;
 };
+
+// Chains per warp of a launch: 32, or as many fewer as still leave the launch's warps resident at once. A launch
+// of few chains is bound by the latency of one warp, which grows with its lanes: their dense events are taken a
+// group of lanes at a time, one round after another, and their Taylor degrees differ. One spectrum of 61 chains (2 s
+// CW, two pools and MT) took 292 us in the kernel with 32 chains per warp, 83 us with one. The chain kernel counts
+// one block per SM as resident: its unrolled term loops stream from the instruction cache, and 714 chains (a fit of
+// 100-sample trains) in 2 chains per warp on 90 blocks took 49.7 ms of tangent passes, in 1 per warp on 179 blocks, two
+// on some SMs, 76.6 (32 per warp: 53.0). A power of two from `least` (the chains a warp's lane groups take at once) to 32.
+constexpr int kSMs = 148;
+inline int chains_per_warp(long long chains, int blocks_per_sm, int warps, int least) {
+    int c = 32;
+    const long long slots = (long long)kSMs * blocks_per_sm * warps;
+    while (c > least && (chains + c / 2 - 1) / (c / 2) <= slots) c /= 2;
+    return c;
+}
 
 template <int NC>
 struct Layout {
@@ -336,101 +375,166 @@ struct Chain {
     // unnormalised powers p_k = X^k [M; 1] are accumulated with weights 1/k!, so each term is one sparse
     // operator product and one fused multiply-add per state entry. The coefficients (scaled by h) are
     // formed at each sub-step, so that they are not held in registers across the rest of the event.
-    // The loops run to the warp's largest (s, m); each chain uses only its own (ns_own, m_own), so a
-    // chain's result never depends on which chains share its warp.
+    // Every lane runs its own (ns, m): a chain's result never depends on which chains share its warp. Where the
+    // lanes of a warp agree (cost-sorted warps mostly do) the loops do not diverge.
     //
-    // In the float64 kernel without tangents, the terms of a chain from tt.f32_from[m_own] on (each below
+    // In the float64 kernel without tangents, the terms of a chain from tt.f32_from[m] on (each below
     // 1e-6 of the state, in the balanced norm of coef_norm) are formed in float32 and summed in a float32
     // accumulator that is added to M once per sub-step: their rounding, a few units of 2^-24 of terms
     // below 1e-6, is at most ~2e-13 of the state per event, the order of the truncation tolerance.
-    // The switch point is the chain's own: where the lanes of a warp disagree on it, the sub-step runs
-    // once per distinct switch point, each lane adding its terms only in its own pass (weight 0 in the
-    // others), so the result stays independent of the chains that share the warp. Cost-sorted warps
-    // almost always agree (one pass). Returns the number of passes over all sub-steps.
-    static __device__ __forceinline__ int taylor_apply(const ChainConst<NC, D>& cst, const EvRec<R>& rec, D g_mt,
-                                                       R h, int ns_w, int m_w, int ns_own, int m_own,
-                                                       State<NC, D>& M, const TaylorTable& tt) {
+    // The switch point is the chain's own too: the lanes leave the float64 loop at their own term and meet again
+    // before the float32 loop, so a warp takes one pass per sub-step (its largest float64 count plus its largest
+    // float32 count) however its switch points differ. Passing over the sub-step once per distinct switch point
+    // instead cost a warp of 32 different offsets (one spectrum) up to ten passes: 1 voxel x 102 offsets x 4,041
+    // events took 78.9 ms so, 22.1 ms in one pass (cost-sorted warps, 2,048 voxels: 90.5 against 92.8 ms).
+    static __device__ __forceinline__ void taylor_apply(const ChainConst<NC, D>& cst, const EvRec<R>& rec, D g_mt,
+                                                        R h, int ns, int m, State<NC, D>& M, const TaylorTable& tt) {
         constexpr bool kMixed = std::is_same<R, double>::value && NT == 0;
+        const int k32 = kMixed ? tt.f32_from[m] : m + 1;
         // The terms are added to M as they are formed (later terms derive from `term`, not from M), so no
-        // separate accumulator is held; a lane past its own sub-steps or degree adds with weight 0.
-        // fma(1, t, M) rounds like M + t and fma(0, t, M) is M: the result is that of summing apart.
-        int passes = 0;
+        // separate accumulator is held.
 #pragma unroll 1
-        for (int j = 0; j < ns_w; ++j) {
-            const bool on = j < ns_own;
-            // this lane's switch point (0: no sub-step of its own here); lanes still to be served
-            const int k32_own = on ? (kMixed ? tt.f32_from[m_own] : m_w + 1) : 0;
-            unsigned pend = __ballot_sync(0xffffffffu, k32_own != 0);
+        for (int j = 0; j < ns; ++j) {
+            StepCoef<NC, D> s;
+            event_coef(cst, rec, g_mt, s);
+            scale_coef(s, h);
+            State<NC, D> term;
+            matvec<true>(s, M, term, &cst, h);
+            fma_state(M, R(1), term);
+            int k = 2;
 #pragma unroll 1
-            do {
-                const int k32 = __shfl_sync(0xffffffffu, k32_own, __ffs(pend) - 1);
-                const bool member = k32_own == k32;
-                pend &= ~__ballot_sync(0xffffffffu, member);
-                ++passes;
-                const int m_on = member ? m_own : 0;
-                StepCoef<NC, D> s;
-                event_coef(cst, rec, g_mt, s);
-                scale_coef(s, h);
-                State<NC, D> term;
-                matvec<true>(s, M, term, &cst, h);
-                fma_state(M, member ? R(1) : R(0), term);
-                int k = 2;
+            for (; k <= m && k < k32; ++k) {
+                State<NC, D> nt;
+                matvec<false>(s, term, nt);
+                term = nt;
+                fma_state(M, R(tt.inv_fact[k]), term);
+            }
+            if constexpr (kMixed) {
+                if (k <= m) {
+                    // paired float32 instructions over the CEST pools (bmc_tail32.cuh)
+                    using T32 = Tail32<NC>;
+                    typename T32::Coef s32;
+                    typename T32::St t32, a32;
+                    T32::coef(s, s32);
+                    T32::state(term, t32);
+                    T32::zero(a32);
 #pragma unroll 1
-                for (; k <= m_w && k < k32; ++k) {
-                    State<NC, D> nt;
-                    matvec<false>(s, term, nt);
-                    term = nt;
-                    fma_state(M, k <= m_on ? R(tt.inv_fact[k]) : R(0), term);
-                }
-                if constexpr (kMixed) {
-                    if (k <= m_w) {
-                        // paired float32 instructions over the CEST pools (bmc_tail32.cuh)
-                        using T32 = Tail32<NC>;
-                        typename T32::Coef s32;
-                        typename T32::St t32, a32;
-                        T32::coef(s, s32);
-                        T32::state(term, t32);
-                        T32::zero(a32);
-#pragma unroll 1
-                        for (; k <= m_w; ++k) {
-                            typename T32::St n32;
-                            T32::matvec(s32, t32, n32);
-                            t32 = n32;
-                            T32::fma_acc(a32, k <= m_on ? tt.inv_fact_f[k] : 0.f, t32);
-                        }
-                        T32::add_to(M, a32);
+                    for (; k <= m; ++k) {
+                        typename T32::St n32;
+                        T32::matvec(s32, t32, n32);
+                        t32 = n32;
+                        T32::fma_acc(a32, tt.inv_fact_f[k], t32);
                     }
+                    T32::add_to(M, a32);
                 }
-            } while (pend);
+            }
         }
-        return passes;
     }
 
-    // elementwise precision changes between structs made only of Dn<., 0> members (StepCoef, State)
-    template <typename A, typename B>
-    static __device__ __forceinline__ void to_float(const A& a, B& b) {
-        constexpr int n = sizeof(A) / sizeof(double);
-        static_assert(sizeof(B) == n * sizeof(float), "layouts differ");
-        const double* pa = reinterpret_cast<const double*>(&a);
-        float* pb = reinterpret_cast<float*>(&b);
+    // Whether an event leaves the transverse entries at zero: no RF, and all of them (with their tangents) zero.
+    static __device__ __forceinline__ bool longitudinal(const State<NC, D>& M) {
+        auto zero = [](const D& x) {
+            bool z = x.v == R(0);
+            DN_LOOP(z = z && x.d[t] == R(0));
+            return z;
+        };
+        bool z = zero(M.xw) && zero(M.yw);
 #pragma unroll
-        for (int i = 0; i < n; ++i) pb[i] = float(pa[i]);
+        for (int i = 0; i < NC; ++i) z = z && zero(M.xc[i]) && zero(M.yc[i]);
+        return z;
     }
-    template <typename B>
-    static __device__ __forceinline__ void zero_state(B& b) {
-        constexpr int n = sizeof(B) / sizeof(float);
-        float* pb = reinterpret_cast<float*>(&b);
+
+    // exp(X) [M; 1] of a free event (no RF) whose transverse entries are all zero: they stay zero, and the z entries
+    // (water, CEST pools, MT) evolve by their own (NC + 2) x (NC + 2) block, which one thread exponentiates for its
+    // chain: the degree-m Horner recurrence of the block and of its constant column, then s squarings, the norm
+    // without any precession in it.
+    // Recoveries and the delays behind a spoiler are such events. The dense path gives each of them a warp for ~11
+    // Horner steps and ~13 squarings of the whole (N + 1) x (N + 1) matrix: 206,848 chains of four pools with one
+    // 3 s recovery (and one propagator to apply) took 4.89 ms in the chain kernel so, 0.31 ms this way.
+    static __device__ __noinline__ void z_event(const ChainConst<NC, D>& cc, R dt, State<NC, D>& M,
+                                                const TaylorTable& tt) {
+        constexpr int Z = NC + 2;
+        // the infinity norm in the balanced scaling of norm_base
+        R ex = R(0);
 #pragma unroll
-        for (int i = 0; i < n; ++i) pb[i] = 0.f;
-    }
-    template <typename B>
-    static __device__ __forceinline__ void add_float(State<NC, D>& M, const B& a) {
-        constexpr int n = sizeof(B) / sizeof(float);
-        static_assert(sizeof(State<NC, D>) == n * sizeof(double), "layouts differ");
-        double* pm = reinterpret_cast<double*>(&M);
-        const float* pa = reinterpret_cast<const float*>(&a);
+        for (int i = 0; i < NC; ++i) ex += fabs(cc.k[i].v) * R(cc.sf[i]);
+        const R km = fabs(cc.kmt.v) * R(cc.sfm);
+        R nu = fabs(cc.Rw1.v) + ex + km + fabs(cc.cw.v);
+        nu = fmax(nu, fabs(cc.Rm1.v) + km + fabs(cc.cm.v) / R(cc.sfm));
 #pragma unroll
-        for (int i = 0; i < n; ++i) pm[i] = pm[i] + double(pa[i]);
+        for (int i = 0; i < NC; ++i)
+            nu = fmax(nu, fabs(cc.Rc1[i].v) + fabs(cc.k[i].v) * R(cc.sf[i]) + fabs(cc.cc[i].v) / R(cc.sf[i]));
+        nu = nu * dt;
+        const int s = nu > R(tt.dense_theta) ? (int)ceil(log2(double(nu) / tt.dense_theta)) : 0;
+        const R h = R(ldexp(double(dt), -s));
+        D T[Z][Z], phi[Z];                    // T[column][row]
+        // Horner, column by column: v <- e + X v / k (the constant column: phi <- X [phi; 1] / k)
+#pragma unroll
+        for (int j = 0; j <= Z; ++j) {
+            D v[Z];
+#pragma unroll
+            for (int i = 0; i < Z; ++i) v[i] = dconst<R, NT>(i == j ? R(1) : R(0));
+#pragma unroll 1
+            for (int k = tt.dense_m; k >= 1; --k) {
+                const R ik = h * R(tt.inv_k[k]);
+                D w = dfma(cc.kmt, v[Z - 1], -(cc.Rw1 * v[0]));
+                D m = dfma(cc.kwmt, v[0], -(cc.Rm1 * v[Z - 1]));
+                if (j == Z) {
+                    w = w + cc.cw;
+                    m = m + cc.cm;
+                }
+#pragma unroll
+                for (int i = 0; i < NC; ++i) {
+                    w = dfma(cc.k[i], v[1 + i], w);
+                    D c = dfma(cc.kwc[i], v[0], -(cc.Rc1[i] * v[1 + i]));
+                    if (j == Z) c = c + cc.cc[i];
+                    v[1 + i] = ik * c;
+                }
+                v[0] = ik * w;
+                v[Z - 1] = ik * m;
+                if (j < Z) v[j] = v[j] + R(1);
+            }
+#pragma unroll
+            for (int i = 0; i < Z; ++i) (j < Z ? T[j < Z ? j : 0][i] : phi[i]) = v[i];
+        }
+#pragma unroll 1
+        for (int q = 0; q < s; ++q) {
+            D n[Z][Z];
+#pragma unroll
+            for (int i = 0; i < Z; ++i) {
+                D p = phi[i];
+#pragma unroll
+                for (int l = 0; l < Z; ++l) p = dfma(T[l][i], phi[l], p);
+                n[0][i] = p;                  // parked: phi is read by every row
+            }
+#pragma unroll
+            for (int i = 0; i < Z; ++i) phi[i] = n[0][i];
+#pragma unroll
+            for (int j = 0; j < Z; ++j)
+#pragma unroll
+                for (int i = 0; i < Z; ++i) {
+                    D x = T[0][i] * T[j][0];
+#pragma unroll
+                    for (int l = 1; l < Z; ++l) x = dfma(T[l][i], T[j][l], x);
+                    n[j][i] = x;
+                }
+#pragma unroll
+            for (int j = 0; j < Z; ++j)
+#pragma unroll
+                for (int i = 0; i < Z; ++i) T[j][i] = n[j][i];
+        }
+        D z[Z];
+#pragma unroll
+        for (int i = 0; i < Z; ++i) {
+            D x = dfma(T[0][i], M.zw, phi[i]);
+#pragma unroll
+            for (int l = 0; l < NC; ++l) x = dfma(T[1 + l][i], M.zc[l], x);
+            z[i] = dfma(T[Z - 1][i], M.zm, x);
+        }
+        M.zw = z[0];
+#pragma unroll
+        for (int i = 0; i < NC; ++i) M.zc[i] = z[1 + i];
+        M.zm = z[Z - 1];
     }
 
     static __device__ __forceinline__ void spoil(State<NC, D>& M) {

@@ -10,8 +10,8 @@
 // state.
 //
 // One thread per chain, in launch order (the problems are small: a few truths times the rows of a
-// protocol). An event evolves by the chain kernel's truncated-Taylor action (Chain::taylor_apply, warp
-// synchronous) or, where its norm is above the dense threshold (long CW blocks), by a scaling and
+// protocol). An event evolves by the chain kernel's truncated-Taylor action (Chain::taylor_apply)
+// or, where its norm is above the dense threshold (long CW blocks), by a scaling and
 // squaring that the thread does alone: the columns of exp(X h) by Taylor polynomials, s squarings, one
 // product with [M; 1]. Its matrices live in a global scratch, entry-major with the chains adjacent.
 #pragma once
@@ -214,11 +214,9 @@ __global__ void __launch_bounds__(128) design_kernel(const ChainArgs a, const De
                 while (m < tt.m_max && tt.theta[m] < pr) ++m;
                 m_own = m;
             }
-            const int ns_w = __reduce_max_sync(kFull, (unsigned)ns_own);
-            const int m_w = __reduce_max_sync(kFull, (unsigned)m_own);
-            if (ns_w > 0) {
-                const HD h = tay ? (ns_own == 1 ? rec.dt : rec.dt / HD(double(ns_own))) : HD(0.0);
-                C::taylor_apply(cc, rec, g, h, ns_w, m_w, ns_own, m_own, M, tt);
+            if (tay) {
+                const HD h = ns_own == 1 ? rec.dt : rec.dt / HD(double(ns_own));
+                C::taylor_apply(cc, rec, g, h, ns_own, m_own, M, tt);
             }
         }
         if (type == EV_GRADIENT || type == EV_SPOILER) C::spoil(M);

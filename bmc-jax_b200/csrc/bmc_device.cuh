@@ -294,10 +294,11 @@ __device__ Dn<R, NT> sl_direct(Dn<R, NT> delta, Dn<R, NT> t2) {
 template <typename R, int NT>
 __device__ Dn<R, NT> super_lorentzian(Dn<R, NT> delta, Dn<R, NT> t2, Dn<R, NT> w0) {
     if (fabs(delta.v) >= w0.v) return sl_direct<R, NT>(delta, t2);
-    const Dn<R, NT> p0 = -w0 - R(300), p1 = -w0 - R(100);
-    const Dn<R, NT> p2 = w0 + R(100), p3 = w0 + R(300);
-    const Dn<R, NT> y0 = sl_direct<R, NT>(p0, t2), y1 = sl_direct<R, NT>(p1, t2);
-    const Dn<R, NT> y2 = sl_direct<R, NT>(p2, t2), y3 = sl_direct<R, NT>(p3, t2);
+    // the support points -w0 - 300, -w0 - 100, w0 + 100, w0 + 300: the sum depends on the square of its argument, so
+    // the two on the left have the values (and derivatives) of those on the right, bit for bit
+    const Dn<R, NT> p1 = -w0 - R(100), p2 = w0 + R(100);
+    const Dn<R, NT> y3 = sl_direct<R, NT>(w0 + R(300), t2), y2 = sl_direct<R, NT>(p2, t2);
+    const Dn<R, NT> y0 = y3, y1 = y2;
     const Dn<R, NT> d0 = R(30) * (y1 - y0), d1 = R(30) * (y3 - y2);
     const Dn<R, NT> c = dabs((delta - p1 + R(1)) / (p2 - p1 + R(1)));
     const Dn<R, NT> c2 = c * c, c3 = c2 * c;

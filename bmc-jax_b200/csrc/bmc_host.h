@@ -22,6 +22,10 @@ bmc_status fail(bmc_status s, const char* fmt, ...);
         if (e_ != cudaSuccess) return fail(BMC_ERR_CUDA, "%s: %s", #expr, cudaGetErrorString(e_)); \
     } while (0)
 
+// The Taylor tables: one per precision (BMC_F64, BMC_F32, BMC_MIXED), and for the primal passes of a fit the float64
+// one without a float32 tail, as the tangent kernels have none: the tail's rounding (~1e-13 in Z) differs between the
+// costs that a fit compares, and near a minimum a step lowers the cost by less.
+constexpr int kTableFit = 3, kTables = 4;
 bmc_status tables(int precision, const TaylorTable** out);
 bmc_status host_table_of(const TaylorTable* tt, TaylorTable* out);
 bmc_status workspace(size_t bytes, cudaStream_t st, void** out);
@@ -73,6 +77,9 @@ struct NoAllocScratch {
     int* status;
     int4* seg;      // every row's repeated block
     void* rec;      // the event records
+    void* train;    // rows, amplitudes and propagators of shaped pulses
+    size_t train_bytes;
+    const TaylorTable* tt64;   // the float64 table, which the propagators are formed with
 };
 
 // Everything that is compiled per pool count.

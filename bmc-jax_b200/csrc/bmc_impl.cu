@@ -13,6 +13,7 @@
 #include "bmc_adjoint.cuh"
 #include "bmc_adjoint_block.cuh"
 #include "bmc_design.cuh"
+#include "bmc_train.cuh"
 
 #ifndef BMC_NC
 #error "compile with -DBMC_NC=<CEST pools>"
@@ -33,7 +34,7 @@ bmc_status prep_events(const bmc_problem* pr, const bmc_events* ev, EvRec<R>* ou
 }
 
 template <int NC, typename R, int NT, bool U, bool COUNT>
-bmc_status launch_chain_impl(const ChainArgs& a, const TaylorTable* tt, cudaStream_t st) {
+bmc_status launch_chain_impl(ChainArgs a, const TaylorTable* tt, cudaStream_t st) {
     constexpr int kWarps = ChainLaunch<NC, NT>::kWarps;
     const size_t smem = kWarps * sizeof(DenseSmem<NC, typename DenseReal<R>::type, NT>) +
                         32 * kWarps * sizeof(ChainConst<NC, Dn<R, NT>>);
@@ -47,8 +48,10 @@ bmc_status launch_chain_impl(const ChainArgs& a, const TaylorTable* tt, cudaStre
                                       (int)smem));
         if (dev < 64) configured.fetch_or(1ull << dev, std::memory_order_acq_rel);
     }
-    const long long nch = U ? a.n_chains : (long long)a.n_vox * a.n_off;
-    const long long blocks = (nch + kWarps * 32 - 1) / (kWarps * 32);
+    long long nch = (U ? a.n_chains : (long long)a.n_vox * a.n_off) * (a.node_out ? a.n_nodes : 1);
+    if (a.chain_count) nch = a.chain_count;
+    a.cpw = chains_per_warp(nch, 1, kWarps, 1);
+    const long long blocks = (nch + kWarps * a.cpw - 1) / (kWarps * a.cpw);
     if (blocks > 0x7fffffffLL) return fail(BMC_ERR_INVALID, "%lld chains exceed one launch", nch);
     if (blocks == 0) return BMC_OK;
     TaylorTable th;
@@ -70,7 +73,7 @@ bmc_status launch_chain(const ChainArgs& a, const TaylorTable* tt, cudaStream_t 
 }
 
 template <int NC, bool kTan = true>
-bmc_status launch_adjoint(const ChainArgs& a, const int* row_ev, int n_tan, const TaylorTable* tt, cudaStream_t st) {
+bmc_status launch_adjoint(ChainArgs a, const int* row_ev, int n_tan, const TaylorTable* tt, cudaStream_t st) {
     const size_t smem = kAdjWarps * AdjGroup<NC>::G * sizeof(AdjSlot<NC>);
     static std::atomic<unsigned long long> configured{0};
     int dev = 0;
@@ -81,7 +84,8 @@ bmc_status launch_adjoint(const ChainArgs& a, const int* row_ev, int n_tan, cons
         if (dev < 64) configured.fetch_or(1ull << dev, std::memory_order_acq_rel);
     }
     const long long nch = (long long)a.n_vox * a.n_off;
-    const long long blocks = (nch + kAdjWarps * 32 - 1) / (kAdjWarps * 32);
+    a.cpw = chains_per_warp(nch, kTan ? 2 : BMC_ADJ_PRIMAL_BLOCKS, kAdjWarps, AdjGroup<NC>::G);
+    const long long blocks = (nch + kAdjWarps * a.cpw - 1) / (kAdjWarps * a.cpw);
     if (blocks > 0x7fffffffLL) return fail(BMC_ERR_INVALID, "%lld chains exceed one launch", nch);
     if (blocks == 0) return BMC_OK;
     TaylorTable th;
@@ -92,7 +96,7 @@ bmc_status launch_adjoint(const ChainArgs& a, const int* row_ev, int n_tan, cons
 }
 
 template <int NC, bool kTan = true>
-bmc_status launch_adjoint_block(const ChainArgs& a, const int4* blk, int n_tan, const TaylorTable* tt, cudaStream_t st) {
+bmc_status launch_adjoint_block(ChainArgs a, const int4* blk, int n_tan, const TaylorTable* tt, cudaStream_t st) {
     const size_t smem = kAdjBlkWarps * DenseGroup<NC>::G * sizeof(AdjBlkSlot<NC, kTan>);
     static std::atomic<unsigned long long> configured{0};
     int dev = 0;
@@ -102,12 +106,31 @@ bmc_status launch_adjoint_block(const ChainArgs& a, const int4* blk, int n_tan, 
                                       (int)smem));
         if (dev < 64) configured.fetch_or(1ull << dev, std::memory_order_acq_rel);
     }
-    const long long blocks = (a.n_chains + kAdjBlkWarps * 32 - 1) / (kAdjBlkWarps * 32);
+    // one round per warp: the rounds of a warp run one after another whatever its lanes hold, so short warps only
+    // balance the launch better (192 voxels, 1 to 5 pools: 129 ms per joint fit with 32 chains per warp, 38 with as
+    // many as the resident warps leave, 35 with one round)
+    a.cpw = DenseGroup<NC>::G;
+    const long long blocks = (a.n_chains + kAdjBlkWarps * a.cpw - 1) / (kAdjBlkWarps * a.cpw);
     if (blocks > 0x7fffffffLL) return fail(BMC_ERR_INVALID, "%lld chains exceed one launch", a.n_chains);
     if (blocks == 0) return BMC_OK;
     TaylorTable th;
     if (bmc_status s = host_table_of(tt, &th); s != BMC_OK) return s;
     adjoint_block_kernel<NC, kTan><<<(unsigned)blocks, kAdjBlkWarps * 32, smem, st>>>(a, blk, n_tan, th);
+    CUDA_TRY(cudaGetLastError());
+    return BMC_OK;
+}
+
+// Whether the nodes of a spread run as chains of their own (ChainArgs::node_out): where the chains alone fill less
+// than half of the resident lanes, and the nodes' results take at most 256 MB. 101 chains of 16 nodes (five pools, 20
+// pulses of 100 samples) took 1.37 s in 4 warps.
+bool split_nodes(long long chains, const bmc_spread* sp, size_t values) {
+    return sp && sp->n_nodes > 1 && chains < (long long)kSMs * BMC_FWD_MIN_BLOCKS * 4 * 16 &&
+           values * sp->n_nodes * sizeof(double) <= (size_t(256) << 20);
+}
+
+template <typename R>
+bmc_status sum_nodes(const ChainArgs& a, long long n, const double* part, double* out, cudaStream_t st) {
+    node_sum_kernel<std::is_same<R, double>::value><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(a, part, n, out);
     CUDA_TRY(cudaGetLastError());
     return BMC_OK;
 }
@@ -135,16 +158,127 @@ bmc_status order_chains(ChainArgs& a, Carve& cv, cudaStream_t st) {
 template <int NC>
 constexpr int tangents_per_pass() { return NC <= 1 ? 2 : 1; }
 
+// Shaped-pulse trains of a call: the rows' units and amplitudes, and the propagators (with those of `tangents`
+// derivatives) of `chunk` chains at a time: kTrainChunk, or what the call has if that is less (300 MB with four pools).
+constexpr long long kTrainChunk = 131072;
+template <int NC>
+struct Trains {
+    int max_samples = 0, mats = 1;
+    long long chunk = 0;
+    TrainArgs tr{};
+    const TaylorTable* tt64 = nullptr;   // the float64 table, which the propagators are formed with
+
+    // tables too short for two pulses have no trains
+    static bool wanted(const bmc_problem* pr) { return pr->n_events >= 2 * kTrainMinSamples; }
+
+    size_t per_chain() const { return sizeof(double) * mats * TrainShape<NC>::N * TrainShape<NC>::NS + sizeof(int); }
+    size_t fixed_bytes(const bmc_problem* pr, int tangents) {
+        max_samples = std::min(pr->n_events, kTrainMaxSamples);
+        mats = 1 + tangents;
+        return align256(sizeof(TrainRow) * pr->n_offsets) +
+               align256(sizeof(double) * (size_t)max_samples * pr->n_offsets) + 512;
+    }
+    size_t bytes(const bmc_problem* pr, long long chains, int tangents) {
+        const size_t fixed = fixed_bytes(pr, tangents);
+        chunk = std::min(chains, kTrainChunk / mats);
+        return fixed + (size_t)chunk * per_chain();
+    }
+    // carves the scratch, finds the rows' trains and marks the records `rec` (a.ev's)
+    bmc_status scan(ChainArgs& a, EvRec<double>* rec, Carve& cv, cudaStream_t st) {
+        TrainRow* rows = cv.take<TrainRow>(a.n_off);
+        double* rho = cv.take<double>((size_t)max_samples * a.n_off);
+        tr.rho = rho;
+        tr.max_samples = max_samples;
+        tr.prop = cv.take<double>((size_t)chunk * mats * TrainShape<NC>::N * TrainShape<NC>::NS);
+        tr.ok = cv.take<int>(chunk);
+        train_scan_kernel<<<a.n_off, kTrainScanThreads, 0, st>>>(rec, a.n_ev, a.n_off, train_min_uses<NC>(),
+                                                                 const_cast<int4*>(a.seg), rows, rho, max_samples);
+        CUDA_TRY(cudaGetLastError());
+        a.train = rows;
+        a.prop = tr.prop;
+        a.prop_ok = tr.ok;
+        return BMC_OK;
+    }
+
+    template <int DT>
+    bmc_status form(const ChainArgs& a, int tangents, cudaStream_t st) const {
+        constexpr int kWarps = TrainShape<NC>::kWarps;
+        const size_t smem = kWarps * sizeof(TrainSmem<NC, DT>);
+        static std::atomic<unsigned long long> configured{0};
+        int dev = 0;
+        CUDA_TRY(cudaGetDevice(&dev));
+        if (dev >= 64 || !((configured.load(std::memory_order_acquire) >> dev) & 1ull)) {
+            CUDA_TRY(cudaFuncSetAttribute(train_kernel<NC, DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            if (dev < 64) configured.fetch_or(1ull << dev, std::memory_order_acq_rel);
+        }
+        TaylorTable th;
+        if (bmc_status s = host_table_of(tt64, &th); s != BMC_OK) return s;
+        TrainArgs t = tr;
+        t.mats = 1 + tangents;
+        const dim3 grid((unsigned)((a.chain_count + kWarps - 1) / kWarps), DT ? tangents : 1);
+        train_kernel<NC, DT><<<grid, 32 * kWarps, smem, st>>>(a, t, th);
+        CUDA_TRY(cudaGetLastError());
+        return BMC_OK;
+    }
+
+    // One pass over every chain with NT tangents: per chunk of the launch order (and per node, where the nodes do not
+    // run as chains of their own) the propagators, then the chains.
+    template <int NT>
+    bmc_status pass(ChainArgs a, const TaylorTable* tt, cudaStream_t st) const {
+        const long long all = (long long)a.n_vox * a.n_off * (a.node_out ? a.n_nodes : 1);
+        for (a.first_chain = 0; a.first_chain < all; a.first_chain += chunk) {
+            a.chain_count = std::min(chunk, all - a.first_chain);
+            for (int j = 0; j < (a.node_out ? 1 : a.n_nodes); ++j) {
+                if (!a.node_out) {
+                    a.node_lo = j;
+                    a.node_hi = j + 1;
+                }
+                bmc_status s = form<(NT > 0 ? 1 : 0)>(a, NT, st);
+                if (s != BMC_OK || (s = launch_chain<NC, double, NT>(a, tt, st)) != BMC_OK) return s;
+            }
+        }
+        return BMC_OK;
+    }
+};
+
+// every tangent, tangents_per_pass at a time; `trains`: the table's trains (null: none looked for)
 template <int NC, bool U = false>
-bmc_status run_tangents(ChainArgs a, int P, const TaylorTable* tt, cudaStream_t st) {
-    constexpr int TP = tangents_per_pass<NC>();
+bmc_status run_tangents(ChainArgs a, int P, const TaylorTable* tt, cudaStream_t st, const Trains<NC>* trains = nullptr) {
+    constexpr int TP = tangents_per_pass<NC>(), TP2 = TP >= 2 ? 2 : 1;
+    a.n_tan = P;
     for (int t0 = 0; t0 < P; t0 += TP) {
         a.t0 = t0;
-        bmc_status s = (P - t0 >= 2 && TP >= 2) ? launch_chain<NC, double, (TP >= 2 ? 2 : 1), U>(a, tt, st)
-                                                : launch_chain<NC, double, 1, U>(a, tt, st);
+        const bool two = P - t0 >= 2 && TP >= 2;
+        bmc_status s = BMC_OK;
+        if constexpr (!U) {
+            if (trains) {
+                s = two ? trains->template pass<TP2>(a, tt, st) : trains->template pass<1>(a, tt, st);
+                if (s != BMC_OK) return s;
+                continue;
+            }
+        }
+        s = two ? launch_chain<NC, double, TP2, U>(a, tt, st) : launch_chain<NC, double, 1, U>(a, tt, st);
         if (s != BMC_OK) return s;
     }
+    if (a.node_out) {
+        const long long nch = (long long)a.n_vox * a.n_off;
+        bmc_status s = sum_nodes<double>(a, nch, a.node_out, a.out, st);
+        return s != BMC_OK ? s : sum_nodes<double>(a, nch * P, a.node_jout, a.jout, st);
+    }
     return BMC_OK;
+}
+
+// a primal pass, its nodes summed where they ran as chains of their own
+template <int NC, typename R>
+bmc_status run_primal(const ChainArgs& a, const TaylorTable* tt, cudaStream_t st, const Trains<NC>* trains = nullptr) {
+    bmc_status s = BMC_OK;
+    if constexpr (std::is_same<R, double>::value) {
+        s = trains ? trains->template pass<0>(a, tt, st) : launch_chain<NC, R, 0>(a, tt, st);
+    } else {
+        s = launch_chain<NC, R, 0>(a, tt, st);
+    }
+    if (s != BMC_OK || !a.node_out) return s;
+    return sum_nodes<R>(a, (long long)a.n_vox * a.n_off * (a.mz >= 0 ? 1 : Layout<NC>::N), a.node_out, a.out, st);
 }
 
 }  // namespace
@@ -206,8 +340,15 @@ bmc_status Impl<NC>::simulate(const bmc_problem* pr, const double* params, const
     void* ws = nullptr;
     const size_t recb = pr->precision == BMC_F32 ? sizeof(EvRec<float>) : sizeof(EvRec<double>);
     const long long nch = (long long)pr->n_voxels * pr->n_offsets;
-    if ((s = workspace(align256(nrec * recb) + 256 + align256(sizeof(int4) * pr->n_offsets) + order_bytes(nch), st,
-                       &ws)) != BMC_OK)
+    const size_t per_node = (size_t)nch * (pr->mz_loc >= 0 ? 1 : Layout<NC>::N);
+    const bool split = split_nodes(nch, sp, per_node);
+    const size_t part = split ? per_node * sp->n_nodes : 0;
+    Trains<NC> tn;
+    // the counting calls integrate event by event: their counts are the work of that
+    const bool trains = pr->precision != BMC_F32 && !work && Trains<NC>::wanted(pr);
+    if ((s = workspace(align256(nrec * recb) + 256 + align256(sizeof(int4) * pr->n_offsets) + order_bytes(nch) +
+                           align256(part * sizeof(double)) +
+                           (trains ? tn.bytes(pr, split ? nch * sp->n_nodes : nch, 0) : 0), st, &ws)) != BMC_OK)
         return s;
     Carve cv(ws);
     ChainArgs a{};
@@ -217,12 +358,13 @@ bmc_status Impl<NC>::simulate(const bmc_problem* pr, const double* params, const
     a.params = params; a.m0 = m0; a.out = out; a.work = work;
     a.status = cv.take<int>(1);
     CUDA_TRY(cudaMemsetAsync(a.status, 0, sizeof(int), st));
+    if (split) a.node_out = cv.take<double>(part);
     if (pr->precision == BMC_F32) {
         EvRec<float>* rec = cv.take<EvRec<float>>(nrec);
         if ((s = prep_events<float>(pr, ev, rec, st)) != BMC_OK) return s;
         a.ev = rec;
         if ((s = order_chains<NC, float>(a, cv, st)) != BMC_OK) return s;
-        return launch_chain<NC, float, 0>(a, tt, st);
+        return run_primal<NC, float>(a, tt, st);
     }
     EvRec<double>* rec = cv.take<EvRec<double>>(nrec);
     if ((s = prep_events<double>(pr, ev, rec, st)) != BMC_OK) return s;
@@ -231,7 +373,9 @@ bmc_status Impl<NC>::simulate(const bmc_problem* pr, const double* params, const
     if ((s = scan_blocks(rec, pr->n_offsets, pr->n_events, pr->n_offsets, const_cast<int4*>(a.seg), st)) != BMC_OK)
         return s;
     if ((s = order_chains<NC, double>(a, cv, st)) != BMC_OK) return s;
-    return launch_chain<NC, double, 0>(a, tt, st);
+    if (!trains) return run_primal<NC, double>(a, tt, st);
+    if ((s = tables(BMC_F64, &tn.tt64)) != BMC_OK || (s = tn.scan(a, rec, cv, st)) != BMC_OK) return s;
+    return run_primal<NC, double>(a, tt, st, &tn);
 }
 
 template <int NC>
@@ -268,8 +412,15 @@ bmc_status Impl<NC>::jvp(const bmc_problem* pr, const double* params, const bmc_
     const size_t nrec = (size_t)pr->n_offsets * pr->n_events;
     void* ws = nullptr;
     const long long nch = (long long)pr->n_voxels * pr->n_offsets;
+    const size_t per_node = (size_t)nch * (1 + tg->n_tangents);
+    const bool split = split_nodes(nch, sp, per_node);
+    const size_t part = split ? (size_t)nch * sp->n_nodes : 0;
+    Trains<NC> tn;
+    const bool trains = !work && Trains<NC>::wanted(pr);         // counting calls: event by event
+    const size_t train_bytes = trains ? tn.bytes(pr, split ? nch * sp->n_nodes : nch, tangents_per_pass<NC>()) : 0;
     if ((s = workspace(align256(nrec * sizeof(EvRec<double>)) + 256 + align256(sizeof(int4) * pr->n_offsets) +
-                           align256(sizeof(int) * pr->n_offsets) + 256 + order_bytes(nch), st, &ws)) != BMC_OK)
+                           align256(sizeof(int) * pr->n_offsets) + 512 + order_bytes(nch) +
+                           align256(part * (1 + tg->n_tangents) * sizeof(double)) + train_bytes, st, &ws)) != BMC_OK)
         return s;
     Carve cv(ws);
     ChainArgs a{};
@@ -293,7 +444,14 @@ bmc_status Impl<NC>::jvp(const bmc_problem* pr, const double* params, const bmc_
     if ((s = use_adjoint(rec, pr, tg->n_tangents, row_ev, flag, st, &adj)) != BMC_OK) return s;
     if ((s = order_chains<NC, double>(a, cv, st)) != BMC_OK) return s;
     if (adj) return launch_adjoint<NC>(a, row_ev, tg->n_tangents, tt, st);
-    return run_tangents<NC>(a, tg->n_tangents, tt, st);
+    if (split) {
+        a.node_out = cv.take<double>(part);
+        a.node_jout = cv.take<double>(part * tg->n_tangents);
+    }
+    if (!trains) return run_tangents<NC>(a, tg->n_tangents, tt, st);
+    tn.tt64 = tt;
+    if ((s = tn.scan(a, rec, cv, st)) != BMC_OK) return s;
+    return run_tangents<NC>(a, tg->n_tangents, tt, st, &tn);
 }
 
 // Z, its tangents and the derivatives of both along one design direction (design_kernel): one launch
@@ -357,13 +515,19 @@ bmc_status Impl<NC>::lm(const bmc_problem* pr, const double* params, const bmc_e
     const int nv = pr->n_voxels, no = pr->n_offsets, P = fs->n_params;
     constexpr int NF = Layout<NC>::NF, N = Layout<NC>::N;
     const size_t nrec = (size_t)no * pr->n_events;
+    const bool split = split_nodes((long long)nv * no, sp, (size_t)nv * no * (1 + P));
+    const size_t part = split ? (size_t)nv * no * sp->n_nodes : 0;
+    Trains<NC> tn;
+    const bool trains = Trains<NC>::wanted(pr);
     const size_t bytes = align256(nrec * sizeof(EvRec<double>)) + 2 * align256(sizeof(double) * NF * nv) +
                          2 * align256(sizeof(double) * N * nv) + 2 * align256(sizeof(double) * nv) +
                          align256(sizeof(double) * P * nv) + align256(sizeof(double) * P * nv * N) +
                          2 * align256(sizeof(double) * nv * no) + align256(sizeof(double) * P * nv * no) +
                          2 * align256(sizeof(double) * nv * P) + 2 * align256(sizeof(double) * nv) +
                          align256(sizeof(int) * nv) + align256(sizeof(int4) * no) + 4096 +
-                         align256(sizeof(int) * no) + 256 + order_bytes((long long)nv * no);
+                         align256(sizeof(int) * no) + 512 + order_bytes((long long)nv * no) +
+                         align256(part * (1 + P) * sizeof(double)) +
+                         (trains ? tn.bytes(pr, (long long)nv * no * (split ? sp->n_nodes : 1), tangents_per_pass<NC>()) : 0);
     void* ws = nullptr;
     if ((s = workspace(bytes, st, &ws)) != BMC_OK) return s;
     Carve cv(ws);
@@ -415,6 +579,15 @@ bmc_status Impl<NC>::lm(const bmc_problem* pr, const double* params, const bmc_e
     if ((s = use_adjoint(rec, pr, P, row_ev, flag, st, &adj)) != BMC_OK) return s;
     a.params = params; a.m0 = m0;
     if ((s = order_chains<NC, double>(a, cv, st)) != BMC_OK) return s;
+    if (split && !adj) {
+        a.node_out = cv.take<double>(part);
+        a.node_jout = cv.take<double>(part * P);
+    }
+    const TaylorTable* ttf = nullptr;
+    if ((s = tables(kTableFit, &ttf)) != BMC_OK) return s;
+    const Trains<NC>* tp = trains && !adj ? &tn : nullptr;
+    tn.tt64 = tt;
+    if (tp && (s = tn.scan(a, rec, cv, st)) != BMC_OK) return s;
     for (int p = 0; p < P; ++p) a.field_row[p] = fs->field_row[p] == BMC_SLOT_M_START ? BMC_SEED_NONE : fs->field_row[p];
     const int vb = (nv + 127) / 128, wb = (nv + 3) / 4;
     for (int it = 0; it < fs->n_iter; ++it) {
@@ -425,9 +598,9 @@ bmc_status Impl<NC>::lm(const bmc_problem* pr, const double* params, const bmc_e
         ChainArgs aj = a;
         aj.params = px; aj.m0 = m0x; aj.sigma = sp ? sgx : nullptr; aj.seed = seed; aj.dm0 = has_m ? dm0 : nullptr;
         aj.active = need; aj.out = z; aj.jout = J;
-        if ((s = adj ? launch_adjoint<NC>(aj, row_ev, P, tt, st) : run_tangents<NC>(aj, P, tt, st)) != BMC_OK)
+        if ((s = adj ? launch_adjoint<NC>(aj, row_ev, P, tt, st) : run_tangents<NC>(aj, P, tt, st, tp)) != BMC_OK)
             return s;
-        lm_solve_kernel<<<wb, 128, 0, st>>>(nv, no, fs->n_points_skip, ss, z, zm, J, fs->d_free, x, lam, cost, xt);
+        lm_solve_kernel<<<wb, 128, 0, st>>>(nv, no, fs->n_points_skip, it, ss, z, zm, J, fs->d_free, x, lam, cost, xt);
         CUDA_TRY(cudaGetLastError());
         // the trial point
         lm_params_kernel<NC><<<vb, 128, 0, st>>>(nv, ss, params, m0, sig0, xt, fs->d_free, pt, m0t,
@@ -436,7 +609,7 @@ bmc_status Impl<NC>::lm(const bmc_problem* pr, const double* params, const bmc_e
         ChainArgs at = a;
         at.params = pt; at.m0 = m0t; at.sigma = sp ? sgt : nullptr; at.out = zt;
         // the trial point's Z: with the adjoint tangents, the same dense layout without H
-        if ((s = adj ? launch_adjoint<NC, false>(at, row_ev, 0, tt, st) : launch_chain<NC, double, 0>(at, tt, st)) !=
+        if ((s = adj ? launch_adjoint<NC, false>(at, row_ev, 0, tt, st) : run_primal<NC, double>(at, ttf, st, tp)) !=
             BMC_OK)
             return s;
         lm_accept_kernel<<<wb, 128, 0, st>>>(nv, no, fs->n_points_skip, P, it, fs->n_iter, zt, zm, cost, xt, x,
@@ -467,6 +640,17 @@ bmc_status run_noalloc(const bmc_problem* pr, const double* params, const bmc_ev
     if constexpr (std::is_same<R, double>::value) {
         if ((s = scan_blocks(rec, pr->n_offsets, pr->n_events, pr->n_offsets, ws.seg, st)) != BMC_OK) return s;
         a.seg = ws.seg;
+        Trains<NC> tn;
+        if (Trains<NC>::wanted(pr)) {
+            // as many chains at a time as the static array holds (its size covers every table's amplitudes)
+            const size_t fixed = tn.fixed_bytes(pr, 0);
+            tn.chunk = std::min<long long>((long long)pr->n_voxels * pr->n_offsets,
+                                           (long long)((ws.train_bytes - fixed) / tn.per_chain()));
+            tn.tt64 = ws.tt64;
+            Carve cv(ws.train);
+            if ((s = tn.scan(a, rec, cv, st)) != BMC_OK) return s;
+            return run_primal<NC, double>(a, tt, st, &tn);
+        }
     }
     return launch_chain<NC, R, 0>(a, tt, st);
 }

@@ -27,6 +27,10 @@ __device__ __forceinline__ R warp_max(R x) {
 // the block propagator's columns by the truncated Taylor series instead)
 constexpr double kBlockDenseNorm = 4.0;
 
+// the norm above which a free event without transverse magnetisation takes its z block alone (Chain::z_event): its
+// ~11 Horner steps of NC + 3 columns and ~10 squarings cost what the Taylor action costs at a norm of about 8
+constexpr double kZFreeNorm = 8.0;
+
 // lanes per chain in the dense path: one column per lane, so a warp works on 32 / GS chains at once
 template <int NC>
 struct DenseGroup {
@@ -445,6 +449,83 @@ __device__ __forceinline__ void convert_flat(const A& a, B& b) {
 }
 
 // ------------------------------------------------------------------------------------------------
+// propagators of shaped pulses (formed by train_kernel, bmc_train.cuh)
+// ------------------------------------------------------------------------------------------------
+template <int NC>
+struct TrainShape {
+    static constexpr int N = Layout<NC>::N;
+    static constexpr int NT = (N + 7) / 8;                   // tiles of 8
+    // column stride of a matrix in shared memory: even, and 4 modulo 8 in 16-byte units, so that the eight lanes of a
+    // 128-bit read (two columns x four row pairs) fall on distinct banks
+    static constexpr int LD = NT == 1 ? 8 : 24;
+    static constexpr int TS = 8 * NT * LD;                   // doubles of one matrix
+    static constexpr int kSlots = 6;
+    static constexpr int NS = (N + 2) & ~1;                  // row of the stored propagator: N entries, phi, padding
+    // warps per block: the shared memory of a warp (19 KB with four pools) sets the resident warps, so small blocks
+    static constexpr int kWarps = NT == 1 ? 4 : 1;
+    static constexpr int kBlocks = NT == 1 ? 4 : (NT == 2 ? 11 : 7);   // resident blocks the registers are kept for
+};
+
+// M <- R(phase) [P R(-phase) M + phi], P from the propagator `p` (the turned frame's x is along the RF); with tangents
+// their derivatives' propagators follow: dM <- R [P R^-1 dM + dP R^-1 M + dphi]
+template <int NC, int NT>
+__device__ __noinline__ void train_apply(const double* __restrict__ p, double c, double s, State<NC, Dn<double, NT>>& M) {
+    using D = Dn<double, NT>;
+    using C = Chain<NC, double, NT>;
+    constexpr int N = TrainShape<NC>::N, NS = TrainShape<NC>::NS;
+    auto turn = [](D& x, D& y, double c, double s) {
+        const D a = c * x + s * y;
+        y = c * y - s * x;
+        x = a;
+    };
+    turn(M.xw, M.yw, c, s);
+#pragma unroll
+    for (int i = 0; i < NC; ++i) turn(M.xc[i], M.yc[i], c, s);
+    D out[N];
+#pragma unroll 2
+    for (int i = 0; i < N; ++i) {
+        D acc0 = dconst<double, NT>(0.0), acc1 = acc0;
+        const double2* q = reinterpret_cast<const double2*>(p + i * NS);
+#pragma unroll
+        for (int j = 0; j < NS / 2; ++j) {
+            const double2 x = q[j];
+            auto add = [&](D& acc, int col, double P) {
+                if (col > N) return;
+                if (col == N) {
+                    acc.v += P;
+                    return;
+                }
+                const D& m = C::at(M, col);
+                acc.v = fma(P, m.v, acc.v);
+                DN_LOOP(acc.d[t] = fma(P, m.d[t], acc.d[t]));
+            };
+            add(acc0, 2 * j, x.x);
+            add(acc1, 2 * j + 1, x.y);
+        }
+        if constexpr (NT > 0) {
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+                const double2* dq = reinterpret_cast<const double2*>(p + ((1 + t) * N + i) * NS);
+#pragma unroll
+                for (int j = 0; j < NS / 2; ++j) {
+                    const double2 x = dq[j];
+                    if (2 * j < N) acc0.d[t] = fma(x.x, C::at(M, 2 * j).v, acc0.d[t]);
+                    else if (2 * j == N) acc0.d[t] += x.x;
+                    if (2 * j + 1 < N) acc1.d[t] = fma(x.y, C::at(M, 2 * j + 1).v, acc1.d[t]);
+                    else if (2 * j + 1 == N) acc1.d[t] += x.y;
+                }
+            }
+        }
+        out[i] = acc0 + acc1;
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) C::at(M, i) = out[i];
+    turn(M.xw, M.yw, c, -s);
+#pragma unroll
+    for (int i = 0; i < NC; ++i) turn(M.xc[i], M.yc[i], c, -s);
+}
+
+// ------------------------------------------------------------------------------------------------
 // the chain kernel
 // ------------------------------------------------------------------------------------------------
 // COUNT: the launch adds its work counts to a.work (the measurement entry points); the other launches
@@ -464,9 +545,15 @@ chain_kernel(const ChainArgs a, const __grid_constant__ TaylorTable tt) {
     // chains in offset-fastest order: neighbouring lanes are neighbouring offsets of one voxel, so a
     // warp shares parameters and its chains need similar Taylor orders
     const long long nch = UNEVEN ? a.n_chains : (long long)a.n_vox * a.n_off;
-    long long ci = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = ci < nch;
-    if (!valid) ci = nch - 1;
+    const long long all = a.chain_count ? a.chain_count : (a.node_out ? nch * a.n_nodes : nch);
+    const long long first = ((long long)blockIdx.x * ChainLaunch<NC, NT>::kWarps + (threadIdx.x >> 5)) * a.cpw;
+    long long ci = first + lane;
+    const bool valid = lane < a.cpw && ci < all;
+    if (!valid) ci = first < all ? first : all - 1;
+    const long long pos = ci;
+    ci += a.first_chain;
+    const int node0 = a.node_out ? (int)(ci / nch) : a.node_lo, node1 = a.node_out ? node0 + 1 : a.node_hi;
+    if (a.node_out) ci -= node0 * nch;
     if (a.order) ci = a.order[ci];                     // chains sorted by estimated cost (see cost_kernel)
     int v, o;
     const EvRec<R>* __restrict__ ev = reinterpret_cast<const EvRec<R>*>(a.ev);
@@ -498,13 +585,17 @@ chain_kernel(const ChainArgs a, const __grid_constant__ TaylorTable tt) {
     const int blk_end = use_blk ? blk.x + blk.z * blk.y : 0;
     const bool act = valid && (a.active == nullptr || a.active[v] != 0);
     if (__all_sync(kFull, !act)) return;
+    // the chain's shaped pulses have a propagator (float64 kernels)
+    constexpr bool kTrain = !UNEVEN && !COUNT && std::is_same<R, double>::value;
+    bool train = false;
+    if constexpr (kTrain) train = a.prop && act && a.train[o].n > 0 && a.prop_ok[pos] != 0;
 
     const size_t ch = UNEVEN ? (size_t)ci : (size_t)v * a.n_off + o;
     unsigned wk0 = 0, wk1 = 0, wk2 = 0, wk3 = 0, wk4 = 0;   // this chain's work counts (each < 2^32 per launch)
     constexpr bool count = COUNT;
     ChainConst<NC, D>& cc =
         reinterpret_cast<ChainConst<NC, D>*>(smem_raw + ChainLaunch<NC, NT>::kWarps * sizeof(SM))[threadIdx.x];
-    for (int node = 0; node < a.n_nodes; ++node) {
+    for (int node = node0; node < node1; ++node) {
         {
             ChainConst<NC, D> tmp;
             C::load_const(a, v, node, tmp);
@@ -523,6 +614,7 @@ chain_kernel(const ChainArgs a, const __grid_constant__ TaylorTable tt) {
         // the frequency-dependent base of the norm bound, kept while the events' frequency stays fkey
         R fkey = R(NAN);
         typename C::NormBase nb{R(0), R(0)};
+        int train_end = 0;                             // the events before this one are in the propagator
         for (int e = 0; e < n_ev_loop; ++e) {
             // past the end of its own table a lane sees an empty DELAY: no evolution, spoiler or readout
             const bool in = !UNEVEN || e < n_ev_own;
@@ -543,8 +635,27 @@ chain_kernel(const ChainArgs a, const __grid_constant__ TaylorTable tt) {
                     Dense<NC, R, NT>::block(dsm, lane, bstart, ev + o, stride, blk.x, blk.y, blk.z, cc, M, tt, a.status,
                                             count, wk0, wk1, wk2);
             }
-            const bool skip = use_blk && e >= blk.x && e < blk_end;
-            const int type = skip ? EV_DELAY : (int)rec.type;
+            // a shaped pulse: its propagator at its first event; the warp goes on at the next event any lane needs
+            int type = (int)rec.type;
+            if constexpr (kTrain) {
+                const bool tstart = train && (type & kTrainMark) != 0 && e >= train_end;
+                type &= kTrainMark - 1;
+                if (tstart) {
+                    State<NC, D> Mt = M;
+                    train_apply<NC, NT>(a.prop + (size_t)pos * (1 + NT) * N * TrainShape<NC>::NS, rec.c, rec.s, Mt);
+                    M = Mt;
+                    train_end = e + a.train[o].span;
+                }
+                if (__any_sync(kFull, tstart)) {
+                    const int next = (int)__reduce_min_sync(kFull, act ? (unsigned)train_end : 0x7fffffffu);
+                    if (next > e + 1) {
+                        e = next - 1;
+                        continue;
+                    }
+                }
+            }
+            const bool skip = (use_blk && e >= blk.x && e < blk_end) || (kTrain && e < train_end);
+            if (skip) type = EV_DELAY;
             const bool evolve = act && !skip && rec.dt > R(1e-9);
             if (__any_sync(kFull, evolve)) {
                 D g = dconst<R, NT>(R(0));
@@ -572,7 +683,18 @@ chain_kernel(const ChainArgs a, const __grid_constant__ TaylorTable tt) {
                 }
                 // this chain's own choice: dense scaling and squaring for a large norm, else the
                 // Taylor action with the fewest terms whose tail bound meets the tolerance
-                const bool dense_own = evolve && nu > dswitch;
+                // a free event without transverse magnetisation: the z block alone (the counting kernel keeps to
+                // the general path, whose work it counts)
+                bool zfree = false;
+                if constexpr (std::is_same<R, RD>::value && !COUNT) {
+                    zfree = evolve && rec.w1 == R(0) && nu > R(kZFreeNorm) && nu < R(1e50) && C::longitudinal(M);
+                    if (zfree) {
+                        State<NC, D> Mt = M;
+                        C::z_event(cc, rec.dt, Mt, tt);
+                        M = Mt;
+                    }
+                }
+                const bool dense_own = evolve && !zfree && nu > dswitch;
                 if (__any_sync(kFull, dense_own)) {
                     StepCoef<NC, D> sc;                            // unscaled: the dense path scales by dt / 2^s
                     C::event_coef(cc, rec, g, sc);
@@ -588,7 +710,7 @@ chain_kernel(const ChainArgs a, const __grid_constant__ TaylorTable tt) {
                         convert_flat<RD, R, NT>(Md, M);
                     }
                 }
-                const bool tay = evolve && !dense_own;
+                const bool tay = evolve && !dense_own && !zfree;
                 int m_own = 0, ns_own = 0;
                 if (tay) {
                     ns_own = nu > thm ? (int)ceil(nu / thm) : 1;
@@ -602,19 +724,17 @@ chain_kernel(const ChainArgs a, const __grid_constant__ TaylorTable tt) {
                     m_prev = m;
                     m_own = m;
                 }
-                const int ns_w = __reduce_max_sync(kFull, (unsigned)ns_own);
-                const int m_w = __reduce_max_sync(kFull, (unsigned)m_own);
-                if (ns_w > 0) {
-                    const R h = tay ? (ns_own == 1 ? rec.dt : rec.dt / R(ns_own)) : R(0);
-                    const int passes = C::taylor_apply(cc, rec, g, h, ns_w, m_w, ns_own, m_own, M, tt);
-                    if (count && tay) {
+                if (tay) {
+                    const R h = ns_own == 1 ? rec.dt : rec.dt / R(ns_own);
+                    C::taylor_apply(cc, rec, g, h, ns_own, m_own, M, tt);
+                    if (count) {
                         wk0 += unsigned(ns_own * m_own);
                         // of those, the terms formed in float32 (all of them in the float32 kernel)
                         const int k32 = std::is_same<R, float>::value ? 1 : (NT == 0 ? tt.f32_from[m_own] : m_own + 1);
                         wk4 += unsigned(ns_own * (m_own + 1 - k32));
                     }
-                    if (count) wk3 += unsigned(passes * m_w);
                 }
+                if (count) wk3 += __reduce_max_sync(kFull, (unsigned)(ns_own * m_own));
             }
             if (type == EV_GRADIENT || type == EV_SPOILER) C::spoil(M);
             if (a.traj != nullptr && act && in) {
@@ -627,26 +747,32 @@ chain_kernel(const ChainArgs a, const __grid_constant__ TaylorTable tt) {
         // last_M of this isochromat, weighted into the spread mean (written by the chain's own thread)
         if (act) {
             const R wgt = a.n_nodes > 1 ? R(a.w[node]) : R(1);
+            const bool more = !a.node_out && node > 0;   // earlier nodes of this chain are in the output already
+            // the weighted sum in one fused step per node (float32 products rounded first), here or in node_sum_kernel:
+            // the same bits whether the nodes run in a loop or as chains of their own
+            auto put = [&](double* p, R x) {
+                if constexpr (std::is_same<R, double>::value)
+                    *p = a.node_out ? x : fma(wgt, x, more ? *p : 0.0);
+                else
+                    *p = (more ? *p : 0.0) + double(wgt * x);
+            };
+            double* out = a.node_out ? a.node_out + (size_t)node * nch * (a.mz >= 0 ? 1 : N) : a.out;
             if (a.mz >= 0) {
                 D z = dconst<R, NT>(R(0));
 #pragma unroll
                 for (int q = 0; q < N; ++q)
                     if (q == a.mz) z = C::at(M, q);
-                a.out[ch] = (node ? a.out[ch] : 0.0) + double(wgt * z.v);
+                put(out + ch, z.v);
                 if constexpr (NT > 0) {
-                    if (a.jout) {
+                    double* jout = a.node_out ? a.node_jout + (size_t)node * a.n_tan * nch : a.jout;
+                    if (jout) {
 #pragma unroll
-                        for (int t = 0; t < NT; ++t) {
-                            double* jp = UNEVEN ? a.jout + (size_t)(a.t0 + t) * a.n_chains + ch
-                                                : a.jout + ((size_t)(a.t0 + t) * a.n_vox + v) * a.n_off + o;
-                            *jp = (node ? *jp : 0.0) + double(wgt * z.d[t]);
-                        }
+                        for (int t = 0; t < NT; ++t) put(jout + (size_t)(a.t0 + t) * nch + ch, z.d[t]);
                     }
                 }
             } else {
 #pragma unroll
-                for (int q = 0; q < N; ++q)
-                    a.out[ch * N + q] = (node ? a.out[ch * N + q] : 0.0) + double(wgt * C::at(M, q).v);
+                for (int q = 0; q < N; ++q) put(out + ch * N + q, C::at(M, q).v);
             }
         }
     }
@@ -660,6 +786,22 @@ chain_kernel(const ChainArgs a, const __grid_constant__ TaylorTable tt) {
             if (lane == 0 && x) atomicAdd(a.work + q, x);
         }
     }
+}
+
+// out[i] = sum over the nodes of w[node] part[node][i] (float64 kernels; float32: the parts are weighted already),
+// i < n, in node order (the order of a chain that loops over its nodes); n a multiple of n_vox * n_off chains, voxels
+// with active 0 left as they are
+template <bool WEIGH>
+static __global__ void __launch_bounds__(256) node_sum_kernel(const ChainArgs a, const double* __restrict__ part,
+                                                              long long n, double* __restrict__ out) {
+    const long long i = blockIdx.x * 256ll + threadIdx.x;
+    if (i >= n || (a.active && !a.active[i / a.n_off % a.n_vox])) return;
+    double x = 0.0;
+    for (int j = 0; j < a.n_nodes; ++j) {
+        const double y = part[(size_t)j * n + i];
+        x = WEIGH ? fma(a.w[j], y, x) : x + y;
+    }
+    out[i] = x;
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -691,7 +833,7 @@ __global__ void __launch_bounds__(128) cost_kernel(const ChainArgs a, float* __r
     float cost = 0.f;
     for (int e = 0; e < n_ev; ++e) {
         const EvRec<R> rec = ev[(size_t)e * stride + o];
-        if ((int)rec.type != EV_RF || !(rec.dt > R(1e-9))) continue;
+        if (((int)rec.type & (kTrainMark - 1)) != EV_RF || !(rec.dt > R(1e-9))) continue;
         ChainConst<NC, D> cc;
         C::load_const(a, v, 0, cc);
         StepCoef<NC, D> sc;
@@ -719,66 +861,85 @@ __device__ __forceinline__ bool same_rec(const EvRec<R>& x, const EvRec<R>& y) {
     return x.dt == y.dt && x.w1 == y.w1 && x.c == y.c && x.s == y.s && x.wf == y.wf && x.type == y.type;
 }
 
-// One thread per (row, block length): kBlockScanRows rows of kBlockMaxL threads per block. Each thread
-// walks its row for its own L (the candidates at increasing start, the first largest saving kept);
-// the row's first thread then takes the largest saving over L = 1 .. kBlockMaxL in that order, so ties
-// go to the shortest block and then the earliest start.
-constexpr int kBlockScanRows = 16;
-constexpr int kBlockScanThreads = kBlockScanRows * kBlockMaxL;
+// One block per row, warp L - 1 taking block length L: the warp compares 128 events with those L later at a time
+// (bit e of its ballots: event e equals event e + L) and walks the zeros of the bits. From a start a, c ones give
+// r = 1 + c / L copies; with r < 2 no start up to the zero can do better, so the walk goes on behind it. The
+// candidates come at increasing start, the first largest saving is kept; thread 0 then takes the largest over
+// L = 1 .. kBlockMaxL in that order, so ties go to the shortest block and then the earliest start.
+// Bound by the latency of the record loads: a thread per (row, L) that compared one event after another took
+// 1.7 ms on 101 rows x 4,023 events, the warps take 84 us.
+constexpr int kBlockScanThreads = 32 * kBlockMaxL;
 
 template <typename R>
-__global__ void __launch_bounds__(kBlockScanThreads) block_scan_kernel(const EvRec<R>* __restrict__ ev, int n_rows,
-                                                                       int n_ev, int stride, int4* __restrict__ seg) {
-    __shared__ long long sv[kBlockScanThreads];
-    __shared__ int4 sb[kBlockScanThreads];
-    const int tid = threadIdx.x;
-    const int o = blockIdx.x * kBlockScanRows + tid / kBlockMaxL;
-    const int L = tid % kBlockMaxL + 1;
+__global__ void __launch_bounds__(kBlockScanThreads) block_scan_kernel(const EvRec<R>* __restrict__ ev, int n_ev,
+                                                                       int stride, int4* __restrict__ seg) {
+    __shared__ long long sv[kBlockMaxL];
+    __shared__ int4 sb[kBlockMaxL];
+    const int lane = threadIdx.x & 31, L = (threadIdx.x >> 5) + 1;
+    const EvRec<R>* row = ev + blockIdx.x;
     int4 best = make_int4(0, 0, 0, 0);
     long long best_save = 0;
-    if (o < n_rows) {
-        const EvRec<R>* row = ev + o;
-        int a = 0;
-        while (a + 2 * L <= n_ev) {
-            int r = 1;
-            while (a + (r + 1) * L <= n_ev) {
-                bool eq = true;
-                for (int j = 0; j < L && eq; ++j)
-                    eq = same_rec(row[(size_t)(a + j) * stride], row[(size_t)(a + r * L + j) * stride]);
-                if (!eq) break;
-                ++r;
+    auto candidate = [&](int a, int r) {
+        bool adc = false, moves = false, long_ev = false;
+        for (int j = 0; j < L; ++j) {
+            const EvRec<R> x = row[(size_t)(a + j) * stride];
+            adc |= (int)x.type == EV_ADC;
+            moves |= x.dt > R(1e-9);
+            long_ev |= x.dt >= R(kBlockMinDt);
+        }
+        const long long save = (long long)(r - 1) * L;
+        if (!adc && moves && (long_ev || r >= kBlockMinRepeats) && save > best_save) {
+            best = make_int4(a, L, r, 0);
+            best_save = save;
+        }
+    };
+    const int n_eq = n_ev - L;                 // event e has a partner for e < n_eq
+    int a = 0;
+    for (int base = 0; base < n_eq; base += 128) {
+        unsigned w[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int e = base + 32 * q + lane;
+            w[q] = __ballot_sync(kFull, e < n_eq && same_rec(row[(size_t)e * stride], row[(size_t)(e + L) * stride]));
+        }
+#pragma unroll 1
+        for (int q = 0; q < 4; ++q) {
+            const int e0 = base + 32 * q;
+            const unsigned ones = w[q];
+            int pos = a > e0 ? a - e0 : 0;     // bits below pos are behind the walk
+            while (pos < 32) {
+                const unsigned z = ~ones >> pos;
+                if (!z) break;                 // the run goes on into the next word
+                const int e = e0 + pos + __ffs(z) - 1, c = e - a;
+                if (c >= L) {
+                    const int r = 1 + c / L;
+                    candidate(a, r);
+                    a += r * L;
+                } else {
+                    // behind this zero and the zeros that follow it
+                    pos = e - e0 + 1;
+                    const unsigned rest = pos < 32 ? ones >> pos : 0u;
+                    a = rest ? e0 + pos + __ffs(rest) - 1 : e0 + 32;
+                }
+                pos = a - e0;
             }
-            if (r < 2) {
-                ++a;
-                continue;
-            }
-            bool adc = false, moves = false, long_ev = false;
-            for (int j = 0; j < L; ++j) {
-                const EvRec<R> x = row[(size_t)(a + j) * stride];
-                adc |= (int)x.type == EV_ADC;
-                moves |= x.dt > R(1e-9);
-                long_ev |= x.dt >= R(kBlockMinDt);
-            }
-            const long long save = (long long)(r - 1) * L;
-            if (!adc && moves && (long_ev || r >= kBlockMinRepeats) && save > best_save) {
-                best = make_int4(a, L, r, 0);
-                best_save = save;
-            }
-            a += r * L;
         }
     }
-    sv[tid] = best_save;
-    sb[tid] = best;
+    if (n_eq - a >= L) candidate(a, 1 + (n_eq - a) / L);
+    if (lane == 0) {
+        sv[L - 1] = best_save;
+        sb[L - 1] = best;
+    }
     __syncthreads();
-    if (o < n_rows && L == 1) {
+    if (threadIdx.x == 0) {
         long long bs = 0;
         int4 bb = make_int4(0, 0, 0, 0);
         for (int l = 0; l < kBlockMaxL; ++l)
-            if (sv[tid + l] > bs) {
-                bs = sv[tid + l];
-                bb = sb[tid + l];
+            if (sv[l] > bs) {
+                bs = sv[l];
+                bb = sb[l];
             }
-        seg[o] = bb;
+        seg[blockIdx.x] = bb;
     }
 }
 

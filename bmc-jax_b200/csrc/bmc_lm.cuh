@@ -154,8 +154,11 @@ __device__ __forceinline__ void gauss_solve(int P, double* A, double* b) {
     }
 }
 
-// normal equations, the damped solve and the clipped trial point
-static __global__ void lm_solve_kernel(int n_vox, int n_off, int skip, const SlotSpec sp, const double* __restrict__ z,
+// Normal equations, the damped solve and the clipped trial point. The cost at x is taken from these residuals in the
+// first iteration only; later it is the accepted trial point's (lm_accept_kernel), so that the costs that are compared
+// come from the same kernels: the tangent and the primal passes agree to ~1e-13, and near a minimum a step lowers
+// the cost by less than that.
+static __global__ void lm_solve_kernel(int n_vox, int n_off, int skip, int it, const SlotSpec sp, const double* __restrict__ z,
                                 const double* __restrict__ zm, const double* __restrict__ J,
                                 const double* __restrict__ freem, const double* __restrict__ x,
                                 const double* __restrict__ lam, double* __restrict__ cost, double* __restrict__ xt) {
@@ -168,7 +171,7 @@ static __global__ void lm_solve_kernel(int n_vox, int n_off, int skip, const Slo
     double c, g[kMaxT], H[kMaxT * kMaxT];
     normal_sums(lane, v, n_vox, n_off, skip, P, z, zm, J, fr, c, g, H);
     if (lane != 0) return;
-    cost[v] = c;
+    if (it == 0) cost[v] = c;
     const double l = lam[v];
     double A[kMaxT * kMaxT], b[kMaxT];
     for (int p = 0; p < P; ++p) {
@@ -187,7 +190,7 @@ static __global__ void lm_solve_kernel(int n_vox, int n_off, int skip, const Slo
 // accept or reject every voxel's trial point
 static __global__ void lm_accept_kernel(int n_vox, int n_off, int skip, int P, int it, int n_iter,
                                  const double* __restrict__ zt, const double* __restrict__ zm,
-                                 const double* __restrict__ cost, const double* __restrict__ xt,
+                                 double* __restrict__ cost, const double* __restrict__ xt,
                                  double* __restrict__ x, double* __restrict__ lam, int* __restrict__ need,
                                  double* __restrict__ cost_traj, double* __restrict__ x_traj) {
     const int lane = threadIdx.x & 31;
@@ -208,7 +211,8 @@ static __global__ void lm_accept_kernel(int n_vox, int n_off, int skip, int P, i
     }
     lam[v] = better ? lam[v] * 0.5 : lam[v] * 3.0;
     need[v] = better ? 1 : 0;
-    if (cost_traj) cost_traj[(size_t)v * n_iter + it] = better ? cn : cost[v];
+    if (better) cost[v] = cn;
+    if (cost_traj) cost_traj[(size_t)v * n_iter + it] = cost[v];
     if (x_traj) {
         for (int p = 0; p < P; ++p) x_traj[((size_t)v * n_iter + it) * P + p] = x[(size_t)v * P + p];
     }
