@@ -152,12 +152,18 @@ def check(status: int) -> None:
         raise RuntimeError(f"bmc_b200 error {status}: {buf.value.decode(errors='replace')}")
 
 
+_torch = None
+
+
 def torch_cuda():
     """torch, with a CUDA device required (the product path has no CPU fallback)."""
-    import torch
-    if not torch.cuda.is_available():
-        raise RuntimeError("bmc_b200 needs a CUDA device (B200, sm_100a); none is available")
-    return torch
+    global _torch
+    if _torch is None:
+        import torch
+        if not torch.cuda.is_available():
+            raise RuntimeError("bmc_b200 needs a CUDA device (B200, sm_100a); none is available")
+        _torch = torch
+    return _torch
 
 
 def ptr(t) -> C.c_void_p:

@@ -3,7 +3,7 @@ from typing import Dict, Sequence, Tuple
 
 import numpy as np
 
-from .simulation import SimParams, SimEvent, simulate_z
+from .simulation import SimParams, SimEvent, _simulate
 
 __all__ = ["build_param_grid", "generate_dictionary"]
 
@@ -39,6 +39,7 @@ def generate_dictionary(base_params: SimParams, seq_base: SimEvent, M_init, grid
     for a in range(0, n, chunk_size):
         b = min(a + chunk_size, n)
         chunk = SimParams(*[np.asarray(v)[a:b] for v in pb])
-        fp[a:b] = simulate_z(chunk, seq_base, np.broadcast_to(np.asarray(M_init), (b - a, np.size(M_init))),
-                             water_z_index)
+        z = _simulate(chunk, seq_base, np.broadcast_to(np.asarray(M_init), (b - a, np.size(M_init))),
+                      int(water_z_index), device_out=True)
+        fp[a:b] = z.float().cpu().numpy()              # rounded on the device: half the bytes back
     return entries, fp

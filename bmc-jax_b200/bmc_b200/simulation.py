@@ -180,18 +180,19 @@ def repeat_events(events: SimEvent, n_reps: int) -> SimEvent:
 def pack_params(p: SimParams, n_vox: int) -> np.ndarray:
     """SimParams (one sample or a batch of n_vox) -> the ABI layout [13 + 5 n_cest][n_vox] float64."""
     nc = n_cest_of(p)
-    rows = []
+    out = np.empty((13 + 5 * nc, n_vox))
+    r = 0
     for k in SimParams._fields:
         v = np.asarray(getattr(p, k), dtype=np.float64)
         if k in POOL_FIELDS:
-            v = np.broadcast_to(v, (n_vox, nc)) if v.ndim <= 1 else v
-            if v.shape != (n_vox, nc):
+            if v.ndim > 1 and v.shape != (n_vox, nc):
                 raise ValueError(f"{k}: shape {v.shape} for {n_vox} samples of {nc} pools")
-            rows.extend(v.T)
+            out[r:r + nc] = v.T if v.ndim > 1 else np.broadcast_to(v, (nc,))[:, None]
+            r += nc
         else:
-            v = np.broadcast_to(v.reshape(-1) if v.ndim else v, (n_vox,))
-            rows.append(v)
-    return np.ascontiguousarray(np.stack(rows), dtype=np.float64)
+            out[r] = v.reshape(-1) if v.ndim else v
+            r += 1
+    return out
 
 
 def n_samples(p: SimParams) -> Optional[int]:
@@ -199,21 +200,46 @@ def n_samples(p: SimParams) -> Optional[int]:
     return int(np.shape(p.water_r1)[0]) if np.ndim(p.water_r1) > 0 else None
 
 
+# Arrays of up to this many bytes in all go up in one copy; a pageable copy of a few KB costs ~12 us of host time
+# whatever its size (one spectrum: 8 copies), while a larger one would only be copied twice.
+_PACK_BYTES = 1 << 18
+
+
+def upload(*arrays):
+    """(device tensors that hold them, their device addresses) of host arrays given as (array, dtype)."""
+    torch = _lib.torch_cuda()
+    arrays = [np.require(np.asarray(a, dt), requirements=["C"]) for a, dt in arrays]
+    at, total = [], 0
+    for a in arrays:
+        at.append(total)
+        total += (a.nbytes + 255) & ~255
+    if total <= _PACK_BYTES:
+        buf = np.empty(max(total, 1), np.uint8)
+        for a, o in zip(arrays, at):
+            buf[o:o + a.nbytes] = a.reshape(-1).view(np.uint8)
+        dev = torch.from_numpy(buf).to("cuda")
+        base = dev.data_ptr()
+        return [dev], [base + o for o in at]
+    devs = [torch.as_tensor(a if a.flags.writeable else np.require(a, requirements=["W"])).to("cuda") for a in arrays]
+    return devs, [d.data_ptr() for d in devs]
+
+
 class DeviceEvents:
     """An event table on the device (the six reference fields), kept alive for a C call."""
 
     def __init__(self, events: SimEvent):
-        torch = _lib.torch_cuda()
         dt = np.asarray(events.dt)
         if dt.ndim != 2:
             raise ValueError(f"events must be (n_offsets, n_events), got {dt.shape}")
         self.n_offsets, self.n_events = dt.shape
-        cuda = torch.device("cuda")
-        as_i = lambda a: torch.as_tensor(np.ascontiguousarray(np.asarray(a), np.int32)).to(cuda)
-        as_f = lambda a: torch.as_tensor(np.ascontiguousarray(np.asarray(a), np.float64)).to(cuda)
-        self.t = [as_i(events.type), as_f(events.dt), as_f(events.rf_amp), as_f(events.rf_phase),
-                  as_f(events.rf_freq), as_i(events.adc_idx)]
-        self.struct = _lib.Events(*[x.data_ptr() for x in self.t])
+        self.t, p = upload(*self.host_arrays(events))
+        self.struct = _lib.Events(*p, None)           # the library reads no adc_idx
+
+    @staticmethod
+    def host_arrays(events: SimEvent):
+        """(array, dtype) of the fields that the library reads, in the order of the C struct."""
+        return [(events.type, np.int32)] + [(a, np.float64) for a in (events.dt, events.rf_amp, events.rf_phase,
+                                                                      events.rf_freq)]
 
     @classmethod
     def from_tensors(cls, type_, dt, amp, phase, freq, adc):
@@ -244,8 +270,8 @@ def simulate_device(pr, params_dev, dev_ev, m0_dev, out_dev, spread=None):
     return keep
 
 
-def _simulate(params: SimParams, events: SimEvent, M_init, mz: int, spread=None,
-              precision=None) -> np.ndarray:
+def _simulate(params: SimParams, events: SimEvent, M_init, mz: int, spread=None, precision=None,
+              device_out: bool = False):
     torch = _lib.torch_cuda()
     nb = n_samples(params)
     nv = nb if nb is not None else 1
@@ -253,21 +279,28 @@ def _simulate(params: SimParams, events: SimEvent, M_init, mz: int, spread=None,
     N = state_size(nc)
     m0 = np.asarray(M_init, np.float64)
     m0 = np.broadcast_to(m0.reshape(-1, N) if m0.ndim > 1 else m0, (nv, N))
-    dev_ev = DeviceEvents(events)
-    pdev = _device(pack_params(params, nv))
-    mdev = _device(m0)
-    shape = (nv, dev_ev.n_offsets) if mz >= 0 else (nv, dev_ev.n_offsets, N)
-    out = torch.empty(shape, dtype=torch.float64, device="cuda")
-    pr = problem(nv, dev_ev.n_offsets, dev_ev.n_events, nc, mz, precision)
-    keep = None
-    sp = None
+    dt = np.asarray(events.dt)
+    if dt.ndim != 2:
+        raise ValueError(f"events must be (n_offsets, n_events), got {dt.shape}")
+    n_off, n_ev = dt.shape
+    host = DeviceEvents.host_arrays(events) + [(pack_params(params, nv), np.float64), (m0, np.float64)]
     if spread is not None:
         u, w, sigma = spread
-        sdev = _device(np.broadcast_to(np.asarray(sigma, np.float64), (nv,)))
-        sp = _lib.spread_struct(u, w, sdev)
-    keep = simulate_device(pr, pdev, dev_ev, mdev, out, sp)
+        host.append((np.broadcast_to(np.asarray(sigma, np.float64), (nv,)), np.float64))
+    held, p = upload(*host)
+    out = torch.empty((nv, n_off) if mz >= 0 else (nv, n_off, N), dtype=torch.float64, device="cuda")
+    pr = problem(nv, n_off, n_ev, nc, mz, precision)
+    sp = None
+    if spread is not None:
+        u, w = (np.ascontiguousarray(x, np.float64) for x in (u, w))
+        dp = _lib.C.POINTER(_lib.C.c_double)
+        sp = _lib.Spread(int(u.size), u.ctypes.data_as(dp), w.ctypes.data_as(dp), p[7])
+    ev = _lib.Events(*p[:5], None)
+    _lib.check(_lib.lib().bmc_simulate(pr, p[5], ev, p[6], sp, out.data_ptr(), _lib.stream_handle()))
+    if device_out:
+        return out
     res = out.cpu().numpy()
-    del keep
+    del held
     return res if nb is not None else res[0]
 
 

@@ -12,7 +12,8 @@
 //
 // exp(X) and H come together from the dual scaling and squaring of X + eps E, E = v lam^T: the Horner
 // recurrence of exp(X / 2^s) with the tangent direction E / 2^s, then s squarings of the pair
-// [T, H] -> [T T, T H + H T] (exp(2Y + 2 eps F) = exp(Y + eps F)^2). A group of lanes takes one chain,
+// [T, H] -> [T T, T H + H T] (exp(2Y + 2 eps F) = exp(Y + eps F)^2), T kept as T - 1 (T - 1 -> (T - 1)^2 + 2 (T - 1): the
+// slow modes' entries keep their digits). A group of lanes takes one chain,
 // lane j < N holding column j of T and of H. T's last row is e_N^T (the augmented row) and is not
 // stored; H's is (E has a last row: v_N lam^T = lam^T). The augmented column of T, phi = T[0:N, N], is
 // kept apart in shared memory, lane i updating row i (phi <- T phi + phi), and the augmented column
@@ -208,7 +209,8 @@ struct Adjoint {
     }
 
     // One squaring of a slot's pair, in place, by the whole warp (N = 16):
-    //   T <- T T,  H[0:N] <- T H[0:N] + H[0:N] T + phi h^T,  h <- h + h T,  phi <- T phi + phi
+    //   T <- T T + 2 T,  H[0:N] <- T H[0:N] + H[0:N] T + 2 H[0:N] + phi h^T,  h <- 2 h + h T,  phi <- T phi + 2 phi
+    // (T is the exponential less 1)
     // (h = H's augmented row). The rank-one term is a fifth k-step whose A column is phi and whose B row is
     // h; lanes 0-15 form h, lanes 16-31 phi. Everything is read before the warp synchronises and writes.
     template <bool kTan>
@@ -231,14 +233,19 @@ struct Adjoint {
         for (int I = 0; I < 2; ++I)
 #pragma unroll
             for (int J = 0; J < 2; ++J) {
-                cT[I][J][0] = 0.0;
-                cT[I][J][1] = 0.0;
+                cT[I][J][0] = 2.0 * T[(8 * J + 2 * t) * LD + 8 * I + g];
+                cT[I][J][1] = 2.0 * T[(8 * J + 2 * t + 1) * LD + 8 * I + g];
 #pragma unroll
                 for (int K = 0; K < 4; ++K) dmma(cT[I][J][0], cT[I][J][1], aT[I][K], bT[K][J]);
             }
         double cH[2][2][2];
         if constexpr (kTan) {
             double aH[2][4], bH[4][2], aP[2], bP[2];
+            // T + 2 as the left operand gives T H + 2 H
+#pragma unroll
+            for (int I = 0; I < 2; ++I)
+#pragma unroll
+                for (int K = 0; K < 4; ++K) aT[I][K] += 8 * I + g == 4 * K + t ? 2.0 : 0.0;
 #pragma unroll
             for (int I = 0; I < 2; ++I) {
 #pragma unroll
@@ -269,13 +276,13 @@ struct Adjoint {
         double vec = 0.0;
         if (lane < N) {
             if constexpr (kTan) {
-                vec = H[lane * LD + N];
+                vec = 2.0 * H[lane * LD + N];
 #pragma unroll
                 for (int l = 0; l < N; ++l) vec = fma(H[l * LD + N], T[lane * LD + l], vec);
             }
         } else {
             const int i = lane - N;
-            vec = ph[i];
+            vec = 2.0 * ph[i];
 #pragma unroll
             for (int l = 0; l < N; ++l) vec = fma(T[l * LD + i], ph[l], vec);
         }
@@ -316,16 +323,18 @@ adjoint_kernel(const ChainArgs a, const int* __restrict__ row_ev, int n_tan, con
     SL* slots = reinterpret_cast<SL*>(smem_raw) + (threadIdx.x >> 5) * G;
     const int lane = threadIdx.x & 31, grp = lane / GS, gl = lane % GS;
 
-    const long long nch = (long long)a.n_vox * a.n_off;
+    if (a.done && *a.left == 0) return;        // the thread kernel has taken every chain
+    const long long nch = a.live ? *a.live : (long long)a.n_vox * a.n_off;
     const long long first = ((long long)blockIdx.x * kAdjWarps + (threadIdx.x >> 5)) * a.cpw;
+    if (first >= nch) return;
     long long ci = first + lane;
     const bool valid = lane < a.cpw && ci < nch;
     if (!valid) ci = first < nch ? first : nch - 1;
     if (a.order) ci = a.order[ci];
     const int v = (int)(ci / a.n_off), o = (int)(ci % a.n_off);
-    const bool act = valid && (a.active == nullptr || a.active[v] != 0);
-    if (__all_sync(kFull, !act)) return;
     const size_t ch = (size_t)v * a.n_off + o;
+    const bool act = valid && (a.active == nullptr || a.active[v] != 0) && !(a.done && a.done[ch]);
+    if (__all_sync(kFull, !act)) return;
     const EvRec<double> rec = reinterpret_cast<const EvRec<double>*>(a.ev)[(size_t)row_ev[o] * a.n_off + o];
     unsigned wk1 = 0, wk2 = 0;
 
@@ -430,7 +439,7 @@ adjoint_kernel(const ChainArgs a, const int* __restrict__ row_ev, int n_tan, con
                         cdN = ik * dot;
                     }
 #pragma unroll
-                    for (int q = 0; q < N; ++q) C0::at(cv, q).v = (q == gl ? 1.0 : 0.0) + ik * C0::at(yv, q).v;
+                    for (int q = 0; q < N; ++q) C0::at(cv, q).v = (q == gl && k > 1 ? 1.0 : 0.0) + ik * C0::at(yv, q).v;
                 }
             }
             // the augmented column: [phi; 1] <- e_N + X [phi; 1] / k
@@ -448,7 +457,7 @@ adjoint_kernel(const ChainArgs a, const int* __restrict__ row_ev, int n_tan, con
                 for (int q = 0; q < N; ++q) sl->phi[0][q] = C0::at(ph, q).v;
             }
             __syncwarp();
-            // s squarings: [T, H] <- [T T, T H + H T], phi <- T phi + phi
+            // s squarings
             if constexpr (AdjGroup<NC>::kMma) {
                 if (work) {
 #pragma unroll
@@ -489,11 +498,11 @@ adjoint_kernel(const ChainArgs a, const int* __restrict__ row_ev, int n_tan, con
                     if (sq) {
                         const double* ph = sl->phi[q & 1];
                         S nv, nd;
-                        double ndN = cdN, pj = ph[gl];
+                        double ndN = 2.0 * cdN, pj = 2.0 * ph[gl];
 #pragma unroll
                         for (int i = 0; i < N; ++i) {
-                            C0::at(nv, i).v = 0.0;
-                            if constexpr (kTan) C0::at(nd, i).v = ph[i] * cdN;
+                            C0::at(nv, i).v = 2.0 * C0::at(cv, i).v;
+                            if constexpr (kTan) C0::at(nd, i).v = fma(ph[i], cdN, 2.0 * C0::at(cd, i).v);
                         }
 #pragma unroll
                         for (int l = 0; l < N; ++l) {
@@ -520,7 +529,7 @@ adjoint_kernel(const ChainArgs a, const int* __restrict__ row_ev, int n_tan, con
             }
             // z = sum_j (exp(X)^T lam)_j v_j (phi[mz] for j = N), and per tangent
             // tr(dX_p H) + (exp(X)^T lam) . dv_p
-            const double u = work ? A::get(cv, a.mz) : 0.0;
+            const double u = work ? A::get(cv, a.mz) + (gl == a.mz ? 1.0 : 0.0) : 0.0;
             const double zsum = group_sum<GS>(work ? u * sl->v[gl] : 0.0);
             for (int p = 0; p < (kTan ? n_tan : 0); ++p) {
                 double gp = 0.0;

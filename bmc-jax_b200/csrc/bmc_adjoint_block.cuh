@@ -216,7 +216,8 @@ struct AdjBlk {
         }
     }
 
-    // column gl of exp(X_i) into E[i] (T kept in the slot's P during the squarings)
+    // column gl of exp(X_i) into E[i] (T = exp - 1 kept in the slot's P during the squarings T <- T T + 2 T: the slow modes'
+    // entries keep their digits)
     static __device__ void exp_event(SL* sl, int i, int gl, bool work, int s_g, int smax, const TaylorTable& tt) {
         const double caug = gl == N ? 1.0 : 0.0;
         S cv;
@@ -227,7 +228,7 @@ struct AdjBlk {
                 op(sl, i, cv, caug, y);
                 const double ik = tt.inv_k[k];
 #pragma unroll
-                for (int q = 0; q < N; ++q) C0::at(cv, q).v = (q == gl ? 1.0 : 0.0) + ik * C0::at(y, q).v;
+                for (int q = 0; q < N; ++q) C0::at(cv, q).v = (q == gl && k > 1 ? 1.0 : 0.0) + ik * C0::at(y, q).v;
             }
         }
         double* T = sl->P;
@@ -243,7 +244,7 @@ struct AdjBlk {
                 // registers and can stay partly rolled
                 S nv;
 #pragma unroll
-                for (int r = 0; r < N; ++r) C0::at(nv, r).v = caug * T[N * LD + r];
+                for (int r = 0; r < N; ++r) C0::at(nv, r).v = 2.0 * T[gl * LD + r];
 #pragma unroll 4
                 for (int l = 0; l < N; ++l) {
                     const double w = T[gl * LD + l];
@@ -257,12 +258,12 @@ struct AdjBlk {
         if (work) {
             double* Ei = sl->E[i];
 #pragma unroll
-            for (int r = 0; r < N; ++r) Ei[gl * LD + r] = C0::at(cv, r).v;
+            for (int r = 0; r < N; ++r) Ei[gl * LD + r] = C0::at(cv, r).v + (r == gl ? 1.0 : 0.0);
             Ei[gl * LD + N] = caug;
         }
     }
 
-    // G_i = L(X_i, W_i) (W_i in the slot's B): column gl into (cd, cdN); T and H in P and B
+    // G_i = L(X_i, W_i) (W_i in the slot's B): column gl into (cd, cdN); T (less 1) and H in P and B
     static __device__ void frechet_event(SL* sl, int i, int gl, bool work, int s_g, int smax, const TaylorTable& tt,
                                          S& cd, double& cdN) {
         const double caug = gl == N ? 1.0 : 0.0;
@@ -303,7 +304,7 @@ struct AdjBlk {
                 S yv;
                 op(sl, i, cv, caug, yv);
 #pragma unroll
-                for (int q = 0; q < N; ++q) C0::at(cv, q).v = (q == gl ? 1.0 : 0.0) + ik * C0::at(yv, q).v;
+                for (int q = 0; q < N; ++q) C0::at(cv, q).v = (q == gl && k > 1 ? 1.0 : 0.0) + ik * C0::at(yv, q).v;
             }
         }
         __syncwarp();   // W_i is read by every lane before the squarings overwrite B
@@ -322,14 +323,12 @@ struct AdjBlk {
             __syncwarp();
             if (sq) {
                 S nv, nd;
-                double ndN = cdN;
+                double ndN = 2.0 * cdN;
 #pragma unroll
                 for (int r = 0; r < N; ++r) {
-                    const double t_aug = T[N * LD + r], h_aug = H[N * LD + r];
-                    C0::at(nv, r).v = caug * t_aug;
-                    C0::at(nd, r).v = fma(t_aug, cdN, caug * h_aug);
+                    C0::at(nv, r).v = 2.0 * T[gl * LD + r];
+                    C0::at(nd, r).v = fma(T[N * LD + r], cdN, 2.0 * H[gl * LD + r]);
                 }
-                ndN = fma(caug, H[N * LD + N], ndN);
 #pragma unroll 2
                 for (int l = 0; l < N; ++l) {
                     const double wv = T[gl * LD + l], wd = H[gl * LD + l];   // this lane's column, as stored

@@ -41,6 +41,7 @@ struct TaylorTable {
 struct TrainRow {
     int first, n, gap, run;
     int span, uses;
+    int mirrored;              // the pulse's shape is its own mirror image
     double w_max;
 };
 constexpr int kTrainMark = 8;  // added to the type of a record where a unit begins
@@ -96,6 +97,10 @@ struct ChainArgs {
     const TrainRow* train;     // [n_off]
     const double* prop;
     const int* prop_ok;
+    // adjoint passes: the chains that the thread kernel (bmc_sym.cuh) has taken, and whether it left any
+    unsigned char* done;       // [n_vox * n_off] or null
+    int* left;
+    const int* live;           // null, or how many entries of `order` the pass takes (the active voxels' chains)
 };
 
 // Chains per warp of a launch: 32, or as many fewer as still leave the launch's warps resident at once. A launch
@@ -447,7 +452,8 @@ struct Chain {
     // exp(X) [M; 1] of a free event (no RF) whose transverse entries are all zero: they stay zero, and the z entries
     // (water, CEST pools, MT) evolve by their own (NC + 2) x (NC + 2) block, which one thread exponentiates for its
     // chain: the degree-m Horner recurrence of the block and of its constant column, then s squarings, the norm
-    // without any precession in it.
+    // without any precession in it. What is squared is F = exp - 1 (F <- F F + 2 F): the slow modes' entries keep
+    // their digits, where squaring 1 + F doubles their error each time.
     // Recoveries and the delays behind a spoiler are such events. The dense path gives each of them a warp for ~11
     // Horner steps and ~13 squarings of the whole (N + 1) x (N + 1) matrix: 206,848 chains of four pools with one
     // 3 s recovery (and one propagator to apply) took 4.89 ms in the chain kernel so, 0.31 ms this way.
@@ -467,8 +473,8 @@ struct Chain {
         nu = nu * dt;
         const int s = nu > R(tt.dense_theta) ? (int)ceil(log2(double(nu) / tt.dense_theta)) : 0;
         const R h = R(ldexp(double(dt), -s));
-        D T[Z][Z], phi[Z];                    // T[column][row]
-        // Horner, column by column: v <- e + X v / k (the constant column: phi <- X [phi; 1] / k)
+        D T[Z][Z], phi[Z];                    // F: T[column][row]
+        // Horner, column by column: v <- e + X v / k, without e at the end (the constant column: phi <- X [phi; 1] / k)
 #pragma unroll
         for (int j = 0; j <= Z; ++j) {
             D v[Z];
@@ -492,7 +498,7 @@ struct Chain {
                 }
                 v[0] = ik * w;
                 v[Z - 1] = ik * m;
-                if (j < Z) v[j] = v[j] + R(1);
+                if (j < Z && k > 1) v[j] = v[j] + R(1);
             }
 #pragma unroll
             for (int i = 0; i < Z; ++i) (j < Z ? T[j < Z ? j : 0][i] : phi[i]) = v[i];
@@ -502,7 +508,7 @@ struct Chain {
             D n[Z][Z];
 #pragma unroll
             for (int i = 0; i < Z; ++i) {
-                D p = phi[i];
+                D p = phi[i] + phi[i];
 #pragma unroll
                 for (int l = 0; l < Z; ++l) p = dfma(T[l][i], phi[l], p);
                 n[0][i] = p;                  // parked: phi is read by every row
@@ -513,9 +519,9 @@ struct Chain {
             for (int j = 0; j < Z; ++j)
 #pragma unroll
                 for (int i = 0; i < Z; ++i) {
-                    D x = T[0][i] * T[j][0];
+                    D x = T[j][i] + T[j][i];
 #pragma unroll
-                    for (int l = 1; l < Z; ++l) x = dfma(T[l][i], T[j][l], x);
+                    for (int l = 0; l < Z; ++l) x = dfma(T[l][i], T[j][l], x);
                     n[j][i] = x;
                 }
 #pragma unroll
@@ -531,10 +537,10 @@ struct Chain {
             for (int l = 0; l < NC; ++l) x = dfma(T[1 + l][i], M.zc[l], x);
             z[i] = dfma(T[Z - 1][i], M.zm, x);
         }
-        M.zw = z[0];
+        M.zw = M.zw + z[0];
 #pragma unroll
-        for (int i = 0; i < NC; ++i) M.zc[i] = z[1 + i];
-        M.zm = z[Z - 1];
+        for (int i = 0; i < NC; ++i) M.zc[i] = M.zc[i] + z[1 + i];
+        M.zm = M.zm + z[Z - 1];
     }
 
     static __device__ __forceinline__ void spoil(State<NC, D>& M) {

@@ -3,6 +3,7 @@
 #include <type_traits>
 
 #include "bmc_chain.cuh"
+#include "bmc_sym.cuh"
 
 namespace bmc {
 
@@ -30,6 +31,10 @@ constexpr double kBlockDenseNorm = 4.0;
 // the norm above which a free event without transverse magnetisation takes its z block alone (Chain::z_event): its
 // ~11 Horner steps of NC + 3 columns and ~10 squarings cost what the Taylor action costs at a norm of about 8
 constexpr double kZFreeNorm = 8.0;
+
+// the norm above which an event of a small generator goes to sym_event: its ~4,500 multiply-adds against 175 per unit
+// of the norm for the Taylor action (one pool)
+constexpr double kSymNorm = 30.0;
 
 // lanes per chain in the dense path: one column per lane, so a warp works on 32 / GS chains at once
 template <int NC>
@@ -133,10 +138,12 @@ struct Dense {
             if (q == j) C::at(col, q) = dconst<R, NT>(R(1));
     }
 
-    // Column gl of exp(X) into `col`, X the slot's coefficients and constant column (already scaled by
-    // dt / 2^s): the degree-m Horner recurrence T = I + X T / k, k = m .. 1, then s squarings through the
-    // slot's matrix (column j of T T is sum_l T[:, l] T[l][j]). Every lane of the warp calls it (the
-    // squarings synchronise the warp, up to the warp's largest count smax); lanes with `work` compute.
+    // Column gl of F = exp(X) - 1 into `col`, X the slot's coefficients and constant column (already scaled by
+    // dt / 2^s): the degree-m Horner recurrence T = I + X T / k, k = m .. 1, without the last I, then s squarings F <-
+    // F F + 2 F through the slot's matrix (column j of F F is sum_l F[:, l] F[l][j]). Squaring 1 + F instead doubles the
+    // error of the slow modes' entries each time: 7e-11 in Z after a 2 s block of one pool, against 1e-14. Every lane of
+    // the warp calls it (the squarings synchronise the warp, up to the warp's largest count smax); lanes with `work`
+    // compute.
     static __device__ __forceinline__ void exp_column(SL* sl, int gl, bool work, int s, int smax, State<NC, D>& col,
                                                       const TaylorTable& tt) {
         const R caug = (gl == N) ? R(1) : R(0);
@@ -147,7 +154,7 @@ struct Dense {
                 matvec_aug(sl, col, caug, y);
                 C::scal_state(y, R(tt.inv_k[k]));
                 State<NC, D> e;
-                unit(e, gl);
+                unit(e, k > 1 ? gl : -1);
                 C::axpy_state(e, y);
                 col = e;
             }
@@ -157,21 +164,16 @@ struct Dense {
             if (sq) {
 #pragma unroll
                 for (int i = 0; i < N; ++i) sl->mat[gl * LD + i] = C::at(col, i);
-                sl->mat[gl * LD + N] = dconst<R, NT>(caug);
             }
             __syncwarp();
             if (sq) {
-                State<NC, D> nc;
-                unit(nc, -1);
+                State<NC, D> nc = col;
+                C::axpy_state(nc, col);
 #pragma unroll
                 for (int l = 0; l < N; ++l) {
                     const D w = C::at(col, l);
 #pragma unroll
                     for (int i = 0; i < N; ++i) C::at(nc, i) = dfma(sl->mat[l * LD + i], w, C::at(nc, i));
-                }
-                if (caug != R(0)) {           // the augmented column also picks up T[:, aug]
-#pragma unroll
-                    for (int i = 0; i < N; ++i) C::at(nc, i) = C::at(nc, i) + sl->mat[N * LD + i];
                 }
                 col = nc;
             }
@@ -231,7 +233,7 @@ struct Dense {
             const int smax = (int)__reduce_max_sync(kFull, (unsigned)s);
             State<NC, D> col;
             exp_column(sl, gl, work, s, smax, col, tt);
-            // M <- T [M; 1]
+            // M <- M + F [M; 1]
             if (work) {
 #pragma unroll
                 for (int i = 0; i < N; ++i) sl->mat[gl * LD + i] = C::at(col, i);
@@ -240,7 +242,7 @@ struct Dense {
             if (grp_owner >= 0 && gl < N) {
                 D acc = dconst<R, NT>(R(0));
                 for (int j = 0; j < NA; ++j) acc = dfma(sl->mat[j * LD + gl], sl->vec[j], acc);
-                sl->out[gl] = acc;
+                sl->out[gl] = sl->vec[gl] + acc;
             }
             __syncwarp();
             if (my_slot >= 0) {
@@ -358,9 +360,8 @@ struct Dense {
                         for (int i = 0; i < N; ++i) sl->mat[gl * LD + i] = C::at(T, i);
                     }
                     __syncwarp();
-                    if (dense) {                             // column gl of T [P; pa]
-                        State<NC, D> np;
-                        unit(np, -1);
+                    if (dense) {                             // column gl of (1 + F) [P; pa]
+                        State<NC, D> np = P;
 #pragma unroll
                         for (int l = 0; l < N; ++l) {
                             const D w = C::at(P, l);
@@ -463,7 +464,7 @@ struct TrainShape {
     static constexpr int NS = (N + 2) & ~1;                  // row of the stored propagator: N entries, phi, padding
     // warps per block: the shared memory of a warp (19 KB with four pools) sets the resident warps, so small blocks
     static constexpr int kWarps = NT == 1 ? 4 : 1;
-    static constexpr int kBlocks = NT == 1 ? 4 : (NT == 2 ? 11 : 7);   // resident blocks the registers are kept for
+    static constexpr int kBlocks = NT == 1 ? 4 : (NT == 2 ? 8 : 4);   // resident blocks the registers are kept for
 };
 
 // M <- R(phase) [P R(-phase) M + phi], P from the propagator `p` (the turned frame's x is along the RF); with tangents
@@ -694,7 +695,19 @@ chain_kernel(const ChainArgs a, const __grid_constant__ TaylorTable tt) {
                         M = Mt;
                     }
                 }
-                const bool dense_own = evolve && !zfree && nu > dswitch;
+                bool dense_own = evolve && !zfree && nu > dswitch;
+                // small generators: the chain's own thread, where the chain can take that form
+                bool sym = false;
+                if constexpr (NT == 0 && std::is_same<R, RD>::value && !COUNT && Sym<NC>::kFits) {
+                    if (dense_own || (!UNEVEN && evolve && !zfree && nu > R(kSymNorm))) {
+                        StepCoef<NC, D> sc;
+                        C::event_coef(cc, rec, g, sc);
+                        State<NC, D> Mt = M;
+                        sym = sym_event<NC>(a.params, a.n_vox, v, cc, sc, rec, nu, tt, Mt);
+                        if (sym) M = Mt;
+                        dense_own = dense_own && !sym;
+                    }
+                }
                 if (__any_sync(kFull, dense_own)) {
                     StepCoef<NC, D> sc;                            // unscaled: the dense path scales by dt / 2^s
                     C::event_coef(cc, rec, g, sc);
@@ -710,7 +723,7 @@ chain_kernel(const ChainArgs a, const __grid_constant__ TaylorTable tt) {
                         convert_flat<RD, R, NT>(Md, M);
                     }
                 }
-                const bool tay = evolve && !dense_own && !zfree;
+                const bool tay = evolve && !dense_own && !zfree && !sym;
                 int m_own = 0, ns_own = 0;
                 if (tay) {
                     ns_own = nu > thm ? (int)ceil(nu / thm) : 1;

@@ -20,6 +20,10 @@
 //   straight into the B layout from the E_q in shared memory.
 // * The constant column: phi <- phi + P e_k before each product, every lane summing its own columns; the lanes' parts
 //   are added once at the end.
+// * A shape that is its own mirror image costs half: E_1 ... E_m (the second half) is the first half's product with its
+//   order reversed, and every E_k is its own transpose up to signs and the pools' fractions (G E^T G^-1 = E, G = diag(+-f),
+//   detailed balance; bmc_sym.cuh), so Phi_2 = G Phi_1^T G^-1. Only the second half's constant column needs its own
+//   recurrence, a matrix-vector product per sample.
 // * Equal events between the repeats (gaps, spoilers) belong to the unit too; units that follow one another with the
 //   same phase are one propagator P^repeats.
 #pragma once
@@ -32,6 +36,7 @@ constexpr int kTrainMaxSamples = 1024;   // ... and at most this many (its weigh
 constexpr int kTrainMaxPulses = 1024;    // pulses of a row that are looked at
 constexpr int kTrainMaxGap = 4;          // events between two pulses that a unit takes in
 constexpr double kTrainTol = 2e-15;      // interpolation error per event
+constexpr double kTrainMirror = 9e-16;   // 8 x 2^-53: two samples this close (over the largest) mirror each other
 
 // the table's side of a propagator launch; the chains' side (ChainArgs: train, prop, prop_ok, first_chain,
 // chain_count) is the chain kernel's too
@@ -74,11 +79,11 @@ train_scan_kernel(EvRec<double>* __restrict__ ev, int n_ev, int stride, int min_
                   TrainRow* __restrict__ rows, double* __restrict__ rho, int max_samples) {
     __shared__ int starts[kTrainMaxPulses], ends[kTrainMaxPulses];
     __shared__ unsigned char match[kTrainMaxPulses];
-    __shared__ int n_start, n_end, warp_n[kTrainScanThreads / 32][2], flags[2];
+    __shared__ int n_start, n_end, warp_n[kTrainScanThreads / 32][2], flags[3];
     __shared__ double wmax_s;
     EvRec<double>* row = ev + blockIdx.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    TrainRow out{0, 0, 0, 0, 0, 0, 0.0};
+    TrainRow out{0, 0, 0, 0, 0, 0, 0, 0.0};
     if (tid == 0) n_start = n_end = 0;
     __syncthreads();
     auto is_rf = [&](const EvRec<double>& r) { return (int)r.type == EV_RF && r.dt > 1e-9; };
@@ -127,7 +132,7 @@ train_scan_kernel(EvRec<double>* __restrict__ ev, int n_ev, int stride, int min_
         const int ref = (np - 1) / 2, r0 = starts[ref], n = ends[ref] - r0 + 1;
         if (n >= kTrainMinSamples && n <= max_samples) {
             for (int p = tid; p < np; p += kTrainScanThreads) match[p] = ends[p] - starts[p] + 1 == n;
-            if (tid < 2) flags[tid] = 1;
+            if (tid < 3) flags[tid] = 1;
             __syncthreads();
             for (long long i = tid; i < (long long)np * n; i += kTrainScanThreads) {
                 const int p = (int)(i / n), k = (int)(i % n);
@@ -170,6 +175,12 @@ train_scan_kernel(EvRec<double>* __restrict__ ev, int n_ev, int stride, int min_
                 if (lane == 0) wmax_s = m;
             }
             __syncthreads();
+            // mirrored within the rounding of a shape that was computed sample by sample
+            for (int k = tid; k < n / 2; k += kTrainScanThreads)
+                if (!(fabs(row[(size_t)(r0 + k) * stride].w1 - row[(size_t)(r0 + n - 1 - k) * stride].w1) <=
+                      kTrainMirror * wmax_s))
+                    atomicAnd(&flags[2], 0);
+            __syncthreads();
             int uses = 0, first_match = -1;
             for (int p = 0; p < np; ++p)
                 if (match[p]) {
@@ -181,7 +192,7 @@ train_scan_kernel(EvRec<double>* __restrict__ ev, int n_ev, int stride, int min_
             const long long block_saves = blk.z >= 2 ? (long long)(blk.z - 1) * blk.y : 0;
             const double wm = wmax_s;
             if (uses >= min_uses && wm > 0.0 && wm < INFINITY && (long long)(uses - 1) * n > block_saves) {
-                out = TrainRow{r0, n, gap, run, run * unit, uses, wm};
+                out = TrainRow{r0, n, gap, run, run * unit, uses, flags[2], wm};
                 __syncthreads();
                 if (tid == 0) seg[blockIdx.x] = make_int4(0, 0, 0, 0);
                 for (int p = tid; p < np; p += kTrainScanThreads)
@@ -214,6 +225,7 @@ struct alignas(16) TrainSmem {
     using S = TrainShape<NC>;
     double T[1 + NT][S::kSlots][S::TS];          // column-major, padded with zeros
     double phi[1 + NT][S::kSlots][8 * S::NT];
+    double gv[8 * S::NT];                        // G by state entry, signed (1 in the padding)
     TrainCoef<NC, NT> coef;
 };
 
@@ -333,7 +345,7 @@ struct Train {
                 op(sm->coef, q, v, caug, y);
                 const double ik = tt.inv_k[k];
 #pragma unroll
-                for (int i = 0; i < N; ++i) C::at(v, i) = ik * C::at(y, i) + (i == col ? 1.0 : 0.0);
+                for (int i = 0; i < N; ++i) C::at(v, i) = ik * C::at(y, i) + (i == col && k > 1 ? 1.0 : 0.0);
             }
 #pragma unroll
             for (int d = 0; d < ND; ++d) {
@@ -343,11 +355,15 @@ struct Train {
             }
         }
         __syncwarp();
-        for (int q = 0; q < n; ++q)
+        for (int q = 0; q < n; ++q) {
             for (int j = 0; j < s; ++j) square(sm, q, lane);
+            if (lane < N) sm->T[0][q][lane * LD + lane] += 1.0;
+        }
+        __syncwarp();
     }
 
-    // T <- T T, phi <- T phi + phi of slot q (and their derivatives)
+    // F <- F F + 2 F, phi <- F phi + 2 phi of slot q (and their derivatives), F = exp - 1: the slow modes' entries keep
+    // their digits, where squaring 1 + F doubles their error each time
     static __device__ __forceinline__ void square(SM* sm, int q, int lane) {
         const int g = lane >> 2, t = lane & 3;
         double c[ND][NT][NT][2];
@@ -364,7 +380,8 @@ struct Train {
             for (int d = 0; d < ND; ++d)
 #pragma unroll
                 for (int I = 0; I < NT; ++I) {
-                    a[d][I] = sm->T[d][q][(4 * K + t) * LD + 8 * I + g];
+                    // F + 2 as the left operand gives F F + 2 F (and F dF + 2 dF)
+                    a[d][I] = sm->T[d][q][(4 * K + t) * LD + 8 * I + g] + (d == 0 && 8 * I + g == 4 * K + t ? 2.0 : 0.0);
                     b[d][I] = sm->T[d][q][(8 * I + g) * LD + 4 * K + t];
                 }
 #pragma unroll
@@ -381,7 +398,7 @@ struct Train {
         double p[ND];
         if (lane < N) {
 #pragma unroll
-            for (int d = 0; d < ND; ++d) p[d] = sm->phi[d][q][lane];
+            for (int d = 0; d < ND; ++d) p[d] = 2.0 * sm->phi[d][q][lane];
 #pragma unroll
             for (int l = 0; l < N; ++l) {
                 const double x = sm->T[0][q][l * LD + lane], y = sm->phi[0][q][l];
@@ -581,6 +598,103 @@ struct Train {
         __syncwarp();
     }
 
+    // The pools' G = diag(+-f) by state entry: its magnitude (1 for water, and for a pool without exchange)
+    static __device__ __forceinline__ double balance(const double* params, int n_vox, int v, int i, bool& ok) {
+        using L = Layout<NC>;
+        double f = 1.0, k = 0.0;
+        if (i == N - 1) {
+            f = params[(size_t)L::MF * n_vox + v];
+            k = params[(size_t)L::MK * n_vox + v];
+        } else if (i < N - 1 && i % (NC + 1) != 0) {
+            const int p = i % (NC + 1) - 1;
+            f = params[(size_t)(L::CF + p) * n_vox + v];
+            k = params[(size_t)(L::CK + p) * n_vox + v];
+        }
+        if (f > 1e-20) return f;
+        ok = ok && k == 0.0;
+        return 1.0;
+    }
+
+    // A mirrored pulse from its first half: r <- Phi_2 (E_c) Phi_1 with its constant column. `gv` holds G by state entry
+    // in shared memory (signed; slot 1 is free until the end of the sweep only for its own product).
+    template <int NQ>
+    static __device__ __forceinline__ void mirrored(SM* sm, Run& r, const double* __restrict__ rho, int n,
+                                                    const double* gv, int lane) {
+        static_assert(DT == 0, "the propagators' derivatives take the whole pulse");
+        constexpr int kHeld = NT == 1 ? NQ : (NT == 2 && NQ == 4 ? 4 : 0);
+        const int g = lane >> 2, t = lane & 3, m = n / 2;
+        double2 H[kHeld > 0 ? kHeld : 1][NT][NT];
+#pragma unroll
+        for (int q = 0; q < kHeld; ++q)
+#pragma unroll
+            for (int K = 0; K < NT; ++K)
+#pragma unroll
+                for (int J = 0; J < NT; ++J) H[q][K][J] = lds2(sm->T[0][q] + (8 * J + g) * LD + 8 * K + 2 * t);
+        // psi = G^-1 phi_2: psi <- G^-1 v + E^T psi, from the middle out (rows 8 K + 2 t + (x, y) in this lane)
+        double2 ig[NT], psi[NT];
+#pragma unroll
+        for (int K = 0; K < NT; ++K) {
+            ig[K] = make_double2(1.0 / gv[8 * K + 2 * t], 1.0 / gv[8 * K + 2 * t + 1]);
+            psi[K] = make_double2(0.0, 0.0);
+        }
+        Op cur;
+        eval<NQ, kHeld>(sm, H, rho[m - 1], cur, lane);
+        double next = rho[m > 1 ? m - 2 : 0];
+#pragma unroll 1
+        for (int k = m - 1; k >= 0; --k) {
+            const double after = rho[k > 2 ? k - 2 : 0];
+            Op nx;
+            eval<NQ, kHeld>(sm, H, next, nx, lane);
+            apply(r, cur);
+            double x[NT];
+#pragma unroll
+            for (int J = 0; J < NT; ++J) {
+                x[J] = 0.0;
+#pragma unroll
+                for (int K = 0; K < NT; ++K)
+                    x[J] = fma(cur.E[0][K][J].x, psi[K].x, fma(cur.E[0][K][J].y, psi[K].y, x[J]));
+                x[J] += __shfl_xor_sync(kFull, x[J], 1);
+                x[J] += __shfl_xor_sync(kFull, x[J], 2);      // entry 8 J + g
+            }
+#pragma unroll
+            for (int K = 0; K < NT; ++K) {
+                psi[K].x = fma(cur.v[0][K].x, ig[K].x, __shfl_sync(kFull, x[K], 8 * t));
+                psi[K].y = fma(cur.v[0][K].y, ig[K].y, __shfl_sync(kFull, x[K], 8 * t + 4));
+            }
+            cur = nx;
+            next = after;
+        }
+        Op mid;
+        if (n & 1) eval<NQ, kHeld>(sm, H, rho[m], mid, lane);
+        // Phi_1 and phi_1 into slot 1 (the differences are no longer needed), Phi_2 and phi_2 into the registers
+        __syncwarp();
+        put(sm, 1, r, lane);
+        if (g == 0) {
+#pragma unroll
+            for (int K = 0; K < NT; ++K) {
+                sm->phi[0][0][8 * K + 2 * t] = psi[K].x * gv[8 * K + 2 * t];
+                sm->phi[0][0][8 * K + 2 * t + 1] = psi[K].y * gv[8 * K + 2 * t + 1];
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int I = 0; I < NT; ++I) {
+            const int row = 8 * I + g;
+            r.f[0][I] = t == 0 ? sm->phi[0][0][row] : 0.0;
+#pragma unroll
+            for (int J = 0; J < NT; ++J)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int col = 8 * J + 2 * t + e;
+                    r.P[0][I][J][e] = sm->T[0][1][row * LD + col] * (gv[row] / gv[col]);
+                }
+        }
+        if (n & 1) apply(r, mid);
+        Op first;
+        load(sm, 1, first, lane);
+        apply(r, first);
+    }
+
     // The samples of the pulse, from the last to the first; the next sample's matrix is evaluated beside the products
     // with this one's, so that the vector and the tensor FP64 pipes work together.
     template <int NQ>
@@ -679,6 +793,70 @@ train_kernel(const ChainArgs a, const TrainArgs tr, const __grid_constant__ Tayl
     TR::identity(r, lane);
     bool ok = true;
 
+    if (ok) {
+        // the pulse's matrix function at its nodes
+        EvRec<double> rec = ev[(size_t)row.first * a.n_off];
+        rec.w1 = row.w_max;
+        rec.c = 1.0;
+        rec.s = 0.0;
+        D g = dconst<double, DT>(0.0);
+        if (mt) {
+            const D offmt = (rec.wf - cc.dw0) - cc.dwmt;
+            g = cc.ls == 1 ? lorentzian<double, DT>(offmt, cc.t2mt)
+                           : warp_super_lorentzian<DT>(offmt, cc.t2mt, cc.w0sl, lane);
+        }
+        StepCoef<NC, D> sc;
+        C::event_coef(cc, rec, g, sc);
+        const D w1 = sc.w1x;
+        const int s = TR::squarings(rec.dt * C::coef_norm(sc, cc), tt);
+        const int nq = s < 0 ? 0 : TR::interp_nodes(fabs(w1.v) * rec.dt, fabs(w1.v * w1.v * g.v) * rec.dt);
+        ok = nq > 0;
+        if (ok) {
+            const double h = ldexp(rec.dt, -s);
+            __syncwarp();
+            if (lane == 0) TR::put_coef(sm->coef, sc, cc, h);
+            if (lane < nq) {
+                double u = 0.0;
+#pragma unroll
+                for (int q = 0; q < 6; ++q)
+                    if (q == lane) u = nq == 4 ? train_node<4>(q < 4 ? q : 0) : train_node<6>(q);
+                sm->coef.w1[lane] = (h * sqrt(u)) * w1;
+                sm->coef.Rm[lane] = h * dfma(u * (w1 * w1), g, cc.Rm1);
+            }
+            __syncwarp();
+            TR::exponentials(sm, lane, nq, s, tt);
+            const double* rho = tr.rho + (size_t)o * tr.max_samples;
+            bool half = false;
+            if constexpr (DT == 0) {
+                if (row.mirrored) {
+                    half = true;
+                    if (lane < 8 * NT) {
+                        const double f = lane < N ? TR::balance(a.params, a.n_vox, v, lane, half) : 1.0;
+                        sm->gv[lane] = lane >= NC + 1 && lane < 2 * (NC + 1) ? -f : f;
+                    }
+                    half = __all_sync(kFull, half);
+                }
+            }
+            if (nq == 4) TR::template differences<4>(sm, lane);
+            else TR::template differences<6>(sm, lane);
+            if constexpr (DT == 0) {
+                if (half) {
+                    if (nq == 4) TR::template mirrored<4>(sm, r, rho, row.n, sm->gv, lane);
+                    else TR::template mirrored<6>(sm, r, rho, row.n, sm->gv, lane);
+                }
+            }
+            if (!half) {
+                if (nq == 4) TR::template samples<4>(sm, r, rho, row.n, lane);
+                else TR::template samples<6>(sm, r, rho, row.n, lane);
+            }
+        }
+    }
+    if (ok && row.gap > 0) {
+        // the pulse waits in slot 1 for the events behind it
+        __syncwarp();
+        TR::put(sm, 1, r, lane);
+        TR::identity(r, lane);
+    }
     // the events after the pulse, from the last on: P <- P S E (S: a spoiler zeroes the transverse entries)
     for (int j = row.gap - 1; j >= 0 && ok; --j) {
         const EvRec<double> rec = ev[(size_t)(row.first + row.n + j) * a.n_off];
@@ -714,83 +892,48 @@ train_kernel(const ChainArgs a, const TrainArgs tr, const __grid_constant__ Tayl
         TR::step(sm, r, lane);
     }
     if (ok) {
-        // the pulse's matrix function at its nodes
-        EvRec<double> rec = ev[(size_t)row.first * a.n_off];
-        rec.w1 = row.w_max;
-        rec.c = 1.0;
-        rec.s = 0.0;
-        D g = dconst<double, DT>(0.0);
-        if (mt) {
-            const D offmt = (rec.wf - cc.dw0) - cc.dwmt;
-            g = cc.ls == 1 ? lorentzian<double, DT>(offmt, cc.t2mt)
-                           : warp_super_lorentzian<DT>(offmt, cc.t2mt, cc.w0sl, lane);
+        if (row.gap > 0) {
+            typename TR::Op pulse;
+            TR::load(sm, 1, pulse, lane);
+            TR::apply(r, pulse);
         }
-        StepCoef<NC, D> sc;
-        C::event_coef(cc, rec, g, sc);
-        const D w1 = sc.w1x;
-        const int s = TR::squarings(rec.dt * C::coef_norm(sc, cc), tt);
-        const int nq = s < 0 ? 0 : TR::interp_nodes(fabs(w1.v) * rec.dt, fabs(w1.v * w1.v * g.v) * rec.dt);
-        ok = nq > 0;
-        if (ok) {
-            const double h = ldexp(rec.dt, -s);
+        // equal units in a row: P^run, by squaring and multiplying from the leading bit on
+        if (row.run > 1) {
             __syncwarp();
-            if (lane == 0) TR::put_coef(sm->coef, sc, cc, h);
-            if (lane < nq) {
-                double u = 0.0;
+            TR::put(sm, 1, r, lane);
+            const int top = 31 - __clz(row.run);
+            for (int b = top - 1; b >= 0; --b) {
+                TR::put(sm, 0, r, lane);
+                TR::step(sm, r, lane);
+                if ((row.run >> b) & 1) {
+                    // P^(2k + 1) = P^2k P: the multiplicand is in slot 1
+                    __syncwarp();
 #pragma unroll
-                for (int q = 0; q < 6; ++q)
-                    if (q == lane) u = nq == 4 ? train_node<4>(q < 4 ? q : 0) : train_node<6>(q);
-                sm->coef.w1[lane] = (h * sqrt(u)) * w1;
-                sm->coef.Rm[lane] = h * dfma(u * (w1 * w1), g, cc.Rm1);
-            }
-            __syncwarp();
-            TR::exponentials(sm, lane, nq, s, tt);
-            const double* rho = tr.rho + (size_t)o * tr.max_samples;
-            if (nq == 4) {
-                TR::template differences<4>(sm, lane);
-                TR::template samples<4>(sm, r, rho, row.n, lane);
-            } else {
-                TR::template differences<6>(sm, lane);
-                TR::template samples<6>(sm, r, rho, row.n, lane);
-            }
-            // equal units in a row: P^run, by squaring and multiplying from the leading bit on
-            if (row.run > 1) {
-                __syncwarp();
-                TR::put(sm, 1, r, lane);
-                const int top = 31 - __clz(row.run);
-                for (int b = top - 1; b >= 0; --b) {
-                    TR::put(sm, 0, r, lane);
-                    TR::step(sm, r, lane);
-                    if ((row.run >> b) & 1) {
-                        // P^(2k + 1) = P^2k P: the multiplicand is in slot 1
-                        __syncwarp();
-#pragma unroll
-                        for (int d = 0; d < ND; ++d) {
-                            for (int i = lane; i < SH::TS; i += 32) sm->T[d][0][i] = sm->T[d][1][i];
-                            for (int i = lane; i < 8 * NT; i += 32) sm->phi[d][0][i] = sm->phi[d][1][i];
-                        }
-                        __syncwarp();
-                        TR::step(sm, r, lane);
+                    for (int d = 0; d < ND; ++d) {
+                        for (int i = lane; i < SH::TS; i += 32) sm->T[d][0][i] = sm->T[d][1][i];
+                        for (int i = lane; i < 8 * NT; i += 32) sm->phi[d][0][i] = sm->phi[d][1][i];
                     }
+                    __syncwarp();
+                    TR::step(sm, r, lane);
                 }
             }
-            TR::sum_phi(r, lane);
-            const int gg = lane >> 2, t = lane & 3;
+        }
+        TR::sum_phi(r, lane);
+        const int gg = lane >> 2, t = lane & 3;
 #pragma unroll
-            for (int d = 0; d < ND; ++d) {
-                if (d == 0 && blockIdx.y != 0) continue;
-                double* out = tr.prop + ((size_t)pos * tr.mats + (d ? 1 + blockIdx.y : 0)) * (N * SH::NS);
+        for (int d = 0; d < ND; ++d) {
+            if (d == 0 && blockIdx.y != 0) continue;
+            double* out = tr.prop + ((size_t)pos * tr.mats + (d ? 1 + blockIdx.y : 0)) * (N * SH::NS);
 #pragma unroll
-                for (int I = 0; I < NT; ++I) {
-                    const int rw = 8 * I + gg;
-                    if (rw < N) {
+            for (int I = 0; I < NT; ++I) {
+                const int rw = 8 * I + gg;
+                if (rw < N) {
 #pragma unroll
-                        for (int J = 0; J < NT; ++J)
+                    for (int J = 0; J < NT; ++J)
 #pragma unroll
-                            for (int e = 0; e < 2; ++e)
-                                if (8 * J + 2 * t + e < N) out[rw * SH::NS + 8 * J + 2 * t + e] = r.P[d][I][J][e];
-                        if (t == 0) out[rw * SH::NS + N] = r.f[d][I];
-                    }
+                        for (int e = 0; e < 2; ++e)
+                            if (8 * J + 2 * t + e < N) out[rw * SH::NS + 8 * J + 2 * t + e] = r.P[d][I][J][e];
+                    if (t == 0) out[rw * SH::NS + N] = r.f[d][I];
                 }
             }
         }

@@ -80,9 +80,22 @@ def _close(z, P, M0, ev, nc, tol=1e-10):
 @pytest.mark.gpu
 @pytest.mark.parametrize("nc", range(6))
 @pytest.mark.parametrize("samples", [8, 33])
-def test_pool_counts_match_the_oracle(cuda, nc, samples):
+@pytest.mark.parametrize("skew", [0.05, 0.0], ids=["skewed", "mirrored"])
+def test_pool_counts_match_the_oracle(cuda, nc, samples, skew):
     P, M0 = _voxels(3, nc, mt=nc != 1)
-    ev = _table([_row(f, pulses=9, samples=samples) for f in OFFSETS])
+    ev = _table([_row(f, pulses=9, samples=samples, skew=skew) for f in OFFSETS])
+    _close(_simulate(cuda, P, M0, ev, nc), P, M0, ev, nc)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nc", [1, 4])
+def test_mirrored_pulses_need_the_pools_fractions(cuda, nc):
+    """Tiny, zero and negative fractions, with and without exchange: chains without the balance take the whole pulse."""
+    P, M0 = _voxels(6, nc, seed=29)
+    P[3 + nc:3 + 2 * nc, 1:6] = np.array([1e-7, 1e-18, 1e-25, 0.0, -1e-4])[None]
+    M0[:, 2 * nc + 3:3 * nc + 3] = P[3 + nc:3 + 2 * nc].T
+    P[3:3 + nc, 4] = 0.0
+    ev = _table([_row(f, samples=24, skew=0.0) for f in OFFSETS])
     _close(_simulate(cuda, P, M0, ev, nc), P, M0, ev, nc)
 
 
@@ -102,6 +115,9 @@ FORMS = {
     "strong": dict(b1=8.0, tp=0.02),
     "beyond_the_bound": dict(b1=30.0, tp=0.02),
     "negative_lobes": dict(skew=-4.0),
+    "mirrored": dict(skew=0.0, samples=21),
+    "mirrored_even": dict(skew=0.0, samples=40, phase=0.4, phase_step=1.0),
+    "mirrored_strong": dict(skew=0.0, samples=9, b1=8.0, tp=0.01),
     "samples_1100": dict(samples=1100, tp=0.05, pulses=4),
 }
 
