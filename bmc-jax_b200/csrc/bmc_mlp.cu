@@ -142,9 +142,9 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 }
 
 // shared-memory matrix descriptor: K-major, no swizzle, 128 B between core matrices along K (LBO),
-// 1024 B between 8-row groups (SBO), descriptor version 1
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
-    return uint64_t((addr >> 4) & 0x3FFFu) | (uint64_t(128 >> 4) << 16) | (uint64_t(1024 >> 4) << 32) |
+// `group` bytes (1024 for 64-deep tiles) between 8-row groups (SBO), descriptor version 1
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t group = 1024) {
+    return uint64_t((addr >> 4) & 0x3FFFu) | (uint64_t(128 >> 4) << 16) | (uint64_t(group >> 4) << 32) |
            (uint64_t(1) << 46);
 }
 // instruction descriptor: fp32 accumulator, bf16 A and B, both K-major, M = 128, N = n
@@ -562,6 +562,184 @@ __global__ void adam_dev_kernel(LayerMap L, float* __restrict__ p, const float* 
 __global__ void step_advance_kernel(int* d_step) { *d_step += 1; }
 
 // ------------------------------------------------------------------------------------------------
+// inference: the whole network in one kernel
+// ------------------------------------------------------------------------------------------------
+// A CTA takes 128 rows at a time through every layer: their activations stay in shared memory (bf16, the core-matrix
+// layout the MMAs read), the weights stream through a two-stage ring of 32-deep chunks, each layer's first two loaded
+// while the layer before it is in its epilogue, and the accumulator (128 x 256 in TMEM) goes through bias and
+// GELU straight back into shared memory. One kernel per layer instead wrote and read every activation through memory
+// (33 MB a layer at 65,536 rows) and left its SMs idle between a tile's loads, products and epilogue: 254 us
+// a call with 244 inputs, three layers and six outputs, 172 us here. Two CTAs share an SM where the inputs fit beside
+// (up to 256), so one's products and loads run under the other's epilogue; one CTA of 512 threads with a four-stage
+// ring of 64-deep chunks took 183 us. What bounds it now is the instructions of the epilogue (GELU on 50 million
+// values) and of the inputs' normalisation.
+constexpr int kInferThreads = 256;
+constexpr int kInferH = 256;                 // the hidden width it is built for
+constexpr int kInferMaxIn = 320;             // padded inputs (five activation blocks of 64)
+constexpr uint32_t kInferBlock = 128 * 128;  // one activation block: 128 rows x 64 bf16
+constexpr int kInferDepth = 32;              // K of a weight chunk
+constexpr uint32_t kInferStage = kInferH * kInferDepth * 2;
+constexpr int kInferStages = 2;
+constexpr uint32_t kInferVectors = (2 * kInferMaxIn + (kMaxLayers - 1) * kInferH + 64) * 4;   // shift, scale, biases at most
+
+struct InferArgs {
+    const float *x, *shift, *scale;
+    long long batch;
+    int n_in, in_pad, L, n_out, tiles;
+    const bf16* w[kMaxLayers];
+    const float* b[kMaxLayers];
+    float* y;
+    int* status;
+};
+
+static __global__ void __launch_bounds__(kInferThreads, 2) infer_kernel(const InferArgs g) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    __shared__ __align__(8) uint64_t bars[kInferStages];
+    __shared__ uint32_t tmem_slot;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int act_blocks = max(kInferH, g.in_pad) / 64;
+    const uint32_t act = smem_addr(smem), ring = act + act_blocks * kInferBlock;
+    if (warp == 0) tmem_alloc(smem_addr(&tmem_slot), kInferH);
+    if (tid == 0) {
+        for (int i = 0; i < kInferStages; ++i) mbar_init(smem_addr(&bars[i]), 1);
+        fence_barrier_init();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_slot;
+    // the input's shift and scale and every bias, behind the ring
+    float* vec = reinterpret_cast<float*>(smem + act_blocks * kInferBlock + kInferStages * kInferStage);
+    float* bias = vec + 2 * g.in_pad;
+    for (int i = tid; i < g.in_pad; i += kInferThreads) {
+        vec[i] = g.shift && i < g.n_in ? g.shift[i] : 0.0f;
+        vec[g.in_pad + i] = g.scale && i < g.n_in ? g.scale[i] : 1.0f;
+    }
+    for (int i = tid; i < g.L * kInferH + 64; i += kInferThreads) bias[i] = g.b[i / kInferH][i % kInferH];
+    __syncthreads();
+
+    // chunk `c` of layer `l` into its stage; `n` counts the kernel's chunks (stage n % 2, its use n / 2)
+    auto load = [&](int l, int c, uint32_t n) {
+        const int rows = l < g.L ? kInferH : 64, ld = l == 0 ? g.in_pad : kInferH;
+        const uint32_t b = ring + (n % kInferStages) * kInferStage;
+        for (int i = tid; i < rows * 4; i += kInferThreads) {
+            const int r = (i >> 5) * 8 + (i & 7), q = (i >> 3) & 3;
+            cp_async16(b + (r >> 3) * 512 + q * 128 + (r & 7) * 16, g.w[l] + size_t(r) * ld + c * kInferDepth + q * 8);
+        }
+        cp_async_commit();
+    };
+    auto chunks_of = [&](int l) { return (l == 0 ? g.in_pad : kInferH) / kInferDepth; };
+
+    bool ok = true;
+    uint32_t n0 = 0;                         // the current layer's first chunk
+    for (int c = 0; c < min(chunks_of(0), kInferStages); ++c) load(0, c, c);
+    for (int tile = blockIdx.x; ok && tile < g.tiles; tile += gridDim.x) {
+        const long long m0 = (long long)tile * 128;
+        // the rows' inputs, normalised: a warp takes 8 rows x 32 columns at a time, two such pieces in flight
+        constexpr int kWarps = kInferThreads / 32;
+        const int pieces = 16 * (g.in_pad / 32);             // a multiple of 32
+        for (int i0 = warp; i0 < pieces; i0 += 2 * kWarps) {
+            float f[2][8];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int i = i0 + u * kWarps, k0 = ((i >> 4) * 4 + (lane >> 3)) * 8;
+                const long long m = m0 + (i & 15) * 8 + (lane & 7);
+                const float* px = g.x + size_t(m) * g.n_in + k0;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) f[u][j] = m < g.batch && k0 + j < g.n_in ? px[j] : 0.0f;
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int i = i0 + u * kWarps, q = (i >> 4) * 4 + (lane >> 3), r = (i & 15) * 8 + (lane & 7);
+                const bool row = m0 + r < g.batch;
+                __align__(16) bf16 v[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int k = q * 8 + j;
+                    v[j] = __float2bfloat16_rn(row && k < g.n_in ? (f[u][j] - vec[k]) * vec[g.in_pad + k] : 0.0f);
+                }
+                *reinterpret_cast<uint4*>(smem + (q >> 3) * kInferBlock + (r >> 3) * 1024 + (q & 7) * 128 + (r & 7) * 16) =
+                    *reinterpret_cast<const uint4*>(v);
+            }
+        }
+        for (int l = 0; ok && l <= g.L; ++l) {
+            const int nk = chunks_of(l), nn = l < g.L ? kInferH : 64;
+            int issued = min(nk, kInferStages);
+            for (int c = 0; ok && c < nk; ++c) {
+                const uint32_t n = n0 + c;
+                const int pending = issued - (c + 1);
+                if (pending >= 1) cp_async_wait<1>();
+                else cp_async_wait<0>();
+                fence_proxy_async();         // this thread's weights and activations -> visible to the tensor core
+                tc_fence_before();
+                __syncthreads();
+                if (tid == 0) {
+                    tc_fence_after();
+                    const uint32_t a = act + (c >> 1) * kInferBlock + (c & 1) * 512;
+                    const uint32_t b = ring + (n % kInferStages) * kInferStage;
+#pragma unroll
+                    for (int j = 0; j < 2; ++j)
+                        umma_bf16(tmem, smem_desc(a + j * 256), smem_desc(b + j * 256, 512), idesc_bf16(nn), (c | j) != 0);
+                    umma_commit(smem_addr(&bars[n % kInferStages]));
+                }
+                if (issued < nk) {           // the stage is free once this chunk's MMAs are done
+                    const bool w = mbar_wait(smem_addr(&bars[n % kInferStages]), (n / kInferStages) & 1);
+                    ok = __syncthreads_and(w);
+                    if (ok) load(l, issued, n + kInferStages);
+                    ++issued;
+                }
+            }
+            if (!ok) break;
+            // the last commit covers the layer's MMAs: the activations and the ring are free
+            const uint32_t last = n0 + nk - 1;
+            ok = __syncthreads_and(mbar_wait(smem_addr(&bars[last % kInferStages]), (last / kInferStages) & 1));
+            if (!ok) break;
+            tc_fence_after();
+            n0 += nk;
+            const int nl = l < g.L ? l + 1 : 0;
+            if (nl > 0 || tile + gridDim.x < g.tiles)
+                for (int c = 0; c < min(chunks_of(nl), kInferStages); ++c) load(nl, c, n0 + c);
+            const int row = (warp & 3) * 32 + lane;
+            const uint32_t trow = tmem + (uint32_t((warp & 3) * 32) << 16);
+            if (l < g.L) {
+#pragma unroll 1
+                for (int cb = (warp >> 2) * 128; cb < (warp >> 2) * 128 + 128; cb += 16) {
+                    float v[16];
+                    tmem_ld16(trow + cb, v);
+                    const float4* b4 = reinterpret_cast<const float4*>(bias + l * kInferH + cb);
+                    __align__(16) bf16 h[16];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const float4 bb = b4[q];
+                        h[4 * q] = __float2bfloat16_rn(gelu(v[4 * q] + bb.x));
+                        h[4 * q + 1] = __float2bfloat16_rn(gelu(v[4 * q + 1] + bb.y));
+                        h[4 * q + 2] = __float2bfloat16_rn(gelu(v[4 * q + 2] + bb.z));
+                        h[4 * q + 3] = __float2bfloat16_rn(gelu(v[4 * q + 3] + bb.w));
+                    }
+                    uint8_t* p = smem + (cb >> 6) * kInferBlock + (row >> 3) * 1024 + ((cb & 63) >> 3) * 128 + (row & 7) * 16;
+                    *reinterpret_cast<uint4*>(p) = reinterpret_cast<const uint4*>(h)[0];
+                    *reinterpret_cast<uint4*>(p + 128) = reinterpret_cast<const uint4*>(h)[1];
+                }
+            } else {
+                for (int cb = (warp >> 2) * 32; cb < min((warp >> 2) * 32 + 32, g.n_out); cb += 16) {
+                    float v[16];
+                    tmem_ld16(trow + cb, v);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        if (cb + i < g.n_out && m0 + row < g.batch)
+                            g.y[size_t(m0 + row) * g.n_out + cb + i] = v[i] + bias[l * kInferH + cb + i];
+                }
+            }
+        }
+    }
+    cp_async_wait<0>();
+    if (!ok && tid == 0 && g.status) atomicOr(g.status, 1);
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(tmem, kInferH);
+}
+
+// ------------------------------------------------------------------------------------------------
 // host side: shapes, buffer carving, launches
 // ------------------------------------------------------------------------------------------------
 long long rup(long long x, long long m) { return (x + m - 1) / m * m; }
@@ -712,6 +890,32 @@ bmc_status forward_impl(const Shape& s, const float* params, const bf16* shadow,
                         const float* scale, long long batch, float* y, const Work& w, bool keep,
                         cudaStream_t st) {
     const LayerMap M = layer_map(s);
+    if (!keep && y && s.H == kInferH && s.in_pad <= kInferMaxIn && s.out_pad == 64) {
+        InferArgs a{};
+        a.x = x; a.shift = shift; a.scale = scale;
+        a.batch = batch;
+        a.n_in = s.n_in; a.in_pad = s.in_pad; a.L = s.L; a.n_out = s.n_out; a.tiles = w.rows / 128;
+        for (int l = 0; l <= s.L; ++l) {
+            a.w[l] = shadow + M.sh_w[l];
+            a.b[l] = params + M.off_b[l];
+        }
+        a.y = y;
+        a.status = w.status;
+        const uint32_t bytes = uint32_t(std::max(kInferH, s.in_pad) / 64) * kInferBlock + kInferStages * kInferStage +
+                               (2 * s.in_pad + s.L * kInferH + 64) * 4;
+        static std::atomic<unsigned long long> configured{0};
+        int dev = 0;
+        MLP_CUDA_TRY(cudaGetDevice(&dev));
+        if (dev >= 64 || !((configured.load(std::memory_order_acquire) >> dev) & 1ull)) {
+            MLP_CUDA_TRY(cudaFuncSetAttribute(infer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              int((kInferMaxIn / 64) * kInferBlock + kInferStages * kInferStage +
+                                                  kInferVectors)));
+            if (dev < 64) configured.fetch_or(1ull << dev, std::memory_order_acq_rel);
+        }
+        infer_kernel<<<unsigned(std::min(a.tiles, 2 * 148)), kInferThreads, bytes, st>>>(a);
+        MLP_CUDA_TRY(cudaGetLastError());
+        return BMC_OK;
+    }
     if (!keep) {
         // (w.rows is a multiple of 128)
         for (long long r0 = 0; r0 < w.rows; r0 += 65535ll * kPrepRows) {

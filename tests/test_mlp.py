@@ -228,3 +228,25 @@ def test_training_fits_a_teacher_network(cuda):
     hist = net.train(torch.as_tensor(x).cuda(), torch.as_tensor(t.astype(np.float32)).cuda(), epochs=30,
                      batch=1024, lr=2e-3, seed=1)
     assert hist[-1] < 0.1 * hist[0], hist
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_in,n_out,layers,batch", [(244, 6, 3, 4096), (1, 1, 1, 1), (64, 16, 2, 127), (65, 17, 3, 129),
+                                                     (320, 64, 8, 300), (321, 5, 2, 200), (40, 65, 2, 130),
+                                                     (100, 8, 3, 148 * 128 + 1), (256, 48, 2, 2 * 148 * 128 + 77)])
+def test_inference_equals_the_layered_forward(cuda, n_in, n_out, layers, batch):
+    """Inference (the network in one kernel up to 320 inputs and 64 outputs, else a kernel per layer) against the
+    training forward of the same rows: the same bf16 roundings and fp32 sums of the same chunks (1e-5 of the largest
+    output: a bf16 unit of one activation, 2^-8, through a layer of 256 weights of ~1/16 is ~1e-4 of an output's scale
+    and would show)."""
+    torch = cuda
+    from bmc_b200.warmstart import MLP
+    net = MLP(n_in, n_out, 256, layers, seed=layers)
+    rng = np.random.default_rng(n_in)
+    net.set_input_normalisation(rng.uniform(0.2, 0.6, n_in), rng.uniform(1.0, 4.0, n_in))
+    x = torch.as_tensor(rng.uniform(0.0, 1.0, (batch, n_in)).astype(np.float32)).cuda()
+    y = net.forward(x)
+    want = net.forward(x, keep=True)
+    assert net.status(batch) == 0
+    assert y.shape == (batch, n_out) and bool(torch.isfinite(y).all())
+    assert float((y - want).abs().max()) <= 1e-5 * float(want.abs().max())
