@@ -16,7 +16,9 @@
 // slow modes' entries keep their digits). A group of lanes takes one chain,
 // lane j < N holding column j of T and of H. T's last row is e_N^T (the augmented row) and is not
 // stored; H's is (E has a last row: v_N lam^T = lam^T). The augmented column of T, phi = T[0:N, N], is
-// kept apart in shared memory, lane i updating row i (phi <- T phi + phi), and the augmented column
+// kept apart in shared memory, lane i updating row i (phi <- T phi + 2 phi; it starts as the Horner recurrence's matrix
+// before its last step, sum_k X^k / (k + 1)!, times the constant column: a recurrence of its own on one lane while the
+// others waited took 4% of the tangent and 9% of the primal pass with four pools), and the augmented column
 // of H is never formed: it enters column j < N only through T[N][j] = 0, and no tangent reads it. So
 // a chain takes N lanes, not N + 1: with four CEST pools (N = 16) two chains share a warp.
 //
@@ -41,7 +43,6 @@ struct AdjGroup {
     // Otherwise the lanes' own FMAs, odd stride (H's columns have N + 1 rows).
     static constexpr bool kMma = N == 16;
     static constexpr int LD = kMma ? 20 : ((N + 1) | 1);
-    static constexpr int PHI_LANE = N < GS ? N : 0;    // the lane that forms phi's Horner recurrence
 };
 
 // D += A B for one 8x8x4 tile (row-major A, column-major B; lane l holds A[l / 4][l % 4], B[l % 4][l / 4]
@@ -303,6 +304,55 @@ struct Adjoint {
         }
         __syncwarp();
     }
+
+    // the same for T and phi alone, of both slots of the warp at once: 16 DMMAs a slot in chains of four do not fill the
+    // pipe by themselves (DMMA and FP64 pipes were busy 55% of the primal pass's cycles; three blocks per SM instead of
+    // two change nothing)
+    static __device__ __forceinline__ void mma_square_both(SL* sl, int lane) {
+        const int g = lane >> 2, t = lane & 3;
+        double c[2][2][2][2];
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const double* T = sl[p].T;
+            double aT[2][4], bT[4][2];
+#pragma unroll
+            for (int I = 0; I < 2; ++I)
+#pragma unroll
+                for (int K = 0; K < 4; ++K) aT[I][K] = T[(4 * K + t) * LD + 8 * I + g];
+#pragma unroll
+            for (int K = 0; K < 4; ++K)
+#pragma unroll
+                for (int J = 0; J < 2; ++J) bT[K][J] = T[(8 * J + g) * LD + 4 * K + t];
+#pragma unroll
+            for (int I = 0; I < 2; ++I)
+#pragma unroll
+                for (int J = 0; J < 2; ++J)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) c[p][I][J][e] = 2.0 * T[(8 * J + 2 * t + e) * LD + 8 * I + g];
+#pragma unroll
+            for (int K = 0; K < 4; ++K)
+#pragma unroll
+                for (int I = 0; I < 2; ++I)
+#pragma unroll
+                    for (int J = 0; J < 2; ++J) dmma(c[p][I][J][0], c[p][I][J][1], aT[I][K], bT[K][J]);
+        }
+        SL* mine = &sl[lane / N];          // phi: lanes 0-15 the first slot's rows, 16-31 the second's
+        const int i = lane % N;
+        double vec = 2.0 * mine->phi[0][i];
+#pragma unroll
+        for (int l = 0; l < N; ++l) vec = fma(mine->T[l * LD + i], mine->phi[0][l], vec);
+        __syncwarp();
+#pragma unroll
+        for (int p = 0; p < 2; ++p)
+#pragma unroll
+            for (int I = 0; I < 2; ++I)
+#pragma unroll
+                for (int J = 0; J < 2; ++J)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) sl[p].T[(8 * J + 2 * t + e) * LD + 8 * I + g] = c[p][I][J][e];
+        mine->phi[0][i] = vec;
+        __syncwarp();
+    }
 };
 
 // kTan false: z only (the same layout and arithmetic without H), for the LM's trial points. Blocks per SM
@@ -318,7 +368,7 @@ adjoint_kernel(const ChainArgs a, const int* __restrict__ row_ev, int n_tan, con
     using C0 = Chain<NC, double, 0>;
     using S = State<NC, D0>;
     using SL = AdjSlot<NC>;
-    constexpr int N = A::N, GS = A::GS, G = A::G, LD = A::LD, PHI_LANE = AdjGroup<NC>::PHI_LANE;
+    constexpr int N = A::N, GS = A::GS, G = A::G, LD = A::LD;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SL* slots = reinterpret_cast<SL*>(smem_raw) + (threadIdx.x >> 5) * G;
     const int lane = threadIdx.x & 31, grp = lane / GS, gl = lane % GS;
@@ -422,11 +472,17 @@ adjoint_kernel(const ChainArgs a, const int* __restrict__ row_ev, int n_tan, con
             // column gl of exp(X / 2^s) and of its derivative along E / 2^s: Horner, T = I + X T / k
             S cv, cd;
             double cdN = 0.0;
+            // before its last step T is sum_k X^k / (k + 1)!, which takes C h to the augmented column phi
+            auto store_column = [&] {
+#pragma unroll
+                for (int i = 0; i < N; ++i) sl->T[gl * LD + i] = C0::at(cv, i).v;
+            };
             A::unit(cv, gl);
             A::unit(cd, -1);
             if (work) {
                 const double e2 = sl->scale;
                 for (int k = tt.dense_m; k >= 1; --k) {
+                    if (k == 1) store_column();
                     S yv;
                     C0::template matvec<false>(sl->coef, cv, yv);
                     const double ik = tt.inv_k[k];
@@ -442,19 +498,15 @@ adjoint_kernel(const ChainArgs a, const int* __restrict__ row_ev, int n_tan, con
                     for (int q = 0; q < N; ++q) C0::at(cv, q).v = (q == gl && k > 1 ? 1.0 : 0.0) + ik * C0::at(yv, q).v;
                 }
             }
-            // the augmented column: [phi; 1] <- e_N + X [phi; 1] / k
-            if (have && gl == PHI_LANE) {
-                S ph;
-                A::unit(ph, -1);
-                for (int k = tt.dense_m; k >= 1; --k) {
-                    S y;
-                    A::op(sl, ph, 1.0, y);
-                    const double ik = tt.inv_k[k];
+            __syncwarp();
+            if (work) {
+                // phi = T_2 (C h): C's entries are the z rows' (water, the pools) and the MT pool's
+                using L = Layout<NC>;
+                double ph = sl->T[L::izw * LD + gl] * sl->cw;
+                ph = fma(sl->T[L::izm * LD + gl], sl->cm, ph);
 #pragma unroll
-                    for (int q = 0; q < N; ++q) C0::at(ph, q).v = ik * C0::at(y, q).v;
-                }
-#pragma unroll
-                for (int q = 0; q < N; ++q) sl->phi[0][q] = C0::at(ph, q).v;
+                for (int i = 0; i < NC; ++i) ph = fma(sl->T[L::izc(i) * LD + gl], sl->cc[i], ph);
+                sl->phi[0][gl] = ph;
             }
             __syncwarp();
             // s squarings
@@ -468,7 +520,12 @@ adjoint_kernel(const ChainArgs a, const int* __restrict__ row_ev, int n_tan, con
                     if constexpr (kTan) sl->H[gl * LD + N] = cdN;
                 }
                 __syncwarp();
-                for (int q = 0; q < smax; ++q) {
+                int q = 0;
+                if constexpr (!kTan) {
+                    const int both = (int)__reduce_min_sync(kFull, (unsigned)s_g);
+                    for (; q < both; ++q) A::mma_square_both(slots, lane);
+                }
+                for (; q < smax; ++q) {
 #pragma unroll
                     for (int c = 0; c < G; ++c) {
                         const int s_c = __shfl_sync(kFull, s_g, c * GS);

@@ -109,13 +109,21 @@ struct ChainArgs {
 // CW, two pools and MT) took 292 us in the kernel with 32 chains per warp, 83 us with one. The chain kernel counts
 // one block per SM as resident: its unrolled term loops stream from the instruction cache, and 714 chains (a fit of
 // 100-sample trains) in 2 chains per warp on 90 blocks took 49.7 ms of tangent passes, in 1 per warp on 179 blocks, two
-// on some SMs, 76.6 (32 per warp: 53.0). A power of two from `least` (the chains a warp's lane groups take at once) to 32.
+// on some SMs, 76.6 (32 per warp: 53.0). A power of two from `least` (the chains a warp's lane groups take at once) to
+// `most`: 32, or 16 for the adjoint passes of up to kFewWaves waves of warps (adjoint_chains_per_warp), whose last wave
+// is then less empty: 93,452 chains of four pools and MT (ten passes of each kind) took 21.0 ms of tangent and 9.9 ms of primal
+// passes at 32, 20.1 and 8.9 at 16, 20.4 and 9.7 at 8 (2.5 waves); 292,800 such chains (7.7 waves) fit 1% faster at 32.
 constexpr int kSMs = 148;
-inline int chains_per_warp(long long chains, int blocks_per_sm, int warps, int least) {
-    int c = 32;
+constexpr int kFewWaves = 4;
+inline int chains_per_warp(long long chains, int blocks_per_sm, int warps, int least, int most = 32) {
+    int c = most;
     const long long slots = (long long)kSMs * blocks_per_sm * warps;
     while (c > least && (chains + c / 2 - 1) / (c / 2) <= slots) c /= 2;
     return c;
+}
+inline int adjoint_chains_per_warp(long long chains, int blocks_per_sm, int warps, int least) {
+    const bool few = chains <= 32ll * kSMs * blocks_per_sm * warps * kFewWaves;
+    return chains_per_warp(chains, blocks_per_sm, warps, least, few ? 16 : 32);
 }
 
 template <int NC>

@@ -97,7 +97,7 @@ bmc_status launch_adjoint(ChainArgs a, const int* row_ev, int n_tan, const Taylo
             a.done = nullptr;
         }
     }
-    a.cpw = chains_per_warp(nch, kTan ? 2 : BMC_ADJ_PRIMAL_BLOCKS, kAdjWarps, AdjGroup<NC>::G);
+    a.cpw = adjoint_chains_per_warp(nch, kTan ? 2 : BMC_ADJ_PRIMAL_BLOCKS, kAdjWarps, AdjGroup<NC>::G);
     const long long blocks = (nch + kAdjWarps * a.cpw - 1) / (kAdjWarps * a.cpw);
     if (blocks > 0x7fffffffLL) return fail(BMC_ERR_INVALID, "%lld chains exceed one launch", nch);
     if (blocks == 0) return BMC_OK;
