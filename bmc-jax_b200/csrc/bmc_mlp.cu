@@ -577,6 +577,11 @@ constexpr int kInferThreads = 256;
 constexpr int kInferH = 256;                 // the hidden width it is built for
 constexpr int kInferMaxIn = 320;             // padded inputs (five activation blocks of 64)
 constexpr uint32_t kInferBlock = 128 * 128;  // one activation block: 128 rows x 64 bf16
+// Up to this many rows a kernel per layer: it spreads a tile's 256 columns over four CTAs where this kernel leaves them
+// to one, and as long as those CTAs have an SM each (37 tiles of 128 rows) that is the shorter chain. 244 inputs and
+// three layers, this kernel against one per layer: 51.5 us and 45.2 at 1,024 rows, 52.5 and 45.3 at 4,736, 53.0 and
+// 60.1 at 5,120, 57.6 and 92.5 at 18,944.
+constexpr long long kInferFromRows = 148 / (kInferH / 64) * 128;
 constexpr int kInferDepth = 32;              // K of a weight chunk
 constexpr uint32_t kInferStage = kInferH * kInferDepth * 2;
 constexpr int kInferStages = 2;
@@ -890,7 +895,7 @@ bmc_status forward_impl(const Shape& s, const float* params, const bf16* shadow,
                         const float* scale, long long batch, float* y, const Work& w, bool keep,
                         cudaStream_t st) {
     const LayerMap M = layer_map(s);
-    if (!keep && y && s.H == kInferH && s.in_pad <= kInferMaxIn && s.out_pad == 64) {
+    if (!keep && y && s.H == kInferH && s.in_pad <= kInferMaxIn && s.out_pad == 64 && w.rows > kInferFromRows) {
         InferArgs a{};
         a.x = x; a.shift = shift; a.scale = scale;
         a.batch = batch;
