@@ -127,6 +127,16 @@ class ClockSampler:
                 "samples": len(sm)}
 
 
+def count_launches(call):
+    """This library's kernels that one (untimed) call launches."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    return sum("bmc::" in e.name for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA)
+
+
 def max_over_ranks(x: float, device=None) -> float:
     """The largest value of x over every rank (the step time of the slowest GPU); x itself alone."""
     import torch
@@ -252,11 +262,21 @@ def run_ours(args, rank, world, local_rank):
         step()
     torch.cuda.synchronize(dev)
 
-    # executed work of one launch (deterministic), from the kernel's own counters
+    # work of the event-by-event pass (deterministic), from the kernel's own counters, and that pass's own time: the
+    # timed step applies whole shaped pulses' propagators instead, whose work the counters do not see
     work = torch.zeros(5, dtype=torch.int64, device=dev)
-    _lib.check(L.bmc_simulate_counted(pr, C.c_void_p(dP.data_ptr()), dev_ev.struct, C.c_void_p(dM.data_ptr()),
-                                      sp, C.c_void_p(dZ.data_ptr()), C.c_void_p(work.data_ptr()), sh))
-    torch.cuda.synchronize(dev)
+    counted_ms = 0.0
+    for _ in range(2):
+        work.zero_()
+        flush.fill_(1.0)
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        e0.record(stream)
+        _lib.check(L.bmc_simulate_counted(pr, C.c_void_p(dP.data_ptr()), dev_ev.struct, C.c_void_p(dM.data_ptr()),
+                                          sp, C.c_void_p(dZ.data_ptr()), C.c_void_p(work.data_ptr()), sh))
+        e1.record(stream)
+        e1.synchronize()
+        counted_ms = e0.elapsed_time(e1)
+    step_launches = count_launches(step)
     terms, hcols, squar, executed, terms32 = [int(x) for x in work.cpu()]
     nnz = 12 + 15 * nc                                   # nonzeros of A (+ C folded into term 1)
     flop_term = 2 * nnz + 2 * N                          # operator product + scaling + accumulation
@@ -314,7 +334,7 @@ def run_ours(args, rank, world, local_rank):
     best32 = fma_peak(_lib.F32)
     t_ideal = flops64 / (best * 1e12) + flops32 / (best32 * 1e12)
     peak_eff = flops / t_ideal / 1e12 if t_ideal > 0 else best
-    achieved = flops / (ms * 1e-3) / 1e12
+    achieved = flops / (counted_ms * 1e-3) / 1e12        # both of the event-by-event pass
     value = world * nv / (ms * 1e-3)
     f32_err = None
     if prec != _lib.F64:
@@ -351,7 +371,7 @@ def run_ours(args, rank, world, local_rank):
                                              "truncation 1e-13 per sub-step",
                                    _lib.MIXED: "the first Taylor term of every sub-step in float64 (more where their "
                                                "bound theta^k/k! exceeds 3x the state), later terms in float32, "
-                                               "summed into the float64 state once per sub-step; truncation 1e-9 "
+                                               "summed into the float64 state once per sub-step; truncation 1e-8 "
                                                "per sub-step",
                                    _lib.F32: "all Taylor terms and the state in float32; truncation 2^-24"}[prec]},
         "e2e": {"value": world * nv / (e2e_ms * 1e-3), "unit": "Z-spectra/s", "h2d_bytes_per_step": h2d,
@@ -359,7 +379,10 @@ def run_ours(args, rank, world, local_rank):
         "roofline": {"bound": "fp64+fp32 fma", "achieved": achieved, "peak": peak_eff, "unit": "TFLOP/s",
                      "frac": achieved / peak_eff if peak_eff else None,
                      "traffic": traffic, "traffic_unit": "bytes per launch",
-                     "traffic_source": traffic_src, "kernel": "chain_kernel",
+                     "traffic_source": traffic_src,
+                     "kernel": "chain_kernel, event by event (bmc_simulate_counted: its work over its own time; the "
+                               "timed step takes shaped pulses as propagators, whose work is not counted)",
+                     "event_by_event_ms": counted_ms,
                      "flops_per_launch": flops, "flops_fp64_pipe": flops64, "flops_fp32_pipe": flops32,
                      "peak_fp64": best, "peak_fp32": best32,
                      "frac_fp64_equivalent": achieved / best if best else None,
@@ -379,7 +402,7 @@ def run_ours(args, rank, world, local_rank):
                                      "(time of the FP64 share at the FP64 peak plus the FP32 share at the "
                                      "FP32 peak)")},
         "clocks": clocks,
-        "gpu_launches": 2 * args.steps,
+        "gpu_launches": step_launches * args.steps,
     }
     # the float64 kernel on the same inputs, timed the same way over at most three steps, for comparison
     if prec != _lib.F64 and not args.spread_nodes:
@@ -910,9 +933,10 @@ def run_uneven(args, rank, world, local_rank):
 
 
 def lm_tangent_roofline(exp, spec, X_phys, peak):
-    """The LM's tangent pass as the fit runs it (every free parameter's derivative at every offset) on
-    `X_phys`, timed with CUDA events on the launching stream, against the kernels' own counts of the work
-    they executed, in both tangent modes. The automatic mode (what bmc_lm_fit runs) takes the adjoint
+    """The LM's tangent pass (every free parameter's derivative at every offset) on `X_phys`, timed with CUDA
+    events on the launching stream, in both tangent modes: as the fit runs it (`ms`), and as the counting call
+    runs it (`ms_counted`: event by event, by the group kernels), whose own counts of the work it executed give
+    the rates. The automatic mode (what bmc_lm_fit runs) takes the adjoint
     kernel on a single-event table such as the CW ladder: one launch, the exponential and its Frechet
     derivative in the readout's direction as a pair (dual) -- FLOPs per squaring 6 N^2 (N + 1), per Horner
     column product two operator products and a rank-one update -- then every tangent by a contraction
@@ -954,21 +978,27 @@ def lm_tangent_roofline(exp, spec, X_phys, peak):
     for mode in ("auto", "forward"):
         settings.use_tangents(mode)
         try:
-            call()
+            def timed(f):
+                f()
+                torch.cuda.synchronize()
+                e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                e0.record(stream)
+                f()
+                e1.record(stream)
+                e1.synchronize()
+                return e0.elapsed_time(e1)
             work = torch.zeros(5, dtype=torch.int64, device="cuda")
-            _lib.check(L.bmc_simulate_jvp_counted(pr, _lib.ptr(dP), dev_ev.struct, _lib.ptr(dM), None, tg,
-                                                  _lib.ptr(z), _lib.ptr(jz), _lib.ptr(work), sh))
-            torch.cuda.synchronize()
-            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            e0.record(stream)
-            call()
-            e1.record(stream)
-            e1.synchronize()
-            out[mode] = ([int(x) for x in work.cpu()], e0.elapsed_time(e1))
+
+            def counted():
+                work.zero_()
+                _lib.check(L.bmc_simulate_jvp_counted(pr, _lib.ptr(dP), dev_ev.struct, _lib.ptr(dM), None, tg,
+                                                      _lib.ptr(z), _lib.ptr(jz), _lib.ptr(work), sh))
+            ms_counted = timed(counted)
+            out[mode] = ([int(x) for x in work.cpu()], ms_counted, timed(call))
         finally:
             settings.use_tangents("auto")
-    (terms, hcols, squar, _, _), ms = out["auto"]
-    (terms_f, hcols_f, squar_f, _, _), ms_f = out["forward"]
+    (terms, hcols, squar, _, _), ms, ms_fit = out["auto"]
+    (terms_f, hcols_f, squar_f, _, _), ms_f, ms_fit_f = out["forward"]
     flops_f = (terms_f * flop_term + hcols_f * flop_term + squar_f * 2.0 * N * N * (N + 1)) * (1 + 2 * T)
     adjoint = P > 1 and terms == 0 and squar_f == launches_fwd * squar
     if adjoint:
@@ -981,9 +1011,9 @@ def lm_tangent_roofline(exp, spec, X_phys, peak):
     tf_f = flops_f / (ms_f * 1e-3) / 1e12
     return {"bound": "fp64-fma", "achieved": tf, "peak": peak, "unit": "TFLOP/s",
             "frac": tf / peak if peak else None, "traffic": None, "kernel": kernel,
-            "voxels": n, "offsets": dev_ev.n_offsets, "ms": ms, "flops": flops, "taylor_terms": terms,
+            "voxels": n, "offsets": dev_ev.n_offsets, "ms": ms_fit, "ms_counted": ms, "flops": flops, "taylor_terms": terms,
             "dense_columns": hcols, "dense_squarings": squar,
-            "forward_mode": {"ms": ms_f, "launches": launches_fwd, "flops": flops_f, "achieved": tf_f,
+            "forward_mode": {"ms": ms_fit_f, "ms_counted": ms_f, "launches": launches_fwd, "flops": flops_f, "achieved": tf_f,
                              "frac": tf_f / peak if peak else None,
                              "kernel": f"chain_kernel<{nc}, double, {T}>"},
             "peak_source": "the forward leg's FP64 FMA probe of this run (burst)"}
