@@ -755,8 +755,9 @@ struct Train {
     }
 };
 
-// Bound by the FP64 pipes, tensor and vector taking turns: 2.63 ms for 19,493 chains of 200 samples with four pools
-// (dmma pipe 38% active, DFMA pipe 32%), where the Taylor action of every event took 31.6 ms.
+// Bound by the FP64 pipes, tensor and vector taking turns: 1.86 ms for 19,493 chains of 200 samples with four pools
+// (dmma pipe 31% active, DFMA pipe 31%; 2.63 ms where the shape is not its own mirror image), where the Taylor action
+// of every event took 31.6 ms.
 // DT = 1: blockIdx.y is the tangent of the launch whose derivative the block forms, behind the values (tangent 0's
 // blocks write the values too). One tangent costs three times a propagator; the Taylor action of every event with dual
 // numbers took 12.6 ms for the three tangents of 714 chains (one pool, 10 pulses of 100 samples), this 0.53 ms.

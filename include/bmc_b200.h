@@ -232,14 +232,15 @@ bmc_status bmc_normal_blocks(int32_t n_voxels, int32_t n_points, int32_t n_tange
  * bmc_simulate (bit-identical Z: every chain chooses its own Taylor degree and float32 switch point, so
  * the order the chains run in does not matter). Its only scratch, the preprocessed event records and a
  * status word, lives in one static device array of 32 MiB per GPU that loads the library, held until
- * exit, so n_offsets x n_events may be at most 699,045 records in float64 (1,048,568 in float32);
- * larger tables are rejected with BMC_ERR_INVALID and a message. The CUDA driver reserves the array
+ * exit (a second one of 32 MiB holds shaped pulses' propagators, for as many chains at a time as fit),
+ * so n_offsets x n_events may be at most 699,045 records in float64 (1,048,568 in float32);
+ * larger tables are rejected with BMC_ERR_INVALID and a message. The CUDA driver reserves the arrays
  * when it loads the library's device code on a device, which under CUDA's default lazy loading is the
  * first bmc_* call there: a caller whose framework reserves most of the GPU up front (JAX's
  * preallocation) makes one call, e.g. a bmc_simulate_noalloc of a tiny problem, on every device before
  * that reservation, or runs with CUDA_MODULE_LOADING=EAGER. The first call on a device also takes the
- * array's device address and uploads the Taylor tables (issue it before any stream capture). Every call
- * reuses the same array and overwrites the previous call's records: calls that overlap on the GPU
+ * arrays' device addresses and uploads the Taylor tables (issue it before any stream capture). Every call
+ * reuses the same arrays and overwrites the previous call's records: calls that overlap on the GPU
  * (other streams, other host threads) race and must be serialised by the caller. Numerical failures
  * show as NaN in d_out, as for bmc_simulate; the status word is not reported.
  */
@@ -370,7 +371,10 @@ bmc_status bmc_mlp_adam_step_dev(const bmc_mlp_shape* shape, float* d_params, co
  *   zeroed by the caller): [0] Taylor sub-step terms each chain needed (one sparse operator product
  *   each), [1] dense-path Horner column products, [2] dense-path squarings, [3] Taylor terms executed
  *   (a warp runs to the largest need among its chains), [4] of the terms in [0], those formed in float32.
- * bmc_simulate_jvp_counted: bmc_simulate_jvp that adds the same five counts to d_work[5], summed over
+ *   It integrates event by event and by the warp's lane groups: shaped pulses' propagators and exponentials
+ *   by a chain's own thread, which bmc_simulate takes where they are faster, are not counted, so time this
+ *   call, not bmc_simulate, against its counts. The results agree to the precision's tolerance.
+ * bmc_simulate_jvp_counted: bmc_simulate_jvp, likewise event by event, that adds the same five counts to d_work[5], summed over
  *   its launches: in forward mode one per tangent (two per launch for at most one CEST pool), each
  *   carrying the primal and its tangents through the same steps as dual numbers; in the adjoint kernel
  *   one launch whose [1] counts the Horner column products of the pair (exp, Frechet derivative) and
