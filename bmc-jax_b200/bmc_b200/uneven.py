@@ -174,6 +174,7 @@ class _JointSteps:
         self.batch, self.n, self.PL, self.S, self.P = batch, n, PL, S, P
         scl = spec.scales
         self.scl_loc = [float(scl[l]) for l in loc]
+        self.c_scl = (C.c_double * PL)(*self.scl_loc)
         self.scl_s = float(scl[shr[0]]) if S else 0.0
         free = np.zeros((n, PL))
         for g in batch.groups:
@@ -184,6 +185,7 @@ class _JointSteps:
                 g.rows.append(field_row(sl.field, sl.index, g.nc) if ok else None)
                 if ok:
                     free[g.voxels, j] = 1.0
+            g.c_rows = (C.c_int32 * PL)(*[-1 if row is None else row for row in g.rows])
             g.row_s = field_row(spec.slots[shr[0]].field, spec.slots[shr[0]].index, g.nc) if S else None
             for k, v in enumerate(g.voxels):
                 zv = np.asarray(z_meas[v], np.float64).reshape(-1)
@@ -194,8 +196,6 @@ class _JointSteps:
             g.zm = torch.as_tensor(np.concatenate([np.asarray(z_meas[v], np.float64).reshape(-1)
                                                    for v in g.voxels])).cuda()
             g.idx = torch.as_tensor(g.voxels).cuda()
-            g.seg = torch.repeat_interleave(torch.arange(ng, device="cuda"),
-                                            torch.as_tensor(np.diff(g.chain_start)).cuda())
             # tangents: the local slots (zero where a slot does not apply) then the shared one
             tg = _lib.Tangents()
             tg.n_tangents = P
@@ -215,9 +215,10 @@ class _JointSteps:
             g.jz = torch.empty((P, g.n_chains), **f64)
             g.z_n, g.z_t, g.r = (torch.zeros(g.n_chains, **f64) for _ in range(3))
             g.p_n, g.p_t = torch.empty_like(g.params), torch.empty_like(g.params)
-            g.act = torch.ones(ng, dtype=torch.int32, device="cuda")
             g.Hg, g.gg, g.cg = torch.empty((ng, P, P), **f64), torch.empty((ng, P), **f64), torch.empty(ng, **f64)
         f64 = dict(dtype=torch.float64, device="cuda")
+        # one flag for every voxel of any group: they move together
+        self.act = torch.ones(max(len(g.voxels) for g in batch.groups), dtype=torch.int32, device="cuda")
         self.free = torch.as_tensor(free).cuda()
         self.free_np = free
         self.H, self.g, self.c = torch.empty((n, P, P), **f64), torch.empty((n, P), **f64), torch.empty(n, **f64)
@@ -228,24 +229,21 @@ class _JointSteps:
         self.L = _lib.lib()
 
     def _params_into(self, g, buf, x_loc, x_s):
-        buf.copy_(g.params)
-        xv = x_loc.index_select(0, g.idx)
-        for j, row in enumerate(g.rows):
-            if row is not None:
-                buf[row].copy_(xv[:, j] * self.scl_loc[j])
-        if self.S:
-            buf[g.row_s].copy_((x_s * self.scl_s).expand(buf.shape[1]))
+        _lib.check(self.L.bmc_joint_params(buf.shape[1], buf.shape[0], _lib.ptr(g.params), _lib.ptr(g.idx),
+                                           _lib.ptr(x_loc), self.PL, g.c_rows, self.c_scl,
+                                           g.row_s if self.S else -1, self.scl_s, _lib.ptr(x_s) if self.S else None,
+                                           _lib.ptr(buf), _lib.stream_handle()))
 
     def normal(self, x_loc, x_s, moved=None):
         """Every voxel's J^T J, J^T r and r.r at (x_loc, x_s); returns the (1,) total r.r. With `moved` a
         (1,) bool tensor that is False, the kernels skip every voxel and the normal equations stay those of
         the unchanged point (same J, same r)."""
         torch = _lib.torch_cuda()
+        if moved is not None:
+            self.act.copy_(moved.expand(self.act.shape[0]))
         for g in self.batch.groups:
-            if moved is not None:
-                g.act.copy_(moved.to(torch.int32).expand(g.act.shape[0]))
             self._params_into(g, g.p_n, x_loc, x_s)
-            g.plan.run(g.p_n, g.m0, g.tangents, g.jz, z=g.z_n, active=None if moved is None else g.act)
+            g.plan.run(g.p_n, g.m0, g.tangents, g.jz, z=g.z_n, active=None if moved is None else self.act)
             torch.sub(g.z_n, g.zm, out=g.r)
             _lib.check(self.L.bmc_normal_segments(len(g.voxels), self.P, g.n_chains, _lib.ptr(g.d_chain_start),
                                                   _lib.ptr(g.jz), _lib.ptr(g.r), _lib.ptr(g.Hg), _lib.ptr(g.gg),
@@ -271,13 +269,12 @@ class _JointSteps:
 
     def costs(self, x_loc, x_s):
         """(n,) r.r of every voxel at (x_loc, x_s)."""
-        torch = _lib.torch_cuda()
         for g in self.batch.groups:
             self._params_into(g, g.p_t, x_loc, x_s)
             g.plan.run(g.p_t, g.m0, z=g.z_t)
-            rt = g.z_t - g.zm
-            self.cost_v.index_copy_(0, g.idx, torch.zeros(len(g.voxels), dtype=torch.float64,
-                                                          device="cuda").index_add_(0, g.seg, rt * rt))
+            _lib.check(self.L.bmc_segment_costs(len(g.voxels), _lib.ptr(g.d_chain_start), _lib.ptr(g.z_t),
+                                                _lib.ptr(g.zm), _lib.ptr(g.idx), _lib.ptr(self.cost_v),
+                                                _lib.stream_handle()))
         return self.cost_v
 
 

@@ -659,6 +659,43 @@ bmc_status bmc_normal_segments(int32_t n_voxels, int32_t n_params, int64_t n_cha
     return BMC_OK;
 }
 
+bmc_status bmc_joint_params(int32_t n_voxels, int32_t n_fields, const double* d_base, const int64_t* d_index,
+                            const double* d_x, int32_t n_local, const int32_t* rows, const double* scales,
+                            int32_t shared_row, double shared_scale, const double* d_shared, double* d_out,
+                            void* stream) {
+    if (n_voxels < 1 || n_fields < 1 || n_local < 0 || n_local > kMaxJointP - 1 || shared_row >= n_fields)
+        return fail(BMC_ERR_INVALID, "joint parameters: %d voxels, %d fields, %d local values (0..%d), shared row %d",
+                    n_voxels, n_fields, n_local, kMaxJointP - 1, shared_row);
+    if (!d_base || !d_index || !d_out || (n_local && (!d_x || !rows || !scales)) || (shared_row >= 0 && !d_shared))
+        return fail(BMC_ERR_INVALID, "joint parameters: null pointer");
+    JointRows jr{};
+    jr.n = n_local;
+    for (int j = 0; j < n_local; ++j) {
+        if (rows[j] >= n_fields) return fail(BMC_ERR_INVALID, "joint parameters: row %d of %d", rows[j], n_fields);
+        jr.row[j] = rows[j];
+        jr.scale[j] = scales[j];
+    }
+    jr.shared_row = shared_row;
+    jr.shared_scale = shared_scale;
+    const long long n = (long long)n_voxels * n_fields;
+    joint_params_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+        n_voxels, n_fields, d_base, reinterpret_cast<const long long*>(d_index), d_x, d_shared, jr, d_out);
+    CUDA_TRY(cudaGetLastError());
+    return BMC_OK;
+}
+
+bmc_status bmc_segment_costs(int32_t n_voxels, const int64_t* d_chain_start, const double* d_z, const double* d_zm,
+                             const int64_t* d_index, double* d_cost, void* stream) {
+    if (n_voxels < 1) return fail(BMC_ERR_INVALID, "segment costs: %d voxels", n_voxels);
+    if (!d_chain_start || !d_z || !d_zm || !d_index || !d_cost)
+        return fail(BMC_ERR_INVALID, "segment costs: null pointer");
+    segment_costs_kernel<<<(unsigned)(((long long)n_voxels * 32 + 127) / 128), 128, 0, (cudaStream_t)stream>>>(
+        n_voxels, reinterpret_cast<const long long*>(d_chain_start), d_z, d_zm,
+        reinterpret_cast<const long long*>(d_index), d_cost);
+    CUDA_TRY(cudaGetLastError());
+    return BMC_OK;
+}
+
 bmc_status bmc_schur_step(int32_t n_voxels, int32_t n_local, int32_t n_shared, const double* d_H, const double* d_g,
                           const double* d_free, double lam, const double* d_lam, double* d_dx_local,
                           double* d_dx_shared, double* d_work, void* stream) {

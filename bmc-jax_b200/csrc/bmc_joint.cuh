@@ -14,6 +14,45 @@ namespace bmc {
 
 constexpr int kMaxJointP = 9;  // local values + the shared one
 
+// A group's parameters at a point, in one launch: the joint step wrote them a row at a time, two small kernels a row,
+// and with the costs' five per group that was half of an iteration's ~250 launches (192 voxels of five pool counts,
+// 12 iterations: 34.1 ms, now 25.7).
+struct JointRows {
+    int row[kMaxJointP];       // per local value its parameter row, -1: none
+    double scale[kMaxJointP];
+    int n, shared_row;
+    double shared_scale;
+};
+static __global__ void joint_params_kernel(int n_vox, int n_fields, const double* __restrict__ base,
+                                           const long long* __restrict__ index, const double* __restrict__ x,
+                                           const double* __restrict__ xs, const __grid_constant__ JointRows jr,
+                                           double* __restrict__ out) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (long long)n_vox * n_fields) return;
+    const int f = (int)(i / n_vox), v = (int)(i % n_vox);
+    double p = base[i];
+    for (int j = 0; j < jr.n; ++j)
+        if (jr.row[j] == f) p = x[index[v] * jr.n + j] * jr.scale[j];
+    if (jr.shared_row == f) p = xs[0] * jr.shared_scale;
+    out[i] = p;
+}
+
+// a warp per sample, its chains in normal_segments_kernel's order
+static __global__ void segment_costs_kernel(int n_vox, const long long* __restrict__ seg, const double* __restrict__ z,
+                                            const double* __restrict__ zm, const long long* __restrict__ index,
+                                            double* __restrict__ cost) {
+    const int warp = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
+    const int lane = threadIdx.x & 31;
+    if (warp >= n_vox) return;
+    double c = 0.0;
+    for (long long ch = seg[warp] + lane; ch < seg[warp + 1]; ch += 32) {
+        const double r = z[ch] - zm[ch];
+        c = fma(r, r, c);
+    }
+    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    if (lane == 0) cost[index[warp]] = c;
+}
+
 // per sample v: H[v] = sum over its chains c of J[:, c] J[:, c]^T, g[v] = J r, cost[v] = r^T r;
 // chains of sample v are seg[v] .. seg[v+1]-1 of the canonical order; J is [P][n_chains]
 static __global__ void normal_segments_kernel(int n_vox, int P, long long n_chains, const long long* __restrict__ seg,

@@ -309,6 +309,20 @@ bmc_status bmc_uneven_uses_block_kernel(const void* plan, int32_t* out);
 bmc_status bmc_normal_segments(int32_t n_voxels, int32_t n_params, int64_t n_chains, const int64_t* d_chain_start,
                                const double* d_jz, const double* d_r, double* d_H, double* d_g, double* d_c,
                                void* stream);
+/*
+ * The pieces of a joint trial point around bmc_uneven_simulate, for the voxels of one pool count inside a batch.
+ *   bmc_joint_params: d_out [n_fields][n_voxels] = d_base, with row rows[j] (host array; -1: none) replaced by
+ *     d_x[index[v]][j] * scales[j] (d_x [.][n_local], d_index [n_voxels], scales a host array) and row
+ *     shared_row (-1: none) by d_shared[0] * shared_scale; n_local <= 8.
+ *   bmc_segment_costs: d_cost[index[v]] = sum of (d_z - d_zm)^2 over voxel v's chains, in
+ *     bmc_normal_segments' order (so a point's cost is the same double in both).
+ */
+bmc_status bmc_joint_params(int32_t n_voxels, int32_t n_fields, const double* d_base, const int64_t* d_index,
+                            const double* d_x, int32_t n_local, const int32_t* rows, const double* scales,
+                            int32_t shared_row, double shared_scale, const double* d_shared, double* d_out,
+                            void* stream);
+bmc_status bmc_segment_costs(int32_t n_voxels, const int64_t* d_chain_start, const double* d_z, const double* d_zm,
+                             const int64_t* d_index, double* d_cost, void* stream);
 bmc_status bmc_schur_step(int32_t n_voxels, int32_t n_local, int32_t n_shared, const double* d_H, const double* d_g,
                           const double* d_free, double lam, const double* d_lam, double* d_dx_local,
                           double* d_dx_shared, double* d_work, void* stream);
