@@ -216,8 +216,9 @@ __device__ __forceinline__ HD lift<HD>(const double* x, const double* dir, size_
 // ------------------------------------------------------------------------------------------------
 // event records: the shared event table, preprocessed once per call (bmc_prep_events)
 // ------------------------------------------------------------------------------------------------
-// Event types, BMC-JAX simulation/events.py:12-18.
-enum : int { EV_DELAY = 0, EV_RF = 1, EV_GRADIENT = 2, EV_ADC = 3, EV_SPOILER = 4 };
+// Event types, BMC-JAX simulation/events.py:12-18. A record holds EV_OTHER for a caller's type outside them (such an event
+// evolves by its duration and amplitude and does nothing else); from 8 on a record's type is a mark (kTrainMark).
+enum : int { EV_DELAY = 0, EV_RF = 1, EV_GRADIENT = 2, EV_ADC = 3, EV_SPOILER = 4, EV_OTHER = 5 };
 
 template <typename R>
 struct __align__(16) EvRec {

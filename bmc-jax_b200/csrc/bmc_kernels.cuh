@@ -846,7 +846,7 @@ __global__ void __launch_bounds__(128) cost_kernel(const ChainArgs a, float* __r
     float cost = 0.f;
     for (int e = 0; e < n_ev; ++e) {
         const EvRec<R> rec = ev[(size_t)e * stride + o];
-        if (((int)rec.type & (kTrainMark - 1)) != EV_RF || !(rec.dt > R(1e-9))) continue;
+        if ((int)rec.type != EV_RF || !(rec.dt > R(1e-9))) continue;
         ChainConst<NC, D> cc;
         C::load_const(a, v, 0, cc);
         StepCoef<NC, D> sc;
@@ -974,7 +974,7 @@ __global__ void prep_events_kernel(int n_off, int n_ev, const int32_t* __restric
         r.c = R(c);
         r.s = R(s);
         r.wf = R(6.283185307179586 * freq[i]);
-        r.type = R(type[i]);
+        r.type = R((unsigned)type[i] <= (unsigned)EV_SPOILER ? type[i] : (int)EV_OTHER);
         out[e * n_off + o] = r;
     }
 }
