@@ -19,8 +19,8 @@
 // Loss: mean over the batch and the n_out outputs of (y - t)^2. Optimiser: Adam with bias correction.
 //
 // Every wait is bounded (about two seconds of SM clock); a CTA that gives up sets bit 0 of the status
-// word at the start of the work buffer, waits (bounded) for its MMAs in flight, frees its TMEM and
-// returns.
+// word at the start of the work buffer, waits (bounded; bit 1: in vain) for its MMAs in flight, frees its
+// TMEM and returns.
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
@@ -84,12 +84,21 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
         : "memory");
     return done != 0;
 }
-// wait for the phase of the given parity, for at most ~2^32 SM cycles (about two seconds)
-__device__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+// Wait for the phase of the given parity, for at most ~2^32 SM cycles (about two seconds).
+__device__ bool mbar_drain(uint32_t bar, uint32_t parity) {
     const long long t0 = clock64();
     while (!mbar_try_wait(bar, parity))
         if (clock64() - t0 > (1LL << 32)) return false;
     return true;
+}
+// The waits between the products. A test build sets BMC_MLP_GIVE_UP to 1: they then give up at once, and the CTA goes the
+// way of a CTA whose time ran out. The wait for the products in flight before TMEM is freed (mbar_drain) is the same
+// in every build.
+#ifndef BMC_MLP_GIVE_UP
+#define BMC_MLP_GIVE_UP 0
+#endif
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+    return BMC_MLP_GIVE_UP ? false : mbar_drain(bar, parity);
 }
 __device__ __forceinline__ void fence_barrier_init() {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -387,7 +396,8 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_kernel(GemmArgs g) {
     }
     if (committed >= 0) {
         // the last commit covers every earlier MMA of the CTA
-        const bool w = mbar_wait(smem_addr(&bars[committed % kGemmStages]), (committed / kGemmStages) & 1);
+        const bool w = mbar_drain(smem_addr(&bars[committed % kGemmStages]), (committed / kGemmStages) & 1);
+        if (!w && tid == 0 && g.status) atomicOr(g.status, 2);
         ok = ok && w;
     }
     ok = __syncthreads_and(ok);
@@ -637,6 +647,7 @@ static __global__ void __launch_bounds__(kInferThreads, 2) infer_kernel(const In
 
     bool ok = true;
     uint32_t n0 = 0;                         // the current layer's first chunk
+    long long committed = -1;                // the last chunk whose MMAs were issued
     for (int c = 0; c < min(chunks_of(0), kInferStages); ++c) load(0, c, c);
     for (int tile = blockIdx.x; ok && tile < g.tiles; tile += gridDim.x) {
         const long long m0 = (long long)tile * 128;
@@ -687,6 +698,7 @@ static __global__ void __launch_bounds__(kInferThreads, 2) infer_kernel(const In
                         umma_bf16(tmem, smem_desc(a + j * 256), smem_desc(b + j * 256, 512), idesc_bf16(nn), (c | j) != 0);
                     umma_commit(smem_addr(&bars[n % kInferStages]));
                 }
+                committed = n;
                 if (issued < nk) {           // the stage is free once this chunk's MMAs are done
                     const bool w = mbar_wait(smem_addr(&bars[n % kInferStages]), (n / kInferStages) & 1);
                     ok = __syncthreads_and(w);
@@ -738,7 +750,13 @@ static __global__ void __launch_bounds__(kInferThreads, 2) infer_kernel(const In
         }
     }
     cp_async_wait<0>();
-    if (!ok && tid == 0 && g.status) atomicOr(g.status, 1);
+    if (!ok) {
+        // given up (only behind a commit): the last commit covers the MMAs in flight, which write this CTA's TMEM and
+        // read its shared memory
+        const bool w = mbar_drain(smem_addr(&bars[committed % kInferStages]), (committed / kInferStages) & 1);
+        if (tid == 0 && g.status) atomicOr(g.status, w ? 1 : 3);
+        tc_fence_after();
+    }
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, kInferH);

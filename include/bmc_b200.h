@@ -349,8 +349,9 @@ bmc_status bmc_schur_back(int32_t n_voxels, int32_t n_local, int32_t n_shared, c
  * zero (they then stay zero). The shadow (bf16, `shadow_bytes`) holds W_l and W_l^T per layer, as the
  * tensor cores read them; bmc_mlp_sync rebuilds it from d_params and bmc_mlp_adam_step keeps it current.
  * The work buffer (256-byte aligned, `work_bytes` for a batch size) holds the activations a backward
- * pass needs; its first int32 is a status word: bit 0 is set when a GEMM gave up waiting for its
- * tensor-core operations (about two seconds), and the caller clears it.
+ * pass needs; its first int32 is a status word: bit 0 is set when a kernel gave up waiting for its
+ * tensor-core operations (about two seconds), bit 1 when they were not done two seconds later either;
+ * the caller clears it.
  * Inputs x [batch][n_in] float32 are normalised as (x - d_in_shift[i]) * d_in_scale[i] (either may
  * be NULL); outputs d_y [batch][n_out] float32 (may be NULL). Loss: mean over batch and outputs of
  * (y - target)^2, added to *d_loss (may be NULL); gradients overwrite d_grad.

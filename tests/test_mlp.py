@@ -251,3 +251,38 @@ def test_inference_equals_the_layered_forward(cuda, n_in, n_out, layers, batch):
     assert net.status(batch) == 0
     assert y.shape == (batch, n_out) and bool(torch.isfinite(y).all())
     assert float((y - want).abs().max()) <= 1e-5 * float(want.abs().max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,batch,keep", [(LADDER, 5000, 0), ((270, 256, 2, 6), 40000, 0), (LADDER, 300, 1)])
+def test_a_cta_that_gives_up_waits_for_its_products(cuda, tmp_path_factory, shape, batch, keep):
+    """A build whose waits between the products give up at once: every CTA leaves in the middle of its first tile, with
+    products in flight. The status word says that it gave up (bit 0) and that the products were done when TMEM was freed
+    (bit 1 clear); the GPU and the ordinary build go on as before."""
+    import importlib.util
+    import subprocess
+    from conftest import ROOT
+    torch = cuda
+    spec = importlib.util.spec_from_file_location("bmc_build", ROOT / "bmc-jax_b200" / "build.py")
+    B = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(B)
+    d = tmp_path_factory.getbasetemp() / "give_up"
+    so = d / "libmlp_give_up.so"
+    if not so.exists():
+        d.mkdir(exist_ok=True)
+        (d / "err.cu").write_text('#include "%s"\nnamespace bmc { bmc_status record_error(bmc_status s, const char*) '
+                                  '{ return s; } }\n' % B.HEADER)
+        subprocess.run([B.NVCC, *B.FLAGS, "-DBMC_MLP_GIVE_UP=1", "-shared", "-o", str(so), str(B.SRC / "bmc_mlp.cu"),
+                        str(d / "err.cu")], check=True)
+    F = C.CDLL(str(so)).bmc_mlp_forward
+    F.argtypes, F.restype = _lib.lib().bmc_mlp_forward.argtypes, C.c_int
+    net = _net(shape, seed=11)
+    x = torch.as_tensor(_inputs(shape, batch, 12)[0]).cuda()
+    want = net.forward(x)
+    y, work = torch.empty_like(want), torch.zeros_like(net.work(batch))
+    assert F(C.byref(net.shape), _lib.ptr(net.params), _lib.ptr(net.shadow), _lib.ptr(x), None, None, batch, _lib.ptr(y),
+             _lib.ptr(work), keep, _lib.stream_handle()) == 0
+    torch.cuda.synchronize()
+    assert int(work[:4].view(torch.int32).item()) == 1
+    np.testing.assert_array_equal(net.forward(x).cpu().numpy(), want.cpu().numpy())
+    assert net.status(batch) == 0
