@@ -40,11 +40,14 @@ struct TaylorTable {
 // row has no train.
 struct TrainRow {
     int first, n, gap, run;
-    int span, uses;
+    int span;
     int mirrored;              // the pulse's shape is its own mirror image
     double w_max;
 };
 constexpr int kTrainMark = 8;  // added to the type of a record where a unit begins
+// a chain of a table that was looked over for trains: it has its propagator, its row has no train, or the row has one but
+// the chain is beyond the propagator's bounds (it takes its events one by one)
+constexpr int kTrained = 1, kPlain = 2, kRefused = 4, kEveryPart = 7;
 
 struct ChainArgs {
     int n_vox, n_off, n_ev, n_fields;
@@ -93,10 +96,13 @@ struct ChainArgs {
     int node_lo, node_hi;      // with a null node_out: the nodes of this launch (from 1 on added to the output)
     // Part of the launch order (uniform tables; chain_count 0: all): chains first_chain .. first_chain + chain_count
     long long first_chain, chain_count;
-    // Propagators of those chains' shaped pulses (null: none), applied at the marked records
+    // Shaped pulses (train null: none were looked for): the rows' trains, the propagators of those chains, applied at the
+    // marked records, which of them have one, and the chains that this launch takes (kTrained, kPlain, kRefused)
     const TrainRow* train;     // [n_off]
     const double* prop;
-    const int* prop_ok;
+    const unsigned char* prop_ok;
+    int parts;
+    const int* kinds;          // what the table and the chains so far have of the three (a launch without work ends)
     // adjoint passes: the chains that the thread kernel (bmc_sym.cuh) has taken, and whether it left any
     unsigned char* done;       // [n_vox * n_off] or null
     int* left;

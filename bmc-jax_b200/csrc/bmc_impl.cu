@@ -195,29 +195,45 @@ template <int NC>
 constexpr int tangents_per_pass() { return NC <= 1 ? 2 : 1; }
 
 // Shaped-pulse trains of a call: the rows' units and amplitudes, and the propagators (with those of `tangents`
-// derivatives) of `chunk` chains at a time: kTrainChunk, or what the call has if that is less (300 MB with four pools).
-constexpr long long kTrainChunk = 131072;
+// derivatives) of `chunk` chains at a time: whole waves of the chain kernel that applies them, as many as kTrainBytes
+// hold and at least one (131 MB with four pools, 173 with five; 175 and 230 with a tangent), or waves of train_kernel's
+// warps where fewer fit. A call of at most a chunk takes every chain in one launch. A larger one takes, chunk by chunk, the
+// chains that have a propagator, and all others (rows without a train, chains whose propagator is refused) in launches over
+// the whole order, for chunk by chunk each launch ends in a partly empty wave. 16,384 voxels x 101 rows, everything in
+// chunks of 131,072 / now: 64 pulses without a train, four pools 19.6 / 17.3 ms; 20 block pulses, four pools 83 / 72; ten,
+// five pools, in bmc_simulate_noalloc's static scratch (11,000 chains a chunk) 321 / 103. 4,096 voxels x 101 rows of 20
+// shaped pulses: 28.6 / 28.6.
+constexpr size_t kTrainBytes = size_t(160) << 20;
+constexpr long long kTrainWindow = 1ll << 22;        // chains whose flags are kept at once
 template <int NC>
 struct Trains {
     int max_samples = 0, mats = 1;
-    long long chunk = 0;
+    long long chunk = 0, window = 0;
     TrainArgs tr{};
     const TaylorTable* tt64 = nullptr;   // the float64 table, which the propagators are formed with
 
-    // tables too short for two pulses have no trains
-    static bool wanted(const bmc_problem* pr) { return pr->n_events >= 2 * kTrainMinSamples; }
+    // tables too short for the pulses' least uses have no trains
+    static bool wanted(const bmc_problem* pr) { return pr->n_events >= train_min_uses<NC>() * kTrainMinSamples; }
 
-    size_t per_chain() const { return sizeof(double) * mats * TrainShape<NC>::N * TrainShape<NC>::NS + sizeof(int); }
+    size_t per_chain() const { return sizeof(double) * mats * TrainShape<NC>::N * TrainShape<NC>::NS; }
     size_t fixed_bytes(const bmc_problem* pr, int tangents) {
         max_samples = std::min(pr->n_events, kTrainMaxSamples);
         mats = 1 + tangents;
         return align256(sizeof(TrainRow) * pr->n_offsets) +
-               align256(sizeof(double) * (size_t)max_samples * pr->n_offsets) + 512;
+               align256(sizeof(double) * (size_t)max_samples * pr->n_offsets) + 1024;
     }
-    size_t bytes(const bmc_problem* pr, long long chains, int tangents) {
+    // the scratch for `chains` chains, the propagators (and the chains' flags) in at most `most` bytes
+    size_t bytes(const bmc_problem* pr, long long chains, int tangents, size_t most = ~size_t(0) >> 1) {
         const size_t fixed = fixed_bytes(pr, tangents);
-        chunk = std::min(chains, kTrainChunk / mats);
-        return fixed + (size_t)chunk * per_chain();
+        window = std::min(chains, kTrainWindow);
+        // a wave of the chain kernel, more of them up to kTrainBytes; where not one fits, waves of train_kernel's warps
+        const long long full = 128ll * kSMs * (tangents ? ChainLaunch<NC, 1>::kMinBlocks : ChainLaunch<NC, 0>::kMinBlocks);
+        constexpr long long wave = (long long)TrainShape<NC>::warps(0) * TrainShape<NC>::blocks(0) * kSMs;
+        const long long fit = (long long)((most - align256(window)) / per_chain());
+        chunk = std::max<long long>(1, kTrainBytes / (full * per_chain())) * full;
+        if (chunk > fit) chunk = fit >= full ? fit - fit % full : (fit >= wave ? fit - fit % wave : fit);
+        chunk = std::min(chunk, window);
+        return fixed + align256(chunk * per_chain()) + align256(window);
     }
     // carves the scratch, finds the rows' trains and marks the records `rec` (a.ev's)
     bmc_status scan(ChainArgs& a, EvRec<double>* rec, Carve& cv, cudaStream_t st) {
@@ -225,20 +241,22 @@ struct Trains {
         double* rho = cv.take<double>((size_t)max_samples * a.n_off);
         tr.rho = rho;
         tr.max_samples = max_samples;
-        tr.prop = cv.take<double>((size_t)chunk * mats * TrainShape<NC>::N * TrainShape<NC>::NS);
-        tr.ok = cv.take<int>(chunk);
-        train_scan_kernel<<<a.n_off, kTrainScanThreads, 0, st>>>(rec, a.n_ev, a.n_off, train_min_uses<NC>(),
-                                                                 const_cast<int4*>(a.seg), rows, rho, max_samples);
+        tr.prop = cv.take<double>((size_t)chunk * per_chain() / sizeof(double));
+        tr.ok = cv.take<unsigned char>(window);
+        tr.kinds = cv.take<int>(1);
+        CUDA_TRY(cudaMemsetAsync(tr.kinds, 0, sizeof(int), st));
+        train_scan_kernel<<<a.n_off, kTrainScanThreads, 0, st>>>(rec, a.n_ev, a.n_off, train_min_uses<NC>(), a.seg, rows,
+                                                                 rho, max_samples, tr.kinds);
         CUDA_TRY(cudaGetLastError());
         a.train = rows;
         a.prop = tr.prop;
-        a.prop_ok = tr.ok;
+        a.kinds = tr.kinds;
         return BMC_OK;
     }
 
     template <int DT>
-    bmc_status form(const ChainArgs& a, int tangents, cudaStream_t st) const {
-        constexpr int kWarps = TrainShape<NC>::kWarps;
+    bmc_status form(const ChainArgs& a, unsigned char* ok, int tangents, cudaStream_t st) const {
+        constexpr int kWarps = TrainShape<NC>::warps(DT);
         const size_t smem = kWarps * sizeof(TrainSmem<NC, DT>);
         static std::atomic<unsigned long long> configured{0};
         int dev = 0;
@@ -251,26 +269,56 @@ struct Trains {
         if (bmc_status s = host_table_of(tt64, &th); s != BMC_OK) return s;
         TrainArgs t = tr;
         t.mats = 1 + tangents;
+        t.ok = ok;
         const dim3 grid((unsigned)((a.chain_count + kWarps - 1) / kWarps), DT ? tangents : 1);
         train_kernel<NC, DT><<<grid, 32 * kWarps, smem, st>>>(a, t, th);
         CUDA_TRY(cudaGetLastError());
         return BMC_OK;
     }
 
-    // One pass over every chain with NT tangents: per chunk of the launch order (and per node, where the nodes do not
-    // run as chains of their own) the propagators, then the chains.
+    // One pass over every chain with NT tangents. Per node where the nodes do not run as chains of their own: a chain's
+    // nodes are added in their order.
     template <int NT>
     bmc_status pass(ChainArgs a, const TaylorTable* tt, cudaStream_t st) const {
         const long long all = (long long)a.n_vox * a.n_off * (a.node_out ? a.n_nodes : 1);
-        for (a.first_chain = 0; a.first_chain < all; a.first_chain += chunk) {
-            a.chain_count = std::min(chunk, all - a.first_chain);
-            for (int j = 0; j < (a.node_out ? 1 : a.n_nodes); ++j) {
-                if (!a.node_out) {
-                    a.node_lo = j;
-                    a.node_hi = j + 1;
+        const int nodes = a.node_out ? 1 : a.n_nodes;
+        bmc_status s = BMC_OK;
+        auto of_node = [&](int j) {
+            if (a.node_out) return;
+            a.node_lo = j;
+            a.node_hi = j + 1;
+        };
+        if (all <= chunk) {
+            a.parts = kEveryPart;
+            a.prop_ok = tr.ok;
+            a.chain_count = all;
+            for (int j = 0; j < nodes; ++j) {
+                of_node(j);
+                if ((s = form<(NT > 0 ? 1 : 0)>(a, tr.ok, NT, st)) != BMC_OK || (s = launch_chain<NC, double, NT>(a, tt, st)) != BMC_OK)
+                    return s;
+            }
+            return BMC_OK;
+        }
+        // the rows without a train: all nodes of a chain in one launch, or (one node) beside the refused chains
+        a.parts = kPlain;
+        if (nodes > 1 && (s = launch_chain<NC, double, NT>(a, tt, st)) != BMC_OK) return s;
+        for (long long lo = 0; lo < all; lo += window) {
+            const long long end = std::min(all, lo + window);
+            for (int j = 0; j < nodes; ++j) {
+                of_node(j);
+                a.parts = kTrained;
+                for (a.first_chain = lo; a.first_chain < end; a.first_chain += chunk) {
+                    a.chain_count = std::min(chunk, end - a.first_chain);
+                    unsigned char* ok = tr.ok + (a.first_chain - lo);
+                    a.prop_ok = ok;
+                    if ((s = form<(NT > 0 ? 1 : 0)>(a, ok, NT, st)) != BMC_OK || (s = launch_chain<NC, double, NT>(a, tt, st)) != BMC_OK)
+                        return s;
                 }
-                bmc_status s = form<(NT > 0 ? 1 : 0)>(a, NT, st);
-                if (s != BMC_OK || (s = launch_chain<NC, double, NT>(a, tt, st)) != BMC_OK) return s;
+                a.parts = kRefused | (nodes > 1 ? 0 : kPlain);
+                a.first_chain = lo;
+                a.chain_count = end - lo;
+                a.prop_ok = tr.ok;
+                if ((s = launch_chain<NC, double, NT>(a, tt, st)) != BMC_OK) return s;
             }
         }
         return BMC_OK;
@@ -382,9 +430,9 @@ bmc_status Impl<NC>::simulate(const bmc_problem* pr, const double* params, const
     Trains<NC> tn;
     // the counting calls integrate event by event: their counts are the work of that
     const bool trains = pr->precision != BMC_F32 && !work && Trains<NC>::wanted(pr);
-    if ((s = workspace(align256(nrec * recb) + 256 + align256(sizeof(int4) * pr->n_offsets) + order_bytes(nch) +
-                           align256(part * sizeof(double)) +
-                           (trains ? tn.bytes(pr, split ? nch * sp->n_nodes : nch, 0) : 0), st, &ws)) != BMC_OK)
+    const size_t least = align256(nrec * recb) + 256 + align256(sizeof(int4) * pr->n_offsets) + order_bytes(nch);
+    const size_t nodes = least + align256(part * sizeof(double));
+    if ((s = workspace(nodes + (trains ? tn.bytes(pr, split ? nch * sp->n_nodes : nch, 0) : 0), st, &ws)) != BMC_OK)
         return s;
     Carve cv(ws);
     ChainArgs a{};
@@ -452,12 +500,12 @@ bmc_status Impl<NC>::jvp(const bmc_problem* pr, const double* params, const bmc_
     const bool split = split_nodes(nch, sp, per_node);
     const size_t part = split ? (size_t)nch * sp->n_nodes : 0;
     Trains<NC> tn;
-    const bool trains = !work && Trains<NC>::wanted(pr);         // counting calls: event by event
+    const bool trains = !work && Trains<NC>::wanted(pr);               // counting calls: event by event
     const size_t train_bytes = trains ? tn.bytes(pr, split ? nch * sp->n_nodes : nch, tangents_per_pass<NC>()) : 0;
-    if ((s = workspace(align256(nrec * sizeof(EvRec<double>)) + 256 + align256(sizeof(int4) * pr->n_offsets) +
-                           align256(sizeof(int) * pr->n_offsets) + 1024 + order_bytes(nch) + align256(nch) +
-                           align256(part * (1 + tg->n_tangents) * sizeof(double)) + train_bytes, st, &ws)) != BMC_OK)
-        return s;
+    const size_t least = align256(nrec * sizeof(EvRec<double>)) + 256 + align256(sizeof(int4) * pr->n_offsets) +
+                         align256(sizeof(int) * pr->n_offsets) + 1024 + order_bytes(nch) + align256(nch);
+    const size_t nodes = least + align256(part * (1 + tg->n_tangents) * sizeof(double)) + 512;
+    if ((s = workspace(nodes + train_bytes, st, &ws)) != BMC_OK) return s;
     Carve cv(ws);
     ChainArgs a{};
     a.n_vox = pr->n_voxels; a.n_off = pr->n_offsets; a.n_ev = pr->n_events; a.n_fields = Layout<NC>::NF;
@@ -561,18 +609,19 @@ bmc_status Impl<NC>::lm(const bmc_problem* pr, const double* params, const bmc_e
     const size_t part = split ? (size_t)nv * no * sp->n_nodes : 0;
     Trains<NC> tn;
     const bool trains = Trains<NC>::wanted(pr);
-    const size_t bytes = align256(nrec * sizeof(EvRec<double>)) + 2 * align256(sizeof(double) * NF * nv) +
+    const size_t least = align256(nrec * sizeof(EvRec<double>)) + 2 * align256(sizeof(double) * NF * nv) +
                          2 * align256(sizeof(double) * N * nv) + 2 * align256(sizeof(double) * nv) +
                          align256(sizeof(double) * P * nv) + align256(sizeof(double) * P * nv * N) +
                          2 * align256(sizeof(double) * nv * no) + align256(sizeof(double) * P * nv * no) +
                          2 * align256(sizeof(double) * nv * P) + 2 * align256(sizeof(double) * nv) +
                          align256(sizeof(int) * nv) + align256(sizeof(int4) * no) + 4096 +
                          align256(sizeof(int) * no) + 1024 + order_bytes((long long)nv * no) + align256((size_t)nv * no) +
-                         live_bytes((long long)nv * no) +
-                         align256(part * (1 + P) * sizeof(double)) +
-                         (trains ? tn.bytes(pr, (long long)nv * no * (split ? sp->n_nodes : 1), tangents_per_pass<NC>()) : 0);
+                         live_bytes((long long)nv * no);
+    const size_t nodes = least + align256(part * (1 + P) * sizeof(double)) + 512;
     void* ws = nullptr;
-    if ((s = workspace(bytes, st, &ws)) != BMC_OK) return s;
+    if ((s = workspace(nodes + (trains ? tn.bytes(pr, (long long)nv * no * (split ? sp->n_nodes : 1), tangents_per_pass<NC>())
+                                       : 0), st, &ws)) != BMC_OK)
+        return s;
     Carve cv(ws);
     EvRec<double>* rec = cv.take<EvRec<double>>(nrec);
     double* px = cv.take<double>((size_t)NF * nv);
@@ -703,9 +752,7 @@ bmc_status run_noalloc(const bmc_problem* pr, const double* params, const bmc_ev
         Trains<NC> tn;
         if (Trains<NC>::wanted(pr)) {
             // as many chains at a time as the static array holds (its size covers every table's amplitudes)
-            const size_t fixed = tn.fixed_bytes(pr, 0);
-            tn.chunk = std::min<long long>((long long)pr->n_voxels * pr->n_offsets,
-                                           (long long)((ws.train_bytes - fixed) / tn.per_chain()));
+            tn.bytes(pr, (long long)pr->n_voxels * pr->n_offsets, 0, ws.train_bytes - tn.fixed_bytes(pr, 0));
             tn.tt64 = ws.tt64;
             Carve cv(ws.train);
             if ((s = tn.scan(a, rec, cv, st)) != BMC_OK) return s;

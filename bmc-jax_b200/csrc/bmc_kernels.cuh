@@ -462,9 +462,13 @@ struct TrainShape {
     static constexpr int TS = 8 * NT * LD;                   // doubles of one matrix
     static constexpr int kSlots = 6;
     static constexpr int NS = (N + 2) & ~1;                  // row of the stored propagator: N entries, phi, padding
-    // warps per block: the shared memory of a warp (19 KB with four pools) sets the resident warps, so small blocks
-    static constexpr int kWarps = NT == 1 ? 4 : 1;
-    static constexpr int kBlocks = NT == 1 ? 4 : (NT == 2 ? 8 : 4);   // resident blocks the registers are kept for
+    // Warps per block and the resident blocks that the registers are kept for, without and with a tangent. The shared memory
+    // of a warp (19 KB with four pools, twice that with a tangent) sets the resident warps. 20 pulses of 100 samples x 101
+    // rows: 4,096 voxels of four pools 28.6 ms with 4 warps x 2 blocks, 28.9 with 1 x 8 (and a fifth of the time where the
+    // blocks of a table without trains only start and end); 2,048 of five pools 34.3 with 1 x 4, 37.3 with 2 x 2, whose
+    // registers spill; 1,300 of four pools with two tangents 72.0 with one warp a block, 90.8 with four.
+    static constexpr int warps(int tangents) { return NT == 1 || (NT == 2 && !tangents) ? 4 : 1; }
+    static constexpr int blocks(int tangents) { return tangents ? 1 : (NT == 2 ? 2 : 4); }
 };
 
 // M <- R(phase) [P R(-phase) M + phi], P from the propagator `p` (the turned frame's x is along the RF); with tangents
@@ -542,6 +546,11 @@ chain_kernel(const ChainArgs a, const __grid_constant__ TaylorTable tt) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31;
     SM* dsm = reinterpret_cast<SM*>(smem_raw) + (threadIdx.x >> 5);
+    // tables that were looked over for trains
+    constexpr bool kTrain = !UNEVEN && !COUNT && std::is_same<R, double>::value;
+    if constexpr (kTrain) {
+        if (a.train && a.parts != kEveryPart && !(*a.kinds & a.parts)) return;
+    }
 
     // chains in offset-fastest order: neighbouring lanes are neighbouring offsets of one voxel, so a
     // warp shares parameters and its chains need similar Taylor orders
@@ -581,15 +590,20 @@ chain_kernel(const ChainArgs a, const __grid_constant__ TaylorTable tt) {
     if constexpr (std::is_same<R, RD>::value) {
         if (a.seg && !a.traj) blk = a.seg[seg_row];
     }
-    const bool use_blk = blk.z >= 2;
+    bool act = valid && (a.active == nullptr || a.active[v] != 0);
+    bool train = false;                                // the chain has its propagator
+    if constexpr (kTrain) {
+        if (a.train && act) {
+            // (a launch of the plain rows alone has no prop_ok)
+            const int kind = a.train[o].n == 0 ? kPlain : (a.parts != kPlain && a.prop_ok[pos] ? kTrained : kRefused);
+            act = (kind & a.parts) != 0;
+            train = act && kind == kTrained;
+        }
+    }
+    if (__all_sync(kFull, !act)) return;
+    const bool use_blk = blk.z >= 2 && !train;
     const R dswitch = R(a.dense_switch > 0.0 ? a.dense_switch : tt.dense_switch);
     const int blk_end = use_blk ? blk.x + blk.z * blk.y : 0;
-    const bool act = valid && (a.active == nullptr || a.active[v] != 0);
-    if (__all_sync(kFull, !act)) return;
-    // the chain's shaped pulses have a propagator (float64 kernels)
-    constexpr bool kTrain = !UNEVEN && !COUNT && std::is_same<R, double>::value;
-    bool train = false;
-    if constexpr (kTrain) train = a.prop && act && a.train[o].n > 0 && a.prop_ok[pos] != 0;
 
     const size_t ch = UNEVEN ? (size_t)ci : (size_t)v * a.n_off + o;
     unsigned wk0 = 0, wk1 = 0, wk2 = 0, wk3 = 0, wk4 = 0;   // this chain's work counts (each < 2^32 per launch)
@@ -637,10 +651,9 @@ chain_kernel(const ChainArgs a, const __grid_constant__ TaylorTable tt) {
                                             count, wk0, wk1, wk2);
             }
             // a shaped pulse: its propagator at its first event; the warp goes on at the next event any lane needs
-            int type = (int)rec.type;
+            int type = (int)rec.type;                  // (a marked record's, 8 more: an RF event's, which does nothing below)
             if constexpr (kTrain) {
                 const bool tstart = train && (type & kTrainMark) != 0 && e >= train_end;
-                type &= kTrainMark - 1;
                 if (tstart) {
                     State<NC, D> Mt = M;
                     train_apply<NC, NT>(a.prop + (size_t)pos * (1 + NT) * N * TrainShape<NC>::NS, rec.c, rec.s, Mt);

@@ -45,7 +45,8 @@ struct TrainArgs {
     int max_samples;
     double* prop;              // [chains of the launch][mats][N][NS]: P's rows, phi last, then the derivatives'
     int mats;                  // 1 + the launch's tangents
-    int* ok;                   // [chains of the launch]: the propagator was formed
+    unsigned char* ok;         // [chains of the launch]: the propagator was formed
+    int* kinds;                // kTrained and kPlain by the rows, kRefused by the chains (ChainArgs::kinds)
 };
 
 // Uses of a pulse from which its propagator pays, by pool count. One sample costs the propagator 2 NT^3 matrix
@@ -73,17 +74,18 @@ constexpr int kTrainScanThreads = 256;
 
 // Finds each row's pulses (runs of RF events of one duration, frequency and phase), takes the middle one as the
 // reference, and keeps those with its samples; marks the units' first records and writes the reference pulse's
-// relative amplitudes. A row whose repeated block (seg) saves more events keeps that instead, else the block is dropped.
+// relative amplitudes. A row whose repeated block (seg) saves more events has no train; a row with one keeps its
+// block for the chains that have no propagator.
 static __global__ void __launch_bounds__(kTrainScanThreads)
-train_scan_kernel(EvRec<double>* __restrict__ ev, int n_ev, int stride, int min_uses, int4* __restrict__ seg,
-                  TrainRow* __restrict__ rows, double* __restrict__ rho, int max_samples) {
+train_scan_kernel(EvRec<double>* __restrict__ ev, int n_ev, int stride, int min_uses, const int4* __restrict__ seg,
+                  TrainRow* __restrict__ rows, double* __restrict__ rho, int max_samples, int* __restrict__ kinds) {
     __shared__ int starts[kTrainMaxPulses], ends[kTrainMaxPulses];
     __shared__ unsigned char match[kTrainMaxPulses];
     __shared__ int n_start, n_end, warp_n[kTrainScanThreads / 32][2], flags[3];
     __shared__ double wmax_s;
     EvRec<double>* row = ev + blockIdx.x;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    TrainRow out{0, 0, 0, 0, 0, 0, 0, 0.0};
+    TrainRow out{0, 0, 0, 0, 0, 0, 0.0};
     if (tid == 0) n_start = n_end = 0;
     __syncthreads();
     auto is_rf = [&](const EvRec<double>& r) { return (int)r.type == EV_RF && r.dt > 1e-9; };
@@ -192,9 +194,7 @@ train_scan_kernel(EvRec<double>* __restrict__ ev, int n_ev, int stride, int min_
             const long long block_saves = blk.z >= 2 ? (long long)(blk.z - 1) * blk.y : 0;
             const double wm = wmax_s;
             if (uses >= min_uses && wm > 0.0 && wm < INFINITY && (long long)(uses - 1) * n > block_saves) {
-                out = TrainRow{r0, n, gap, run, run * unit, uses, flags[2], wm};
-                __syncthreads();
-                if (tid == 0) seg[blockIdx.x] = make_int4(0, 0, 0, 0);
+                out = TrainRow{r0, n, gap, run, run * unit, flags[2], wm};
                 for (int p = tid; p < np; p += kTrainScanThreads)
                     if (match[p] && (run == 1 || p == first_match)) {
                         EvRec<double>& m = row[(size_t)starts[p] * stride];
@@ -205,7 +205,10 @@ train_scan_kernel(EvRec<double>* __restrict__ ev, int n_ev, int stride, int min_
             }
         }
     }
-    if (tid == 0) rows[blockIdx.x] = out;
+    if (tid == 0) {
+        rows[blockIdx.x] = out;
+        atomicOr(kinds, out.n > 0 ? kTrained : kPlain);
+    }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -762,7 +765,7 @@ struct Train {
 // blocks write the values too). One tangent costs three times a propagator; the Taylor action of every event with dual
 // numbers took 12.6 ms for the three tangents of 714 chains (one pool, 10 pulses of 100 samples), this 0.53 ms.
 template <int NC, int DT>
-__global__ void __launch_bounds__(32 * TrainShape<NC>::kWarps, DT == 0 ? TrainShape<NC>::kBlocks : 1)
+__global__ void __launch_bounds__(32 * TrainShape<NC>::warps(DT), TrainShape<NC>::blocks(DT))
 train_kernel(const ChainArgs a, const TrainArgs tr, const __grid_constant__ TaylorTable tt) {
     using TR = Train<NC, DT>;
     using SH = TrainShape<NC>;
@@ -772,8 +775,8 @@ train_kernel(const ChainArgs a, const TrainArgs tr, const __grid_constant__ Tayl
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     TrainSmem<NC, DT>* sm = reinterpret_cast<TrainSmem<NC, DT>*>(smem_raw) + warp;
-    const long long pos = (long long)blockIdx.x * SH::kWarps + warp;
-    if (pos >= a.chain_count) return;
+    const long long pos = (long long)blockIdx.x * SH::warps(DT) + warp;
+    if (pos >= a.chain_count || !(*tr.kinds & kTrained)) return;
     const long long nch = (long long)a.n_vox * a.n_off;
     long long ci = a.first_chain + pos;
     const int node = a.node_out ? (int)(ci / nch) : a.node_lo;
@@ -793,7 +796,6 @@ train_kernel(const ChainArgs a, const TrainArgs tr, const __grid_constant__ Tayl
     typename TR::Run r;
     TR::identity(r, lane);
     bool ok = true;
-
     if (ok) {
         // the pulse's matrix function at its nodes
         EvRec<double> rec = ev[(size_t)row.first * a.n_off];
@@ -939,7 +941,10 @@ train_kernel(const ChainArgs a, const TrainArgs tr, const __grid_constant__ Tayl
             }
         }
     }
-    if (lane == 0 && blockIdx.y == 0) tr.ok[pos] = ok ? 1 : 0;
+    if (lane == 0 && blockIdx.y == 0) {
+        tr.ok[pos] = ok ? 1 : 0;
+        if (!ok) atomicOr(tr.kinds, kRefused);
+    }
 }
 
 }  // namespace bmc

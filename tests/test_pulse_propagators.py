@@ -271,6 +271,67 @@ def test_non_finite_and_extreme_parameters_stay_with_their_voxel(cuda):
     _close(z[keep], np.ascontiguousarray(P[:, keep]), M0[keep], ev, nc)
 
 
+MIXED_ROWS = [("phases", {}), ("plain", {}), ("beyond_the_bound", {}), ("own_delays", {}), ("blocks", {}), ("mirrored_even", {}),
+              ("few", dict(pulses=1))]
+
+
+def _mixed_table():
+    """Rows with a train, without one (pulses of samples of their own; a repeated block), and with one that chains refuse."""
+    rows = []
+    for f, (k, kw) in zip(OFFSETS, MIXED_ROWS):
+        if k == "plain":
+            rows.append([(1, 0.001 * (1 + 0.1 * j), 30.0 + j, 0.2 * j, f) for j in range(9)] + [(4, 0.0, 0.0, 0.0, 0.0),
+                        (0, 0.5, 0.0, 0.0, 0.0), (3, 0.0, 0.0, 0.0, 0.0)])
+        elif k == "blocks":
+            rows.append([(1, 0.05, 40.0, 0.0, f), (0, 0.005, 0.0, 0.0, 0.0)] * 10 + [(3, 0.0, 0.0, 0.0, 0.0)])
+        else:
+            rows.append(_row(f, **{**dict(samples=12, pulses=9), **FORMS.get(k, {}), **kw}))
+    return _table(rows)
+
+
+def _tiled(a, n):
+    return np.ascontiguousarray(np.resize(a.T, (n, a.shape[0])).T)
+
+
+# more chains than one chunk of propagators holds (of bmc_simulate 170,496 with two pools, 56,832 with five; with tangents
+# 37,888 from four pools on, 113,664 with one; of bmc_simulate_noalloc 10,656 with five) and than one window of flags
+# (4,194,304), an odd rest each
+@pytest.mark.gpu
+@pytest.mark.parametrize("nc,n,entry,nodes", [
+    (5, 8203, "bmc_simulate", 1), (5, 2003, "bmc_simulate_noalloc", 1), (5, 2003, "bmc_simulate_noalloc", 3),
+    (5, 3001, "bmc_simulate", 3), (2, 24999, "bmc_simulate", 2), (0, 600701, "bmc_simulate", 1),
+    (0, 600701, "bmc_simulate_noalloc", 1)])
+def test_chunks_of_propagators_give_the_bits_of_one(cuda, nc, n, entry, nodes):
+    """A batch of 61 voxels over and over: every voxel gives what the 61 give, which is the oracle's result."""
+    P, M0 = _voxels(61, nc, seed=37)
+    ev = _mixed_table()
+    spread = None if nodes == 1 else (np.linspace(-1.0, 1.3, nodes), np.arange(1, nodes + 1) / (nodes * (nodes + 1) / 2), 7.0)
+    one = _simulate(cuda, P, M0, ev, nc, spread=spread)
+    many = _simulate(cuda, _tiled(P, n), np.resize(M0, (n, M0.shape[1])), ev, nc, spread=spread, entry=entry)
+    np.testing.assert_array_equal(many, np.resize(one, many.shape))
+    if nodes == 1:
+        _close(one[:2], np.ascontiguousarray(P[:, :2]), M0[:2], ev, nc)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nc,n,T,nodes", [(4, 5501, 3, 1), (1, 17003, 3, 1), (4, 5501, 1, 2), (5, 2801, 1, 3)])
+def test_chunks_of_propagators_with_tangents_give_the_bits_of_one(cuda, nc, n, T, nodes):
+    P, M0 = _voxels(59, nc, seed=41)
+    ev = _mixed_table()
+    spread = None if nodes == 1 else (np.linspace(-1.0, 1.3, nodes), np.arange(1, nodes + 1) / (nodes * (nodes + 1) / 2), 7.0)
+    rows = [3, 3 + nc, 1][:T]
+    seeds = P[rows] * 1.0
+    z1, j1 = _jvp(cuda, P, M0, ev, nc, rows, seeds, spread=spread)
+    z, j = _jvp(cuda, _tiled(P, n), np.resize(M0, (n, M0.shape[1])), ev, nc, rows, _tiled(seeds, n), spread=spread)
+    np.testing.assert_array_equal(z, np.resize(z1, z.shape))
+    for t in range(T):
+        np.testing.assert_array_equal(j[t], np.resize(j1[t], j[t].shape))
+    zc, jc = _jvp(cuda, P, M0, ev, nc, rows, seeds, spread=spread, counted=True)
+    assert np.abs(z1 - zc).max() < 1e-11
+    for t in range(T):
+        assert np.abs(j1[t] - jc[t]).max() <= 1e-9 * np.abs(jc[t]).max()
+
+
 def _bound(n, theta, x):
     from math import factorial as f
     return 2.0 / 4 ** n * sum(theta ** (2 * j) / f(2 * j) * x ** (n - j) / f(n - j) for j in range(n + 1))
