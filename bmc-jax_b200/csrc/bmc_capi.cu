@@ -12,6 +12,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <map>
 #include <mutex>
 #include <string>
@@ -183,29 +184,43 @@ bmc_status tables(int precision, const TaylorTable** out) {
 // is released by cudaFreeAsync on the same stream (after the work already queued there that uses it) and
 // the new one taken by cudaMallocAsync, so growing never synchronises the device. A call that grows the
 // workspace allocates (it is not capturable in a CUDA graph); later calls of the same or a smaller size
-// only enqueue kernels.
-bmc_status workspace(size_t bytes, cudaStream_t st, void** out) {
+// only enqueue kernels. `sizes`: what the call would like, then what it can do with less (the propagators of shaped
+// pulses and the isochromats as chains of their own are scratch for speed: a call that cannot have it, on a full GPU
+// or in a capture, runs without).
+bmc_status workspace(std::initializer_list<size_t> sizes, cudaStream_t st, void** out, int* taken) {
     int dev = 0;
     CUDA_TRY(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lk(g_mu);
     Workspace& w = g_ws[{dev, st}];
-    if (w.bytes < bytes) {
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        CUDA_TRY(cudaStreamIsCapturing(st, &cs));
-        if (cs != cudaStreamCaptureStatusNone)
-            return fail(BMC_ERR_INVALID, "this call needs %zu workspace bytes on a stream that is being captured and "
-                        "has %zu: make one call of this size on the same stream before capturing", bytes, w.bytes);
-        if (w.ptr) {
-            CUDA_TRY(cudaFreeAsync(w.ptr, st));
-            w.ptr = nullptr;
-            w.bytes = 0;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (w.bytes < *sizes.begin()) CUDA_TRY(cudaStreamIsCapturing(st, &cs));
+    cudaError_t e = cudaSuccess;
+    *taken = 0;
+    for (const size_t bytes : sizes) {
+        if (w.bytes < bytes && cs == cudaStreamCaptureStatusNone) {
+            if (w.ptr) {
+                CUDA_TRY(cudaFreeAsync(w.ptr, st));
+                w.ptr = nullptr;
+                w.bytes = 0;
+            }
+            const size_t want = bytes + bytes / 4 + (1 << 20);
+            e = cudaMallocAsync(&w.ptr, want, st);
+            if (e == cudaSuccess) w.bytes = want;
+            else w.ptr = nullptr;
+            if (e == cudaErrorMemoryAllocation) cudaGetLastError();      // not left for the next check
+            else if (e != cudaSuccess) break;
         }
-        const size_t want = bytes + bytes / 4 + (1 << 20);
-        CUDA_TRY(cudaMallocAsync(&w.ptr, want, st));
-        w.bytes = want;
+        if (w.bytes >= bytes) {
+            *out = w.ptr;
+            return BMC_OK;
+        }
+        ++*taken;
     }
-    *out = w.ptr;
-    return BMC_OK;
+    const size_t least = sizes.begin()[sizes.size() - 1];
+    if (cs != cudaStreamCaptureStatusNone)
+        return fail(BMC_ERR_INVALID, "this call needs %zu workspace bytes on a stream that is being captured and "
+                    "has %zu: make one call of this size on the same stream before capturing", least, w.bytes);
+    return fail(BMC_ERR_CUDA, "workspace of %zu bytes: %s", least, cudaGetErrorString(e));
 }
 
 bmc_status check_problem(const bmc_problem* pr, const double* params, const bmc_events* ev, const double* m0) {

@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstddef>
+#include <initializer_list>
 
 #include "../../include/bmc_b200.h"
 
@@ -28,7 +29,12 @@ bmc_status fail(bmc_status s, const char* fmt, ...);
 constexpr int kTableFit = 3, kTables = 4;
 bmc_status tables(int precision, const TaylorTable** out);
 bmc_status host_table_of(const TaylorTable* tt, TaylorTable* out);
-bmc_status workspace(size_t bytes, cudaStream_t st, void** out);
+// the first of the sizes (each at most the one before) that the stream's workspace has or can be grown to; *taken: which
+bmc_status workspace(std::initializer_list<size_t> sizes, cudaStream_t st, void** out, int* taken);
+inline bmc_status workspace(size_t bytes, cudaStream_t st, void** out) {
+    int taken;
+    return workspace({bytes}, st, out, &taken);
+}
 bmc_status fill_spread(ChainArgs& a, const bmc_spread* sp);
 bmc_status scan_blocks(const EvRec<double>* rec, int n_rows, int n_ev, int stride, int4* seg, cudaStream_t st);
 bmc_status use_adjoint(const EvRec<double>* rec, const bmc_problem* pr, int n_tan, int* row_ev, int* flag,

@@ -425,15 +425,19 @@ bmc_status Impl<NC>::simulate(const bmc_problem* pr, const double* params, const
     const size_t recb = pr->precision == BMC_F32 ? sizeof(EvRec<float>) : sizeof(EvRec<double>);
     const long long nch = (long long)pr->n_voxels * pr->n_offsets;
     const size_t per_node = (size_t)nch * (pr->mz_loc >= 0 ? 1 : Layout<NC>::N);
-    const bool split = split_nodes(nch, sp, per_node);
+    bool split = split_nodes(nch, sp, per_node);
     const size_t part = split ? per_node * sp->n_nodes : 0;
     Trains<NC> tn;
     // the counting calls integrate event by event: their counts are the work of that
-    const bool trains = pr->precision != BMC_F32 && !work && Trains<NC>::wanted(pr);
+    bool trains = pr->precision != BMC_F32 && !work && Trains<NC>::wanted(pr);
     const size_t least = align256(nrec * recb) + 256 + align256(sizeof(int4) * pr->n_offsets) + order_bytes(nch);
     const size_t nodes = least + align256(part * sizeof(double));
-    if ((s = workspace(nodes + (trains ? tn.bytes(pr, split ? nch * sp->n_nodes : nch, 0) : 0), st, &ws)) != BMC_OK)
+    int taken = 0;
+    if ((s = workspace({nodes + (trains ? tn.bytes(pr, split ? nch * sp->n_nodes : nch, 0) : 0), nodes, least}, st, &ws,
+                       &taken)) != BMC_OK)
         return s;
+    trains = trains && taken < 1;
+    split = split && taken < 2;
     Carve cv(ws);
     ChainArgs a{};
     a.n_vox = pr->n_voxels; a.n_off = pr->n_offsets; a.n_ev = pr->n_events; a.n_fields = Layout<NC>::NF;
@@ -497,15 +501,18 @@ bmc_status Impl<NC>::jvp(const bmc_problem* pr, const double* params, const bmc_
     void* ws = nullptr;
     const long long nch = (long long)pr->n_voxels * pr->n_offsets;
     const size_t per_node = (size_t)nch * (1 + tg->n_tangents);
-    const bool split = split_nodes(nch, sp, per_node);
+    bool split = split_nodes(nch, sp, per_node);
     const size_t part = split ? (size_t)nch * sp->n_nodes : 0;
     Trains<NC> tn;
-    const bool trains = !work && Trains<NC>::wanted(pr);               // counting calls: event by event
+    bool trains = !work && Trains<NC>::wanted(pr);               // counting calls: event by event
     const size_t train_bytes = trains ? tn.bytes(pr, split ? nch * sp->n_nodes : nch, tangents_per_pass<NC>()) : 0;
     const size_t least = align256(nrec * sizeof(EvRec<double>)) + 256 + align256(sizeof(int4) * pr->n_offsets) +
                          align256(sizeof(int) * pr->n_offsets) + 1024 + order_bytes(nch) + align256(nch);
     const size_t nodes = least + align256(part * (1 + tg->n_tangents) * sizeof(double)) + 512;
-    if ((s = workspace(nodes + train_bytes, st, &ws)) != BMC_OK) return s;
+    int taken = 0;
+    if ((s = workspace({nodes + train_bytes, nodes, least}, st, &ws, &taken)) != BMC_OK) return s;
+    trains = trains && taken < 1;
+    split = split && taken < 2;
     Carve cv(ws);
     ChainArgs a{};
     a.n_vox = pr->n_voxels; a.n_off = pr->n_offsets; a.n_ev = pr->n_events; a.n_fields = Layout<NC>::NF;
@@ -605,10 +612,10 @@ bmc_status Impl<NC>::lm(const bmc_problem* pr, const double* params, const bmc_e
     const int nv = pr->n_voxels, no = pr->n_offsets, P = fs->n_params;
     constexpr int NF = Layout<NC>::NF, N = Layout<NC>::N;
     const size_t nrec = (size_t)no * pr->n_events;
-    const bool split = split_nodes((long long)nv * no, sp, (size_t)nv * no * (1 + P));
+    bool split = split_nodes((long long)nv * no, sp, (size_t)nv * no * (1 + P));
     const size_t part = split ? (size_t)nv * no * sp->n_nodes : 0;
     Trains<NC> tn;
-    const bool trains = Trains<NC>::wanted(pr);
+    bool trains = Trains<NC>::wanted(pr);
     const size_t least = align256(nrec * sizeof(EvRec<double>)) + 2 * align256(sizeof(double) * NF * nv) +
                          2 * align256(sizeof(double) * N * nv) + 2 * align256(sizeof(double) * nv) +
                          align256(sizeof(double) * P * nv) + align256(sizeof(double) * P * nv * N) +
@@ -619,9 +626,12 @@ bmc_status Impl<NC>::lm(const bmc_problem* pr, const double* params, const bmc_e
                          live_bytes((long long)nv * no);
     const size_t nodes = least + align256(part * (1 + P) * sizeof(double)) + 512;
     void* ws = nullptr;
-    if ((s = workspace(nodes + (trains ? tn.bytes(pr, (long long)nv * no * (split ? sp->n_nodes : 1), tangents_per_pass<NC>())
-                                       : 0), st, &ws)) != BMC_OK)
+    int taken = 0;
+    if ((s = workspace({nodes + (trains ? tn.bytes(pr, (long long)nv * no * (split ? sp->n_nodes : 1), tangents_per_pass<NC>())
+                                        : 0), nodes, least}, st, &ws, &taken)) != BMC_OK)
         return s;
+    trains = trains && taken < 1;
+    split = split && taken < 2;
     Carve cv(ws);
     EvRec<double>* rec = cv.take<EvRec<double>>(nrec);
     double* px = cv.take<double>((size_t)NF * nv);

@@ -332,6 +332,41 @@ def test_chunks_of_propagators_with_tangents_give_the_bits_of_one(cuda, nc, n, T
         assert np.abs(j1[t] - jc[t]).max() <= 1e-9 * np.abs(jc[t]).max()
 
 
+@pytest.mark.gpu
+def test_a_call_without_room_for_propagators_runs_without(cuda):
+    """Scratch for speed is not needed: a captured call whose stream's workspace holds the call but not the propagators
+    (here: left by a counting call, which forms none) is accepted and integrates event by event."""
+    torch = cuda
+    from bmc_b200 import _lib
+    from bmc_b200.simulation import DeviceEvents, problem
+    nc, n = 4, 3000
+    P, M0 = _voxels(n, nc, seed=43)
+    ev = _table([_row(f, pulses=9, samples=12) for f in OFFSETS])
+    rows = ev.dt.shape[0]
+    dev, dP, dM = DeviceEvents(ev), torch.as_tensor(P).cuda(), torch.as_tensor(M0).cuda()
+    pr = problem(n, rows, ev.dt.shape[1], nc, 2 * (1 + nc), _lib.F64)
+    z = torch.zeros((n, rows), dtype=torch.float64, device="cuda")
+    want = _simulate(torch, P, M0, ev, nc)
+    _simulate(torch, P, M0, ev, nc, entry="bmc_simulate_noalloc")        # every kernel loaded before the capture
+    L = _lib.lib()
+    stream = torch.cuda.Stream()
+    work = torch.zeros(5, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    call = lambda f, *extra: _lib.check(f(pr, _lib.ptr(dP), dev.struct, _lib.ptr(dM), None, _lib.ptr(z), *extra,
+                                          _lib.stream_handle()))
+    with torch.cuda.stream(stream):
+        call(L.bmc_simulate_counted, _lib.ptr(work))
+        stream.synchronize()
+        z.zero_()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream):
+            call(L.bmc_simulate)
+        g.replay()
+        stream.synchronize()
+    assert np.abs(z.cpu().numpy() - want).max() < 1e-10
+    del g
+
+
 def _bound(n, theta, x):
     from math import factorial as f
     return 2.0 / 4 ** n * sum(theta ** (2 * j) / f(2 * j) * x ** (n - j) / f(n - j) for j in range(n + 1))
