@@ -284,6 +284,8 @@ def _joint_lm(steps, x_loc, x_s, lo_l, hi_l, lo_s, hi_s, lam0, n_iter, allsum=No
     damping for the whole problem; the damped step from the Schur sums of every rank; the trial point
     clipped into the bounds; accepted if the summed cost falls (lam x 0.5, the normal equations refreshed
     at the new point), else lam x 3 and the same normal equations again (the same x gives the same J).
+    The cost kept is the accepted trial point's: the first is taken from the normal equations' residuals, and the tangent
+    and the primal passes agree to ~1e-13 only, while near a minimum a step lowers the cost by less.
 
     `steps` supplies the local arithmetic (normal, eliminate, back, costs: see _JointSteps); every
     quantity is a torch tensor on the steps' device, and the loop reads no value back to the host
@@ -309,10 +311,9 @@ def _joint_lm(steps, x_loc, x_s, lo_l, hi_l, lo_s, hi_s, lam0, n_iter, allsum=No
         x_loc.copy_(torch.where(better, xt, x_loc))
         x_s.copy_(torch.where(better, xst, x_s))
         lam.copy_(torch.where(better, lam * 0.5, lam * 3.0))
-        if last:
-            c.copy_(torch.where(better, ct, c))
-        else:
-            c.copy_(torch.where(better, red(steps.normal(x_loc, x_s, better).clone()), c))
+        c.copy_(torch.where(better, ct, c))
+        if not last:
+            steps.normal(x_loc, x_s, better)
 
     n_iter = int(n_iter)
     it = 0

@@ -315,7 +315,8 @@ bmc_status bmc_normal_segments(int32_t n_voxels, int32_t n_params, int64_t n_cha
  *     d_x[index[v]][j] * scales[j] (d_x [.][n_local], d_index [n_voxels], scales a host array) and row
  *     shared_row (-1: none) by d_shared[0] * shared_scale; n_local <= 8.
  *   bmc_segment_costs: d_cost[index[v]] = sum of (d_z - d_zm)^2 over voxel v's chains, in
- *     bmc_normal_segments' order (so a point's cost is the same double in both).
+ *     bmc_normal_segments' order (so the cost is the same double in both for the same Z; the passes with and without
+ *     tangents agree in Z to rounding, ~1e-13, so a fit compares trial costs with one another).
  */
 bmc_status bmc_joint_params(int32_t n_voxels, int32_t n_fields, const double* d_base, const int64_t* d_index,
                             const double* d_x, int32_t n_local, const int32_t* rows, const double* scales,

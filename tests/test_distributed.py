@@ -162,12 +162,12 @@ class _CpuSteps:
         return self.torch.tensor(((y - self.data) ** 2).sum(axis=1))
 
 
-def _toy_fit(data, free, ranks_of=None, allsum=None, n_iter=8):
+def _toy_fit(data, free, ranks_of=None, allsum=None, n_iter=8, steps_of=_CpuSteps):
     import torch
     from bmc_b200.uneven import _joint_lm
     n = data.shape[0]
     mine = np.arange(n) if ranks_of is None else ranks_of
-    steps = _CpuSteps(data[mine], free[mine])
+    steps = steps_of(data[mine], free[mine])
     x_loc = torch.tensor(np.tile([1.0, 0.8], (mine.size, 1)), dtype=torch.float64)
     x_s = torch.tensor([0.1], dtype=torch.float64)
     lo_l, hi_l = torch.tensor([0.0, 0.0], dtype=torch.float64), torch.tensor([5.0, 5.0], dtype=torch.float64)
@@ -244,3 +244,23 @@ def test_sharded_joint_lm_takes_the_one_rank_and_dense_steps():
     xo = O.levenberg_marquardt(resid_jac, x0, lo, hi, n_iter=8, free=fr)
     np.testing.assert_allclose(got, xo[:-1].reshape(n, 2), rtol=1e-8)
     assert out[2 * n] == __import__("pytest").approx(xo[-1], rel=1e-8)
+
+
+class _OtherNormalCost(_CpuSteps):
+    """Normal equations from other kernels than the trial costs: the cost they report is off by a part in 1e6."""
+
+    def normal(self, x_loc, x_s, moved=None):
+        return super().normal(x_loc, x_s, moved) * (1.0 - 1e-6)
+
+
+def test_joint_costs_that_are_compared_come_from_one_kernel():
+    """The normal equations' cost enters the first comparison alone: the fit takes the same steps and reports the same
+    costs where it differs from the trial points' (here it would refuse every step that gains less than 1e-6)."""
+    data = _toy()
+    free = np.ones((data.shape[0], 2))
+    x, s, c = _toy_fit(data, free, n_iter=12)
+    x1, s1, c1 = _toy_fit(data, free, n_iter=12, steps_of=_OtherNormalCost)
+    assert np.diff(c.numpy())[5:].min() > -1e-6 * float(c[-1])         # the last steps gain less
+    np.testing.assert_array_equal(c1.numpy(), c.numpy())
+    np.testing.assert_array_equal(x1.numpy(), x.numpy())
+    assert float(s1[0]) == float(s[0])
