@@ -196,7 +196,7 @@ constexpr int tangents_per_pass() { return NC <= 1 ? 2 : 1; }
 
 // Shaped-pulse trains of a call: the rows' units and amplitudes, and the propagators (with those of `tangents`
 // derivatives) of `chunk` chains at a time: whole waves of the chain kernel that applies them, as many as kTrainBytes
-// hold and at least one (131 MB with four pools, 173 with five; 175 and 230 with a tangent), or waves of train_kernel's
+// hold and at least one (131 MB with four pools, 115 with five; 175 and 230 with a tangent), or waves of train_kernel's
 // warps where fewer fit. A call of at most a chunk takes every chain in one launch. A larger one takes, chunk by chunk, the
 // chains that have a propagator, and all others (rows without a train, chains whose propagator is refused) in launches over
 // the whole order, for chunk by chunk each launch ends in a partly empty wave. 16,384 voxels x 101 rows, everything in

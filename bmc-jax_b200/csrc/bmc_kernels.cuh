@@ -47,15 +47,18 @@ struct DenseGroup {
     static constexpr int LD = NA | 1;
 };
 
-// Warps per block and the blocks per SM the register allocation aims at, per instantiation (the forward
-// kernels' count measured; a build may set BMC_FWD_MIN_BLOCKS for a sweep).
+// Warps per block and the blocks per SM the register allocation aims at, per instantiation (measured; a build may set
+// BMC_FWD_MIN_BLOCKS for a sweep). In float64 with five pools two blocks: with the 168 registers of three, the loops of the
+// Taylor action spill (8,192 voxels x 101 rows of 64 pulses: 17.2 ms with three, 9.5 with two; 20 block pulses 51.7 and 49.3; one
+// spectrum of 20 pulses x 20 samples event by event 24.8 and 11.9). With four pools two blocks gain 6% on events and lose 5% on
+// repeated blocks.
 #ifndef BMC_FWD_MIN_BLOCKS
 #define BMC_FWD_MIN_BLOCKS 3
 #endif
-template <int NC, int NT>
+template <int NC, int NT, typename R = double>
 struct ChainLaunch {
     static constexpr int kWarps = 4;
-    static constexpr int kMinBlocks = NT == 0 ? BMC_FWD_MIN_BLOCKS : 2;
+    static constexpr int kMinBlocks = NT == 0 && (NC < 5 || sizeof(R) == 4) ? BMC_FWD_MIN_BLOCKS : 2;
 };
 
 template <int NC, typename R, int NT>
@@ -536,7 +539,7 @@ __device__ __noinline__ void train_apply(const double* __restrict__ p, double c,
 // COUNT: the launch adds its work counts to a.work (the measurement entry points); the other launches
 // carry no counters at all.
 template <int NC, typename R, int NT, bool UNEVEN = false, bool COUNT = false>
-__global__ void __launch_bounds__(32 * ChainLaunch<NC, NT>::kWarps, ChainLaunch<NC, NT>::kMinBlocks)
+__global__ void __launch_bounds__(32 * ChainLaunch<NC, NT>::kWarps, ChainLaunch<NC, NT, R>::kMinBlocks)
 chain_kernel(const ChainArgs a, const __grid_constant__ TaylorTable tt) {
     using D = Dn<R, NT>;
     using C = Chain<NC, R, NT>;

@@ -293,7 +293,7 @@ def _tiled(a, n):
     return np.ascontiguousarray(np.resize(a.T, (n, a.shape[0])).T)
 
 
-# more chains than one chunk of propagators holds (of bmc_simulate 170,496 with two pools, 56,832 with five; with tangents
+# more chains than one chunk of propagators holds (of bmc_simulate 170,496 with two pools, 37,888 with five; with tangents
 # 37,888 from four pools on, 113,664 with one; of bmc_simulate_noalloc 10,656 with five) and than one window of flags
 # (4,194,304), an odd rest each
 @pytest.mark.gpu
