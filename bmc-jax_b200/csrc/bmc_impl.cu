@@ -212,8 +212,8 @@ struct Trains {
     TrainArgs tr{};
     const TaylorTable* tt64 = nullptr;   // the float64 table, which the propagators are formed with
 
-    // tables too short for the pulses' least uses have no trains
-    static bool wanted(const bmc_problem* pr) { return pr->n_events >= train_min_uses<NC>() * kTrainMinSamples; }
+    // whether the table can have trains
+    static bool wanted(const bmc_problem* pr, bool tangents) { return pr->n_events >= train_min_events<NC>(tangents); }
 
     size_t per_chain() const { return sizeof(double) * mats * TrainShape<NC>::N * TrainShape<NC>::NS; }
     size_t fixed_bytes(const bmc_problem* pr, int tangents) {
@@ -245,7 +245,7 @@ struct Trains {
         tr.ok = cv.take<unsigned char>(window);
         tr.kinds = cv.take<int>(1);
         CUDA_TRY(cudaMemsetAsync(tr.kinds, 0, sizeof(int), st));
-        train_scan_kernel<<<a.n_off, kTrainScanThreads, 0, st>>>(rec, a.n_ev, a.n_off, train_min_uses<NC>(), a.seg, rows,
+        train_scan_kernel<<<a.n_off, kTrainScanThreads, 0, st>>>(rec, a.n_ev, a.n_off, train_cost<NC>(mats > 1), a.seg, rows,
                                                                  rho, max_samples, tr.kinds);
         CUDA_TRY(cudaGetLastError());
         a.train = rows;
@@ -429,7 +429,7 @@ bmc_status Impl<NC>::simulate(const bmc_problem* pr, const double* params, const
     const size_t part = split ? per_node * sp->n_nodes : 0;
     Trains<NC> tn;
     // the counting calls integrate event by event: their counts are the work of that
-    bool trains = pr->precision != BMC_F32 && !work && Trains<NC>::wanted(pr);
+    bool trains = pr->precision != BMC_F32 && !work && Trains<NC>::wanted(pr, false);
     const size_t least = align256(nrec * recb) + 256 + align256(sizeof(int4) * pr->n_offsets) + order_bytes(nch);
     const size_t nodes = least + align256(part * sizeof(double));
     int taken = 0;
@@ -504,7 +504,7 @@ bmc_status Impl<NC>::jvp(const bmc_problem* pr, const double* params, const bmc_
     bool split = split_nodes(nch, sp, per_node);
     const size_t part = split ? (size_t)nch * sp->n_nodes : 0;
     Trains<NC> tn;
-    bool trains = !work && Trains<NC>::wanted(pr);               // counting calls: event by event
+    bool trains = !work && Trains<NC>::wanted(pr, true);               // counting calls: event by event
     const size_t train_bytes = trains ? tn.bytes(pr, split ? nch * sp->n_nodes : nch, tangents_per_pass<NC>()) : 0;
     const size_t least = align256(nrec * sizeof(EvRec<double>)) + 256 + align256(sizeof(int4) * pr->n_offsets) +
                          align256(sizeof(int) * pr->n_offsets) + 1024 + order_bytes(nch) + align256(nch);
@@ -615,7 +615,7 @@ bmc_status Impl<NC>::lm(const bmc_problem* pr, const double* params, const bmc_e
     bool split = split_nodes((long long)nv * no, sp, (size_t)nv * no * (1 + P));
     const size_t part = split ? (size_t)nv * no * sp->n_nodes : 0;
     Trains<NC> tn;
-    bool trains = Trains<NC>::wanted(pr);
+    bool trains = Trains<NC>::wanted(pr, true);
     const size_t least = align256(nrec * sizeof(EvRec<double>)) + 2 * align256(sizeof(double) * NF * nv) +
                          2 * align256(sizeof(double) * N * nv) + 2 * align256(sizeof(double) * nv) +
                          align256(sizeof(double) * P * nv) + align256(sizeof(double) * P * nv * N) +
@@ -760,7 +760,7 @@ bmc_status run_noalloc(const bmc_problem* pr, const double* params, const bmc_ev
         if ((s = scan_blocks(rec, pr->n_offsets, pr->n_events, pr->n_offsets, ws.seg, st)) != BMC_OK) return s;
         a.seg = ws.seg;
         Trains<NC> tn;
-        if (Trains<NC>::wanted(pr)) {
+        if (Trains<NC>::wanted(pr, false)) {
             // as many chains at a time as the static array holds (its size covers every table's amplitudes)
             tn.bytes(pr, (long long)pr->n_voxels * pr->n_offsets, 0, ws.train_bytes - tn.fixed_bytes(pr, 0));
             tn.tt64 = ws.tt64;

@@ -49,10 +49,30 @@ struct TrainArgs {
     int* kinds;                // kTrained and kPlain by the rows, kRefused by the chains (ChainArgs::kinds)
 };
 
-// Uses of a pulse from which its propagator pays, by pool count. One sample costs the propagator 2 NT^3 matrix
-// products of 8 x 8 x 4 plus the interpolation, whatever the uses; the Taylor action costs ~20 sparse products per use.
+// From when on a pulse's propagator pays: uses x (samples, and kTrainGapEvents for a gap's delays) >= fixed + sample x samples, in
+// Taylor actions of one event: the cost of a propagator's exponentials at the nodes, and of its products and interpolation
+// for one sample (kTrainSkewed times that without the mirror image). Measured by pool count on 51,712 chains (25,856 with a
+// tangent), pulses of 10, 30 and 100 samples (0.5 ms, 1 uT) with and without a 5 ms gap, 2 to 8 uses, against the Taylor
+// action before there were propagators, its lanes in step (now up to twice as fast). With four pools and a gap, propagator /
+// that in ms: 4 x 10 samples 2.31 / 1.61, 8 x 10 2.44 / 3.12, 4 x 30 2.59 / 3.15, 2 x 100 3.55 / 4.26; with two pools 4 x 10 1.72 /
+// 1.20, 8 x 10 1.77 / 2.26. The line knows the table alone, so that a chain's result does not depend on how many others the
+// call has: twice as many chains move it up by a quarter, an eighth of them down by half, and one spectrum gains from two
+// uses on (four pools, 2 x 10 samples: 0.08 ms against 0.28).
+constexpr double kTrainGapEvents = 5.0, kTrainSkewed = 1.75;
+struct TrainCost {
+    double fixed, sample, skewed;
+};
 template <int NC>
-constexpr int train_min_uses() { return NC <= 1 ? 2 : (NC <= 4 ? 4 : 8); }
+constexpr TrainCost train_cost(bool tangents) {
+    constexpr double fixed[2][6] = {{110, 44, 78, 77, 88, 150}, {52, 43, 75, 59, 54, 93}};
+    constexpr double sample[2][6] = {{1.4, 0.42, 1.0, 0.95, 0.75, 2.2}, {2.0, 0.78, 2.55, 1.1, 1.0, 2.8}};
+    return {fixed[tangents][NC], sample[tangents][NC], sample[tangents][NC] * (tangents ? 1.0 : kTrainSkewed)};
+}
+// the fewest events that a table with a train has (a pulse of kTrainMinSamples and its gap)
+template <int NC>
+constexpr int train_min_events(bool tangents) {
+    return (int)(train_cost<NC>(tangents).fixed * kTrainMinSamples / (kTrainMinSamples + kTrainGapEvents));
+}
 
 // Chebyshev nodes of (0, 1), ascending: sin^2(pi (2 q + 1) / (4 n))
 template <int NQ>
@@ -77,7 +97,7 @@ constexpr int kTrainScanThreads = 256;
 // relative amplitudes. A row whose repeated block (seg) saves more events has no train; a row with one keeps its
 // block for the chains that have no propagator.
 static __global__ void __launch_bounds__(kTrainScanThreads)
-train_scan_kernel(EvRec<double>* __restrict__ ev, int n_ev, int stride, int min_uses, const int4* __restrict__ seg,
+train_scan_kernel(EvRec<double>* __restrict__ ev, int n_ev, int stride, const TrainCost cost, const int4* __restrict__ seg,
                   TrainRow* __restrict__ rows, double* __restrict__ rho, int max_samples, int* __restrict__ kinds) {
     __shared__ int starts[kTrainMaxPulses], ends[kTrainMaxPulses];
     __shared__ unsigned char match[kTrainMaxPulses];
@@ -130,7 +150,7 @@ train_scan_kernel(EvRec<double>* __restrict__ ev, int n_ev, int stride, int min_
         __syncthreads();
     }
     const int np = n_start;
-    if (np >= min_uses && np <= kTrainMaxPulses && np == n_end) {     // the same in every thread of the block
+    if (np >= 2 && np <= kTrainMaxPulses && np == n_end) {     // the same in every thread of the block
         const int ref = (np - 1) / 2, r0 = starts[ref], n = ends[ref] - r0 + 1;
         if (n >= kTrainMinSamples && n <= max_samples) {
             for (int p = tid; p < np; p += kTrainScanThreads) match[p] = ends[p] - starts[p] + 1 == n;
@@ -193,7 +213,9 @@ train_scan_kernel(EvRec<double>* __restrict__ ev, int n_ev, int stride, int min_
             const int4 blk = seg[blockIdx.x];
             const long long block_saves = blk.z >= 2 ? (long long)(blk.z - 1) * blk.y : 0;
             const double wm = wmax_s;
-            if (uses >= min_uses && wm > 0.0 && wm < INFINITY && (long long)(uses - 1) * n > block_saves) {
+            const bool pays = uses >= 2 && uses * (n + (gap > 0 ? kTrainGapEvents : 0.0)) >=
+                                               cost.fixed + n * (flags[2] ? cost.sample : cost.skewed);
+            if (pays && wm > 0.0 && wm < INFINITY && (long long)(uses - 1) * n > block_saves) {
                 out = TrainRow{r0, n, gap, run, run * unit, flags[2], wm};
                 for (int p = tid; p < np; p += kTrainScanThreads)
                     if (match[p] && (run == 1 || p == first_match)) {

@@ -17,7 +17,7 @@ def _renamed(ev, where, t):
 
 
 def _train():
-    ev = _table([_row(f, pulses=6, samples=12, gap=((0, 0.004),)) for f in OFFSETS])
+    ev = _table([_row(f, pulses=9, samples=12, gap=((0, 0.004),)) for f in OFFSETS])
     delays = (ev.type == 0) & (ev.dt > 0)
     delays[:, -3:] = False
     return ev, delays

@@ -67,6 +67,19 @@ def _simulate(torch, P, M0, ev, nc, precision=0, spread=None, entry="bmc_simulat
     return out.cpu().numpy()
 
 
+def _counted(torch, P, M0, ev, nc):
+    """Z of the counting call, which integrates every event."""
+    from bmc_b200 import _lib
+    from bmc_b200.simulation import DeviceEvents, problem
+    n, rows = P.shape[1], ev.dt.shape[0]
+    dev, dP, dM = DeviceEvents(ev), torch.as_tensor(P).cuda(), torch.as_tensor(np.ascontiguousarray(M0)).cuda()
+    out, work = torch.empty((n, rows), dtype=torch.float64, device="cuda"), torch.zeros(5, dtype=torch.int64, device="cuda")
+    _lib.check(_lib.lib().bmc_simulate_counted(problem(n, rows, ev.dt.shape[1], nc, 2 * (1 + nc), _lib.F64), _lib.ptr(dP),
+                                               dev.struct, _lib.ptr(dM), None, _lib.ptr(out), _lib.ptr(work),
+                                               _lib.stream_handle()))
+    return out.cpu().numpy()
+
+
 OFFSETS = np.array([-900.0, -447.2, -30.0, 0.0, 127.7, 447.2, 1200.0])
 
 
@@ -83,8 +96,36 @@ def _close(z, P, M0, ev, nc, tol=1e-10):
 @pytest.mark.parametrize("skew", [0.05, 0.0], ids=["skewed", "mirrored"])
 def test_pool_counts_match_the_oracle(cuda, nc, samples, skew):
     P, M0 = _voxels(3, nc, mt=nc != 1)
-    ev = _table([_row(f, pulses=9, samples=samples, skew=skew) for f in OFFSETS])
-    _close(_simulate(cuda, P, M0, ev, nc), P, M0, ev, nc)
+    for pulses in (9, 16):                                 # (five pools: from 14 pulses of 8 samples on)
+        ev = _table([_row(f, pulses=pulses, samples=samples, skew=skew) for f in OFFSETS])
+        _close(_simulate(cuda, P, M0, ev, nc), P, M0, ev, nc)
+
+
+# when a propagator is formed: uses x samples >= FIXED + SAMPLE x samples for a mirrored pulse without a gap (train_cost)
+FIXED, SAMPLE = [110, 44, 78, 77, 88, 150], [1.4, 0.42, 1.0, 0.95, 0.75, 2.2]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nc", range(6))
+@pytest.mark.parametrize("samples", [8, 30])
+def test_few_pulses_are_integrated_event_by_event(cuda, nc, samples):
+    """One use below the line the events are integrated as the counting call does, bit for bit; at the line the propagator
+    gives the same to 1e-11 in other roundings."""
+    P, M0 = _voxels(3, nc, seed=47)
+    need = int(np.ceil((FIXED[nc] + SAMPLE[nc] * samples) / samples))
+    for uses in (need - 1, need):
+        rows = []
+        for f in OFFSETS:
+            t = (np.arange(samples) + 0.5) / samples
+            amp = 60.0 * np.exp(-((t - 0.5) ** 2) / 0.06)
+            amp = 0.5 * (amp + amp[::-1])
+            rows.append([(1, 5e-4, a, 0.3 * j, f) for j in range(uses) for a in amp] + [(3, 0.0, 0.0, 0.0, 0.0)])
+        ev = _table(rows)
+        z = _simulate(cuda, P, M0, ev, nc)
+        _close(z, P, M0, ev, nc)
+        c = _counted(cuda, P, M0, ev, nc)
+        assert np.abs(z - c).max() < 1e-11
+        assert np.array_equal(z, c) == (uses < need), (uses, need)
 
 
 @pytest.mark.gpu
@@ -118,6 +159,8 @@ FORMS = {
     "mirrored": dict(skew=0.0, samples=21),
     "mirrored_even": dict(skew=0.0, samples=40, phase=0.4, phase_step=1.0),
     "mirrored_strong": dict(skew=0.0, samples=9, b1=8.0, tp=0.01),
+    "mirrored_strong_8": dict(skew=0.0, samples=9, b1=8.0, tp=0.01, pulses=8),
+    "own_delays_9": dict(gap=((4, 0.0009), (0, 0.01)), gap_step=1e-4, phase_step=0.9, pulses=9),
     "samples_1100": dict(samples=1100, tp=0.05, pulses=4),
 }
 
@@ -215,7 +258,7 @@ def _jvp(torch, P, M0, ev, nc, rows, seeds, dm0=None, spread=None, counted=False
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("nc", [0, 1, 2, 4, 5])
-@pytest.mark.parametrize("form", ["plain", "phases", "spoiled", "own_delays", "few", "strong", "readout_between"])
+@pytest.mark.parametrize("form", ["plain", "phases", "spoiled", "own_delays", "own_delays_9", "few", "strong", "readout_between"])
 def test_tangents_match_the_event_by_event_path(cuda, nc, form):
     """Every kind of tangent (rates, fractions, shifts, B0, B1, MT, the start state, the spread's width) through the
     propagators against forward mode over every event (the counting call): 1e-9 of each tangent's largest value."""
@@ -285,7 +328,7 @@ def _mixed_table():
         elif k == "blocks":
             rows.append([(1, 0.05, 40.0, 0.0, f), (0, 0.005, 0.0, 0.0, 0.0)] * 10 + [(3, 0.0, 0.0, 0.0, 0.0)])
         else:
-            rows.append(_row(f, **{**dict(samples=12, pulses=9), **FORMS.get(k, {}), **kw}))
+            rows.append(_row(f, **{**dict(samples=12, pulses=16), **FORMS.get(k, {}), **kw}))
     return _table(rows)
 
 
@@ -341,7 +384,7 @@ def test_a_call_without_room_for_propagators_runs_without(cuda):
     from bmc_b200.simulation import DeviceEvents, problem
     nc, n = 4, 3000
     P, M0 = _voxels(n, nc, seed=43)
-    ev = _table([_row(f, pulses=9, samples=12) for f in OFFSETS])
+    ev = _table([_row(f, pulses=14, samples=12) for f in OFFSETS])
     rows = ev.dt.shape[0]
     dev, dP, dM = DeviceEvents(ev), torch.as_tensor(P).cuda(), torch.as_tensor(M0).cuda()
     pr = problem(n, rows, ev.dt.shape[1], nc, 2 * (1 + nc), _lib.F64)
