@@ -372,7 +372,6 @@ adjoint_block_kernel(const ChainArgs a, const int4* __restrict__ blk, int n_tan,
     long long ci = first + lane;
     const bool valid = lane < a.cpw && ci < nch;
     if (!valid) ci = first < nch ? first : nch - 1;
-    if (a.order) ci = a.order[ci];
     const int2 vm = a.chain_map[ci];
     const int v = vm.x, o = vm.y;
     const int t = a.vox_table[v];

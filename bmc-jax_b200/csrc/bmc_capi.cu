@@ -2,8 +2,8 @@
 //
 // Host side of the library: argument checks, a per-device workspace cache, the truncated-Taylor tables, the
 // dispatch over pool count, uneven plans and the joint step. What is compiled per pool count (the launches of
-// a call, the Levenberg-Marquardt loop) is in bmc_impl.cu. Every launch is asynchronous on the caller's stream,
-// with no host synchronisation inside a call.
+// a call, the Levenberg-Marquardt loop) is in bmc_impl.cu. Every launch is asynchronous on the caller's stream; a call
+// synchronises with the host only to choose the adjoint kernel (use_adjoint).
 #include <cuda_runtime.h>
 
 #include <algorithm>

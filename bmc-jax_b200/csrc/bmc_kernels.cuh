@@ -28,8 +28,10 @@ __device__ __forceinline__ R warp_max(R x) {
 // the block propagator's columns by the truncated Taylor series instead)
 constexpr double kBlockDenseNorm = 4.0;
 
-// the norm above which a free event without transverse magnetisation takes its z block alone (Chain::z_event): its
-// ~11 Horner steps of NC + 3 columns and ~10 squarings cost what the Taylor action costs at a norm of about 8
+// the norm above which a free event without transverse magnetisation takes its z block alone (Chain::z_event) rather than the
+// Taylor action. 103,424 chains x 40 delays behind spoilers: even at mean norms of 4.4 (one pool, 0.72 ms a call both ways),
+// 4.8 (two), 6.6 (four) and 8.5 (five); delays of 1 ms (norms 7 to 10) by the block / the action: 0.75 / 0.92, 0.95 / 1.25, 1.72 /
+// 2.21, 2.19 / 2.40 ms.
 constexpr double kZFreeNorm = 8.0;
 
 // the norm above which an event of a small generator goes to sym_event: its ~4,500 multiply-adds against 175 per unit
@@ -879,7 +881,7 @@ __global__ void __launch_bounds__(128) cost_kernel(const ChainArgs a, float* __r
 // L <= kBlockMaxL events that saves the most events, among the blocks that hold no readout, evolve the
 // state, and either hold an event of at least kBlockMinDt (exponentiated densely, the work the reuse
 // saves) or repeat so often (r >= kBlockMinRepeats) that the per-column work of short events pays;
-// (0, 0, 0) where there is none. One thread per row.
+// (0, 0, 0) where there is none.
 // ------------------------------------------------------------------------------------------------
 constexpr int kBlockMaxL = 8;
 constexpr double kBlockMinDt = 1e-3;
