@@ -357,7 +357,9 @@ def run_ours(args, rank, world, local_rank):
         "metric": "Z-spectra/s (batched forward simulation)", "value": value, "unit": "Z-spectra/s",
         "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms,
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": {_lib.F64: "f64", _lib.F32: "f32", _lib.MIXED: "f64 state + f32 Taylor tail (mixed)"}[prec],
+        "dtype": {_lib.F64: "f64", _lib.F32: "f32",
+                  _lib.MIXED: "f64 (the pulses' propagators); f64 state + f32 Taylor tail for the other events "
+                              "(mixed)"}[prec],
         "data": "synthetic (seeded)",
         "config": {"workload": f"forward simulation: {nv} voxels per GPU x {n_off} offsets x {n_ev} events, "
                                f"water + {nc} CEST pools + super-Lorentzian MT (state {N}, augmented {NA}), "
@@ -366,13 +368,13 @@ def run_ours(args, rank, world, local_rank):
                    "parallelism": f"dp{world} (voxels sharded, no collective)",
                    "l2": "flushed between timed steps (256 MB write, untimed)", "b0_spread": spread_cfg,
                    "float32_accuracy": f32_err,
-                   "taylor_tail": {_lib.F64: "Taylor terms below 1e-6 of the state (bound theta^k/k!) formed in "
-                                             "float32, summed into the float64 state once per sub-step; "
-                                             "truncation 1e-13 per sub-step",
-                                   _lib.MIXED: "the first Taylor term of every sub-step in float64 (more where their "
-                                               "bound theta^k/k! exceeds 3x the state), later terms in float32, "
-                                               "summed into the float64 state once per sub-step; truncation 1e-8 "
-                                               "per sub-step",
+                   "taylor_tail": {_lib.F64: "events outside the pulses' propagators (float64): Taylor terms below 1e-6 "
+                                             "of the state (bound theta^k/k!) formed in float32, summed into the float64 "
+                                             "state once per sub-step; truncation 1e-13 per sub-step",
+                                   _lib.MIXED: "events outside the pulses' propagators (float64): the first Taylor "
+                                               "term of every sub-step in float64 (more where their bound theta^k/k! exceeds "
+                                               "3x the state), later terms in float32, summed into the float64 state "
+                                               "once per sub-step; truncation 1e-8 per sub-step",
                                    _lib.F32: "all Taylor terms and the state in float32; truncation 2^-24"}[prec]},
         "e2e": {"value": world * nv / (e2e_ms * 1e-3), "unit": "Z-spectra/s", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h, "ms_per_step": e2e_ms, "steps": e2e_steps},
@@ -381,7 +383,8 @@ def run_ours(args, rank, world, local_rank):
                      "traffic": traffic, "traffic_unit": "bytes per launch",
                      "traffic_source": traffic_src,
                      "kernel": "chain_kernel, event by event (bmc_simulate_counted: its work over its own time; the "
-                               "timed step takes shaped pulses as propagators, whose work is not counted)",
+                               "timed step takes shaped pulses as propagators, whose work is not counted: train_kernel, "
+                               "FP64 datapath 63% of its cycles by ncu, profiles/train_kernel_193vox.md)",
                      "event_by_event_ms": counted_ms,
                      "flops_per_launch": flops, "flops_fp64_pipe": flops64, "flops_fp32_pipe": flops32,
                      "peak_fp64": best, "peak_fp32": best32,
