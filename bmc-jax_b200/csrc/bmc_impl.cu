@@ -288,14 +288,17 @@ struct Trains {
             a.node_lo = j;
             a.node_hi = j + 1;
         };
+        auto with_propagators = [&](unsigned char* ok) {
+            a.prop_ok = ok;
+            const bmc_status e = form<(NT > 0 ? 1 : 0)>(a, ok, NT, st);
+            return e != BMC_OK ? e : launch_chain<NC, double, NT>(a, tt, st);
+        };
         if (all <= chunk) {
             a.parts = kEveryPart;
-            a.prop_ok = tr.ok;
             a.chain_count = all;
             for (int j = 0; j < nodes; ++j) {
                 of_node(j);
-                if ((s = form<(NT > 0 ? 1 : 0)>(a, tr.ok, NT, st)) != BMC_OK || (s = launch_chain<NC, double, NT>(a, tt, st)) != BMC_OK)
-                    return s;
+                if ((s = with_propagators(tr.ok)) != BMC_OK) return s;
             }
             return BMC_OK;
         }
@@ -309,10 +312,7 @@ struct Trains {
                 a.parts = kTrained;
                 for (a.first_chain = lo; a.first_chain < end; a.first_chain += chunk) {
                     a.chain_count = std::min(chunk, end - a.first_chain);
-                    unsigned char* ok = tr.ok + (a.first_chain - lo);
-                    a.prop_ok = ok;
-                    if ((s = form<(NT > 0 ? 1 : 0)>(a, ok, NT, st)) != BMC_OK || (s = launch_chain<NC, double, NT>(a, tt, st)) != BMC_OK)
-                        return s;
+                    if ((s = with_propagators(tr.ok + (a.first_chain - lo))) != BMC_OK) return s;
                 }
                 a.parts = kRefused | (nodes > 1 ? 0 : kPlain);
                 a.first_chain = lo;
